@@ -19,7 +19,7 @@ __device__ __forceinline__ void quantize_store_vec4(float4 v, long i, bool live,
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-    const float d = amax / 127.0f;
+    const float d = quant_scale(amax);
     int sum = 0;
     const uint32_t packed = amax != 0.0f ? quantize4_pack(v, d, sum) : 0u;
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
@@ -42,7 +42,7 @@ __device__ __forceinline__ void quantize_row_vec4(float4 v, int i, bool live, ui
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-    const float d = amax / 127.0f;
+    const float d = quant_scale(amax);
     int sum = 0;
     const uint32_t packed = amax != 0.0f ? quantize4_pack(v, d, sum) : 0u;
     if (live) {
