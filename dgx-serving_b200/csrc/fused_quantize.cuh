@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(256) rmsnorm_quantize_kernel(const float *__re
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const size_t row = blockIdx.x;
     const float *xr = X + row * hh;
+    pdl_wait();              // X may come from the kernel before this one; see quantize_x_q8_vec_kernel for the order
     pdl_launch_dependents();
     float ss = 0.f;
     for (int i = tid; i < hh; i += 256) { const float v = xr[i]; ss = fmaf(v, v, ss); }
@@ -117,8 +118,8 @@ __global__ void __launch_bounds__(256) glu_quantize_kernel(const float4 *__restr
     // row_vecs = IN/4; rows of G and U start pitch_vecs float4s apart (== row_vecs: dense; a fused gate|up tensor
     // [S][2*IN] has pitch 2*IN/4 and U = G + IN)
     const long stride = (long)gridDim.x * blockDim.x;
+    pdl_wait();   // G and U come from the kernel before this one
     pdl_launch_dependents();
-    pdl_wait();   // G and U come from the kernel before this one (a no-op unless launched for programmatic dependent launch)
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i - (threadIdx.x & 31) < nvec; i += stride) {
         const bool live = i < nvec;
         float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -135,17 +136,14 @@ __global__ void __launch_bounds__(256) glu_quantize_kernel(const float4 *__restr
 inline int launch_rmsnorm_quantize(const float *X, const float *W, float eps, int variant, float *Y, int8_t *xq, float *xs,
                                    int32_t *xsum, int IN, int S, cudaStream_t st) {
     uint32_t *q = reinterpret_cast<uint32_t *>(xq);
-    switch (variant) {
-        case 0: rmsnorm_quantize_kernel<0><<<S, 256, 0, st>>>(X, W, eps, Y, q, xs, xsum, IN); break;
-        case 1: rmsnorm_quantize_kernel<1><<<S, 256, 0, st>>>(X, W, eps, Y, q, xs, xsum, IN); break;
-        default: rmsnorm_quantize_kernel<2><<<S, 256, 0, st>>>(X, W, eps, Y, q, xs, xsum, IN); break;
-    }
+    auto kern = variant == 0 ? rmsnorm_quantize_kernel<0> : variant == 1 ? rmsnorm_quantize_kernel<1> : rmsnorm_quantize_kernel<2>;
+    cudaError_t e = launch_pdl(kern, dim3((unsigned)S), dim3(256), 0, st, X, W, eps, Y, q, xs, xsum, IN);
+    if (e != cudaSuccess) return cuda_fail(e, "rmsnorm_quantize_x_q8 launch");
     return launch_status("rmsnorm_quantize_x_q8");
 }
 
 inline int launch_glu_quantize(const float *G, const float *U, int act, float *Y, int8_t *xq, float *xs, int32_t *xsum, int IN,
-                               int S, cudaStream_t st, long pitch = 0 /* floats between rows of G / U; 0 = IN */,
-                               bool pdl = false /* launch for programmatic dependent launch (inside a chain of such kernels) */) {
+                               int S, cudaStream_t st, long pitch = 0 /* floats between rows of G / U; 0 = IN */) {
     const long nvec = (long)S * IN / 4;
     long want = (nvec + 255) / 256, cap = (long)sm_count() * 8;
     const unsigned grid = (unsigned)(want < cap ? want : cap);
@@ -153,12 +151,8 @@ inline int launch_glu_quantize(const float *G, const float *U, int act, float *Y
     float4 *y = reinterpret_cast<float4 *>(Y);
     uint32_t *q = reinterpret_cast<uint32_t *>(xq);
     const long pv = (pitch > 0 ? pitch : IN) / 4;
-    if (pdl) {
-        cudaError_t e = act == 0 ? launch_pdl(glu_quantize_kernel<0>, dim3(grid), dim3(256), 0, st, g, u, y, q, xs, xsum, nvec, IN / 4, pv)
-                                 : launch_pdl(glu_quantize_kernel<1>, dim3(grid), dim3(256), 0, st, g, u, y, q, xs, xsum, nvec, IN / 4, pv);
-        if (e != cudaSuccess) return cuda_fail(e, "glu_quantize_x_q8 launch");
-    } else if (act == 0) glu_quantize_kernel<0><<<grid, 256, 0, st>>>(g, u, y, q, xs, xsum, nvec, IN / 4, pv);
-    else glu_quantize_kernel<1><<<grid, 256, 0, st>>>(g, u, y, q, xs, xsum, nvec, IN / 4, pv);
+    cudaError_t e = launch_pdl(act == 0 ? glu_quantize_kernel<0> : glu_quantize_kernel<1>, dim3(grid), dim3(256), 0, st, g, u, y, q, xs, xsum, nvec, IN / 4, pv);
+    if (e != cudaSuccess) return cuda_fail(e, "glu_quantize_x_q8 launch");
     return launch_status("glu_quantize_x_q8");
 }
 
