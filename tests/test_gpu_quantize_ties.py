@@ -3,7 +3,7 @@
 Pointers that are not 16-byte aligned take quantize_x_q8_scalar_kernel, which divides every element; aligned ones take the
 vector kernel, which divides only where x / d lies too near a half-integer for the reciprocal to decide.  Both are defined
 as q = rintf(x / d), d = amax / 127, so every bit has to agree.  Inputs: quotients on and one ulp beside every half-integer,
-scales from subnormal to near overflow, zero blocks, infinities and NaN."""
+scales from near the smallest normal number to near overflow, zero blocks, infinities and NaN."""
 import numpy as np
 import pytest
 
@@ -20,7 +20,7 @@ def _blocks(kind, rng):
         x = np.where(rng.random((n, 32)) < 0.5, x, np.nextafter(x, np.float32(np.inf) * np.sign(rng.normal(size=(n, 32))).astype(np.float32)))
         x[:, 0] = amax[:, 0]
     elif kind == "range":
-        x *= np.exp2(rng.uniform(-149, 126, (n, 1))).astype(np.float32)
+        x *= np.exp2(rng.uniform(-115, 126, (n, 1))).astype(np.float32)       # d stays a normal number: then x / d <= 127
         x[::7] = 0.0
         x[3::97, 5] = np.float32(np.finfo(np.float32).max)
     elif kind == "special":
