@@ -1,0 +1,359 @@
+// W4A8 prefill / verify / grouped-expert GEMM whose group dots never leave the register file.
+//   Y[m,n] = sum_b ((float)D[m,n,b] * xs[m,b]) * sw[n,b],   D[m,n,b] = sum_{k in group b} X[m,k]*(Wq[n,k]-8)
+// Same semantics and fp32 order as gemm_w4a8_tc.cuh (t = (float)D*xs rounded, acc = fma(t, sw, acc), groups ascending:
+// the reference's kernels/gemm_mmq.cuh:104-105), hence the same bits.
+//
+// What bounds it.  Both operands carry a scale per 32-element group, so whatever computes the dots, every (m, n, group)
+// costs a conversion, a multiply and an fma on the CUDA cores.  On tcgen05 the dots come out in tensor memory and every
+// group pays, on top of that, a commit, a barrier, tcgen05.ld and a release through four accumulator buffers: about 950 SM
+// cycles per 128 x 128 outputs and group, at 6 % tensor-pipe use, and always for 128 rows.  mma.sync m16n8k32 leaves the
+// dots in the registers that the epilogue reads: no hand-off, and a tile has as many rows as there are, in steps of 16.
+// Alone (a loop without loads) MMA 314, I2F 337 and packed mul + fma 370 cycles per 128 x 128 group, together about 500;
+// with the operand and scale traffic the kernel needs 864 with 128 x 128 tiles.  It issues on 44 % of the cycles with two
+// warps per scheduler; the rest are waits on loads from shared memory, on MMA results and on the register file.
+// Measured: 2048 x 17408 x 5120 1118 us (tcgen05 1218), 512 rows 310 (333), 333 x 15360 x 3840 165 (192), 48 x 3840 x 15360 in three
+// K ranges 52 (87).  Slower here: integer-to-float through a preset accumulator (1.5 * 2^23) instead of I2F (1133 against 989
+// cycles), scalar instead of packed fp32 (1044 against 864), scales through registers (977 against 864; they spill).
+//
+// Data flow.  cp.async brings K-tiles of 4 groups into a STAGES-deep ring, laid out [group][row][32 B] for the int8
+// activations and [group][row][16 B] for the packed weights, so that a warp's fragment reads are contiguous (LDS.64 and
+// LDS.32, no conflicts); groups are 32 bytes further apart than they need, which makes the copies' writes conflict-free
+// too.  A lane's word of weights expands to its two B registers with three logic operations (unpack8_x16: even and odd
+// elements), the matching A registers are two byte permutes of eight activations.  Any order of K inside a group gives
+// the same integer.  Scales travel with their K-tile, [row][group], one 16-byte
+// piece per row (element by element where rows of scales are not a multiple of four or not aligned).  One __syncthreads per
+// K-tile; two or three CTAs per SM cover each other's.
+#pragma once
+#include <type_traits>
+#include "common.cuh"
+#include "gemm_w4a8_tc.cuh"
+
+namespace w4a8 {
+namespace gemm_mma {
+
+constexpr int GPK = 4;                    // groups per K-tile
+// live = false writes zeros and reads nothing
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// D(16x8, s32) = A(16x32, s8, row) * B(32x8, s8, col)
+__device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ void fma2(uint64_t &acc, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+// TM m16 tiles x TN n8 tiles per warp, WM x WN warps, CTAs per SM the register and shared-memory budget is cut for.
+template <int TM_, int TN_, int WM_, int WN_, int STAGES_, int CTAS_>
+struct Cfg {
+    static constexpr int TM = TM_, TN = TN_, WM = WM_, WN = WN_, STAGES = STAGES_, CTAS = CTAS_;
+    static constexpr int BM = 16 * TM * WM, BN = 8 * TN * WN, THREADS = 32 * WM * WN;
+    static constexpr int A_GROUP = BM * 32 + 32, B_GROUP = BN * 16 + 32;      // bytes; + 32 keeps the copies' writes conflict-free
+    static constexpr int OFF_SX = GPK * (A_GROUP + B_GROUP), OFF_SW = OFF_SX + BM * GPK * 4;      // scales: [row][group]
+    static constexpr int STAGE = OFF_SW + BN * GPK * 4, SMEM = STAGES * STAGE;
+    static constexpr int RB = (BN + THREADS - 1) / THREADS, RA = (BM + THREADS - 1) / THREADS;   // scale rows per thread
+};
+
+using gemm::GroupList;
+
+template <class C, typename ST, bool GROUPED>
+__global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
+    const int8_t *__restrict__ X, const float *__restrict__ xs, const uint8_t *__restrict__ Wq, const ST *__restrict__ sw,
+    float *__restrict__ Y, int M, int N, int K, int m_tiles, int n_tiles, int gsplit, bool vec_scales, const GroupList gl) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    constexpr int TM = C::TM, TN = C::TN, BM = C::BM, BN = C::BN, NT = C::THREADS, STAGES = C::STAGES;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int wm = warp % C::WM, wn = warp / C::WM;
+    const int nb = K / QBLK;
+
+    // ---- this CTA's unit of work: an output tile (M fastest, so that CTAs running together share weight tiles in L2) and a
+    // range of groups [g0, g1); grouped: 128 outputs of one item (up to BM rows of one expert)
+    int m0, mend, n0, g0 = 0, g1 = nb, split = 0;
+    size_t wrow0 = 0;
+    if (GROUPED) {
+        const int item = blockIdx.x / n_tiles;
+        if (item >= *gl.num_items) return;
+        const int4 it = __ldg(gl.items + item);
+        m0 = it.y; mend = it.y + it.z; n0 = (blockIdx.x % n_tiles) * BN; wrow0 = (size_t)it.x * N;
+    } else {
+        const int tiles = m_tiles * n_tiles, tile = blockIdx.x % tiles;
+        split = blockIdx.x / tiles;
+        m0 = (tile % m_tiles) * BM; mend = M; n0 = (tile / m_tiles) * BN;
+        g0 = min(nb, split * gsplit); g1 = min(nb, g0 + gsplit);
+    }
+    const int nkt = (g1 - g0 + GPK - 1) / GPK;
+
+    // ---- copies: thread -> 16-byte chunk of a row (8 of 128 bytes of activations, 4 of 64 bytes of weights).  Rows past
+    // the end re-read the last one and are never stored; chunks past the last group are skipped and never read.
+    constexpr int AI = (BM * 8 + NT - 1) / NT, BI = (BN * 4 + NT - 1) / NT;
+    static_assert(BM * 8 % NT == 0 && BN * 4 % NT == 0, "whole copy instructions");
+    const uint32_t smem_u = (uint32_t)__cvta_generic_to_shared(smem);
+    const int ca = tid & 7, cb = tid & 3;
+    const int8_t *Xb = X + (size_t)(m0 + (tid >> 3)) * K + ca * 16;
+    const uint8_t *Wb = Wq + (wrow0 + n0 + (tid >> 2)) * (size_t)(K / 2) + cb * 16;
+    const int rows_a = mend - m0 - (tid >> 3), rows_b = N - n0 - (tid >> 2);      // live rows from this thread's first one on
+    const uint32_t adst = smem_u + (ca >> 1) * C::A_GROUP + (tid >> 3) * 32 + (ca & 1) * 16;
+    const uint32_t bdst = smem_u + GPK * C::A_GROUP + cb * C::B_GROUP + (tid >> 2) * 16;
+    auto copy = [&](int kt) {
+        if (kt < nkt) {
+            const int b0 = g0 + kt * GPK, ng = g1 - b0;          // groups left
+            const uint32_t so = (uint32_t)(kt % STAGES) * C::STAGE;
+            if ((ca >> 1) < ng) {
+                const int8_t *src = Xb + (size_t)b0 * 32;
+#pragma unroll
+                for (int i = 0; i < AI; i++) {
+                    const bool live = i * (NT / 8) < rows_a;
+                    cp_async16(adst + so + i * (NT / 8) * 32, live ? src + (size_t)i * (NT / 8) * K : X, live);
+                }
+            }
+            if (cb < ng) {
+                const uint8_t *src = Wb + (size_t)b0 * 16;
+#pragma unroll
+                for (int i = 0; i < BI; i++) {
+                    const bool live = i * (NT / 4) < rows_b;
+                    cp_async16(bdst + so + i * (NT / 4) * 16, live ? src + (size_t)i * (NT / 4) * (K / 2) : Wq, live);
+                }
+            }
+            // scales: a row's GPK of them are one 16-byte (fp16: 8-byte) piece when they line up, else element by element
+            const bool vec = vec_scales && ng >= GPK;
+#pragma unroll
+            for (int r = 0; r < C::RA; r++) {
+                const int m = tid + r * NT;
+                if (BM % NT == 0 || m < BM) {
+                    const float *p = xs + (size_t)min(m0 + m, mend - 1) * nb + b0;
+                    const uint32_t o = so + C::OFF_SX + m * (GPK * 4);
+                    if (vec) cp_async16(smem_u + o, p, true);
+                    else
+                        for (int q = 0; q < GPK; q++)
+                            if (q < ng) *reinterpret_cast<float *>(smem + o + 4 * q) = p[q];
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < C::RB; r++) {
+                const int n = tid + r * NT;
+                if (BN % NT == 0 || n < BN) {
+                    const ST *p = sw + (wrow0 + min(n0 + n, N - 1)) * (size_t)nb + b0;
+                    const uint32_t o = so + C::OFF_SW + n * (GPK * 4);
+                    if (vec) {
+                        if (sizeof(ST) == 4) cp_async16(smem_u + o, p, true);
+                        else cp_async8(smem_u + o, p);
+                    } else
+                        for (int q = 0; q < GPK; q++)
+                            if (q < ng) *reinterpret_cast<ST *>(smem + o + sizeof(ST) * q) = p[q];
+                }
+            }
+        }
+        cp_async_commit();
+    };
+
+    uint64_t acc[TM][TN][2];            // pairs of fp32 sums: row g (columns 2t, 2t + 1), row g + 8
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN; j++) acc[i][j][0] = acc[i][j][1] = 0ull;
+
+    const int rows_w = mend - m0 - wm * 16 * TM;                               // live rows of this warp (may be <= 0)
+    const int live = GROUPED ? min(TM, (rows_w + 15) / 16) : TM;               // live m16 tiles
+    // ng groups of this warp's tile; L = live m16 tiles.  Software pipeline over the columns (n8 tiles) of all groups: the
+    // MMAs of the next column are issued before the current one's results are used, because a result takes far longer
+    // than the dozen instructions that use it and a warp issues in order.
+    auto groups = [&](auto LT, auto NGT, const unsigned char *stage, int bfirst) {
+        constexpr int L = decltype(LT)::value, NG = decltype(NGT)::value;
+        const unsigned char *As = stage + bfirst * C::A_GROUP + (wm * 16 * TM + g) * 32 + t * 8;
+        const unsigned char *Bs = stage + GPK * C::A_GROUP + bfirst * C::B_GROUP + (wn * 8 * TN + g) * 16 + t * 4;
+        const unsigned char *sx = stage + C::OFF_SX + (wm * 16 * TM + g) * (GPK * 4) + bfirst * 4;
+        const unsigned char *ss = stage + C::OFF_SW + (wn * 8 * TN + 2 * t) * (GPK * 4) + bfirst * sizeof(ST);
+        uint32_t a[L][4];
+        int c[2][L][4];
+        float xx[2][L][2], sv[2][2];
+        auto start = [&](int q) {                      // column q % TN of group q / TN: operands, scales, MMAs
+            const int bg = q / TN, j = q % TN;
+            if (j == 0) {
+#pragma unroll
+                for (int i = 0; i < L; i++) {
+                    const uint2 v0 = *reinterpret_cast<const uint2 *>(As + bg * C::A_GROUP + i * 512), v1 = *reinterpret_cast<const uint2 *>(As + bg * C::A_GROUP + i * 512 + 256);
+                    split_even_odd(v0.x, v0.y, a[i][0], a[i][2]);
+                    split_even_odd(v1.x, v1.y, a[i][1], a[i][3]);
+                    xx[bg & 1][i][0] = *reinterpret_cast<const float *>(sx + bg * 4 + (16 * i) * (GPK * 4)) * 0.0625f;         // exact 1/16
+                    xx[bg & 1][i][1] = *reinterpret_cast<const float *>(sx + bg * 4 + (16 * i + 8) * (GPK * 4)) * 0.0625f;
+                }
+            }
+            uint32_t b0, b1;
+            unpack8_x16(*reinterpret_cast<const uint32_t *>(Bs + bg * C::B_GROUP + j * 128), b0, b1);
+            sv[q & 1][0] = sval(*reinterpret_cast<const ST *>(ss + bg * sizeof(ST) + 8 * j * (GPK * 4)));
+            sv[q & 1][1] = sval(*reinterpret_cast<const ST *>(ss + bg * sizeof(ST) + (8 * j + 1) * (GPK * 4)));
+#pragma unroll
+            for (int i = 0; i < L; i++) mma_s8(c[q & 1][i], a[i], b0, b1);
+        };
+        start(0);
+#pragma unroll
+        for (int q = 0; q < NG * TN; q++) {
+            if (q + 1 < NG * TN) start(q + 1);
+            const int bg = q / TN, j = q % TN;
+            const uint64_t s2 = pack2(sv[q & 1][0], sv[q & 1][1]);
+#pragma unroll
+            for (int i = 0; i < L; i++) {
+                const int (&d)[4] = c[q & 1][i];
+                const float x0 = xx[bg & 1][i][0], x1 = xx[bg & 1][i][1];
+                fma2(acc[i][j][0], mul2(pack2(__int2float_rn(d[0]), __int2float_rn(d[1])), pack2(x0, x0)), s2);
+                fma2(acc[i][j][1], mul2(pack2(__int2float_rn(d[2]), __int2float_rn(d[3])), pack2(x1, x1)), s2);
+            }
+        }
+    };
+
+    // ---- main loop
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; s++) copy(s);
+    for (int kt = 0; kt < nkt; kt++) {
+        cp_async_wait<STAGES - 2>();                  // K-tile kt has landed (this thread's copies) ...
+        __syncthreads();                              // ... and everybody's; K-tile kt - 1 is done with
+        copy(kt + STAGES - 1);                        // into the slot K-tile kt - 1 used
+        const unsigned char *stage = smem + (kt % STAGES) * C::STAGE;
+        const int ng = min(GPK, g1 - (g0 + kt * GPK));
+        auto ktile = [&](auto LT) {
+            if (ng == GPK) groups(LT, std::integral_constant<int, GPK>(), stage, 0);
+            else {
+#pragma unroll 1
+                for (int b = 0; b < ng; b++) groups(LT, std::integral_constant<int, 1>(), stage, b);
+            }
+        };
+        if constexpr (!GROUPED) ktile(std::integral_constant<int, TM>());
+        else {                                        // an item's rows rarely fill the tile: only its live m16 tiles cost anything
+            if (TM >= 4 && live == 4) ktile(std::integral_constant<int, TM < 4 ? TM : 4>());
+            else if (TM >= 3 && live == 3) ktile(std::integral_constant<int, TM < 3 ? TM : 3>());
+            else if (TM >= 2 && live == 2) ktile(std::integral_constant<int, TM < 2 ? TM : 2>());
+            else if (live == 1) ktile(std::integral_constant<int, 1>());
+        }
+    }
+    cp_async_wait<0>();
+
+    // ---- store: a fragment row is two consecutive columns per lane, four lanes fill a 32-byte sector
+    float *Yb = Y + (size_t)split * ((size_t)M * N);
+    const bool v2 = ((reinterpret_cast<uintptr_t>(Yb) & 7) == 0) && (N & 1) == 0;
+#pragma unroll
+    for (int i = 0; i < TM; i++) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int m = m0 + wm * 16 * TM + 16 * i + 8 * h + g;
+            if (m < mend) {
+                float *yr = Yb + (size_t)m * N;
+#pragma unroll
+                for (int j = 0; j < TN; j++) {
+                    const int n = n0 + wn * 8 * TN + 8 * j + 2 * t;
+                    float lo, hi;
+                    unpack2(acc[i][j][h], lo, hi);
+                    if (v2 && n + 1 < N) *reinterpret_cast<float2 *>(yr + n) = make_float2(lo, hi);
+                    else {
+                        if (n < N) yr[n] = lo;
+                        if (n + 1 < N) yr[n + 1] = hi;
+                    }
+                }
+            }
+        }
+    }
+}
+
+// ---- host side ------------------------------------------------------------------------------------
+template <class C, typename ST, bool GROUPED>
+inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int M, int N, int K, int nsplit,
+                    int gsplit, cudaStream_t st, const GroupList &gl = GroupList(), int max_items = 0) {
+    auto kern = gemm_w4a8_mma_kernel<C, ST, GROUPED>;
+    static PerDevice<bool> configured_dev;              // the opt-in is a per-device function attribute
+    bool &configured = configured_dev.get();
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+        if (e != cudaSuccess) return cuda_fail(e, "gemm_mma smem opt-in");
+        configured = true;
+    }
+    const int m_tiles = (M + C::BM - 1) / C::BM, n_tiles = (N + C::BN - 1) / C::BN, nb = K / QBLK;
+    const bool vec = nb % GPK == 0 && (GROUPED || gsplit % GPK == 0 || nsplit == 1) && aligned(xs, 16) && aligned(sw, 4 * sizeof(ST));
+    const long units = GROUPED ? (long)max_items * n_tiles : (long)m_tiles * n_tiles * nsplit;
+    if (units > 0x7FFFFFFFL) return fail(W4A8_ERR_UNSUPPORTED, "gemm: %ld work units", units);
+    kern<<<(unsigned)units, C::THREADS, C::SMEM, st>>>(X, xs, Wq, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, vec, gl);
+    return launch_status("gemm_w4a8_mma");
+}
+
+using Cfg128 = Cfg<4, 8, 2, 2, 4, 2>;                       // 128 x 128, four warps of 64 x 64, two CTAs per SM
+template <int TM>
+using CfgRows = Cfg<TM, 4, 1, 4, 4, TM == 1 ? 4 : 3>;       // 16 TM x 128, four warps side by side, three (four) CTAs per SM
+
+// Which kernel and tile a dense product takes.  Up to 64 rows always a tile of the rows rounded up to 16 (a 128-row tile
+// computes its dead rows too: 5120 x 17408, 40 rows, 51.8 us against 83.2 on tcgen05 and 123 with 128 x 128 tiles here).
+// Above that the padding of the last row tile, the number of CTAs left over for the last wave and the rate of each kind
+// of tile decide; all three follow from the counts and the time a tile needs per group of K with 1, 2, 3 of its kind on
+// an SM, measured over nine shapes between 96 x 4096 x 4096 and 2048 x 17408 x 5120 (ns):
+//   tcgen05 128 x 128  505 (one per SM)      here 128 x 128  570, 920      48 x 128  320, 500, 700      64 x 128  380, 620, 970
+// The sum over waves reproduces those nine to 6 % and picks the fastest of the four on each of them, for example 333 x 15360:
+// 48 rows (165 us; tcgen05 192), 333 x 6000: tcgen05 (69; 48 rows 87), 512 x 17408: 128 x 128 (310; tcgen05 333).
+enum class Tile { TC, T128, R48, R64 };
+inline Tile pick(long M, long N, int nsplit) {
+    struct Kind { Tile tile; int rows, per_sm; long ns[3]; };
+    static const Kind kinds[4] = {{Tile::TC, 128, 1, {505, 0, 0}}, {Tile::T128, 128, 2, {570, 920, 0}},
+                                  {Tile::R48, 48, 3, {320, 500, 700}}, {Tile::R64, 64, 3, {380, 620, 970}}};
+    const long sms = sm_count(), n_tiles = (N + 127) / 128 * nsplit;
+    Tile best = Tile::TC;
+    long best_ns = 0;
+    for (const Kind &k : kinds) {
+        const long ctas = (M + k.rows - 1) / k.rows * n_tiles, wave = sms * k.per_sm, rest = ctas % wave;
+        const long ns = ctas / wave * k.ns[k.per_sm - 1] + (rest ? k.ns[(rest + sms - 1) / sms - 1] : 0);
+        if (best_ns == 0 || ns < best_ns) { best = k.tile; best_ns = ns; }
+    }
+    return best;
+}
+
+template <typename ST>
+inline int launch_t(const int8_t *X, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int M, int N, int K, int nsplit,
+                    int gsplit, cudaStream_t st) {
+    if (M <= 16) return launch_c<CfgRows<1>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+    if (M <= 32) return launch_c<CfgRows<2>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+    if (M <= 48) return launch_c<CfgRows<3>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+    if (M <= 64) return launch_c<CfgRows<4>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+    switch (pick(M, N, nsplit)) {
+        case Tile::T128: return launch_c<Cfg128, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+        case Tile::R48: return launch_c<CfgRows<3>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+        case Tile::R64: return launch_c<CfgRows<4>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+        default: break;
+    }
+    return gemm::launch_tc_t<ST, false>(X, xs, Wq, sw, Y, nullptr, M, N, K, nsplit, gsplit, st, OutArgs());
+}
+
+// nsplit = 1: Y is the output.  nsplit > 1: Y is the [nsplit][M][N] partial-sum workspace and gsplit the number of groups
+// per split (a split without groups stores zeros).  X and Wq 16-byte aligned; the caller checks.
+inline int launch(const int8_t *X, const float *xs, const uint8_t *Wq, const void *sw, float *Y, int M, int N, int K, int scale_dtype,
+                  int nsplit, int gsplit, cudaStream_t st) {
+    if (scale_dtype == 1) return launch_t<__half>(X, xs, Wq, (const __half *)sw, Y, M, N, K, nsplit, gsplit, st);
+    return launch_t<float>(X, xs, Wq, (const float *)sw, Y, M, N, K, nsplit, gsplit, st);
+}
+
+// Grouped experts, as gemm::launch_tc_grouped: Y[sorted row, n] for the rows the item list names.
+inline int launch_grouped(const int8_t *X, const float *xs, const uint8_t *Wq, const void *sw, float *Y, int rows, int N, int K,
+                          int scale_dtype, const GroupList &gl, int max_items, cudaStream_t st) {
+    using C = CfgRows<4>;
+    static_assert(C::BM == gemm::BNG, "an item's rows are one tile");
+    if (scale_dtype == 1) return launch_c<C, __half, true>(X, xs, Wq, (const __half *)sw, Y, rows, N, K, 1, K / QBLK, st, gl, max_items);
+    return launch_c<C, float, true>(X, xs, Wq, (const float *)sw, Y, rows, N, K, 1, K / QBLK, st, gl, max_items);
+}
+
+}  // namespace gemm_mma
+}  // namespace w4a8

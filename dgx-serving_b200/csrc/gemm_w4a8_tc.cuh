@@ -719,15 +719,6 @@ inline int launch_tc_e(const int8_t *X, const float *xs, const uint8_t *Wq, cons
     return launch_status("gemm_w4a8_tc");
 }
 
-// Grouped experts: Y[sorted row, n] for the rows and experts the item list names (rows of experts without an item,
-// and rows no item covers, are not written).  Same arithmetic per (row, expert) as launch_tc.
-inline int launch_tc_grouped(const int8_t *X, const float *xs, const uint8_t *Wq, const void *sw, float *Y, int rows, int N, int K,
-                             int scale_dtype, int experts, const GroupList &gl, int max_items, cudaStream_t st) {
-    if (scale_dtype == 1)
-        return launch_tc_e<__half, false, 2, false, true>(X, xs, Wq, (const __half *)sw, Y, nullptr, rows, N, K, 1, K / QBLK, st, OutArgs(), gl, experts, max_items);
-    return launch_tc_e<float, false, 2, false, true>(X, xs, Wq, (const float *)sw, Y, nullptr, rows, N, K, 1, K / QBLK, st, OutArgs(), gl, experts, max_items);
-}
-
 // Needs X and Wq 16-byte aligned (TMA global address rule); the caller checks.
 // Epilogue arithmetic variant (see epi_chunk): all variants give identical bits.  W4A8_GEMM_EPI overrides the
 // default for measurements (0 cvt, 1 magic-number conversion, 2 cvt + f32x2, 3 magic + f32x2).

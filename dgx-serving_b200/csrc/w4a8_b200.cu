@@ -17,6 +17,7 @@
 #include "gemv_w4a8_tc.cuh"
 #include "gemm_w4a8_tc.cuh"
 #include "gemm_w4a8_tcf.cuh"
+#include "gemm_w4a8_mma.cuh"
 #include "moe_w4a8.cuh"
 
 namespace w4a8 {
@@ -238,8 +239,8 @@ static int gemv_dispatch(const int8_t *xq, const float *xs, const uint8_t *Wq, c
     return launch_gemv(xq, xs, Wq, sw, Y, IN, OUT, S, scale_dtype, st, oa_in);
 }
 
-// GEMM kernel policy: 0 = fp16-operand tensor-core kernel (kind::f16, exact float group dots), 1 = int8-operand kernel
-// (kind::i8, int32 group dots).  Same results bit for bit.  Environment W4A8_GEMM = f16 | i8.
+// GEMM kernel policy: 0 = fp16-operand tensor-core kernel (kind::f16, exact float group dots), 1 = int8-operand kernels
+// (int32 group dots; gemm_mma::launch picks mma.sync or tcgen05 kind::i8 by size).  Same results bit for bit.  Environment W4A8_GEMM = f16 | i8.
 static int g_gemm_policy = -1;
 static int gemm_policy() {
     if (g_gemm_policy < 0) {
@@ -250,7 +251,7 @@ static int gemm_policy() {
 }
 static int gemm_launch(const int8_t *X, const float *xs, const uint8_t *Wq, const void *sw, float *Y, int M, int N, int K,
                        int scale_dtype, int nsplit, int gsplit, cudaStream_t st) {
-    if (gemm_policy() == 1) return gemm::launch_tc(X, xs, Wq, sw, Y, M, N, K, scale_dtype, nsplit, gsplit, st, OutArgs());
+    if (gemm_policy() == 1) return gemm_mma::launch(X, xs, Wq, sw, Y, M, N, K, scale_dtype, nsplit, gsplit, st);
     return gemmf::launch(X, xs, Wq, sw, Y, M, N, K, scale_dtype, nsplit, gsplit, st);
 }
 
