@@ -105,17 +105,29 @@ def _check(rc):
 
 
 def _ptr(t):
-    if t is None:
-        return None
-    if isinstance(t, int):
+    if t is None or isinstance(t, int):
         return t
     return t.data_ptr()
 
 
+_raw_stream = None
+
+
 def _stream(stream):
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        # the handle of torch's current stream of the current device.  torch.cuda.current_stream() builds a Stream object
+        # around it on every call, a good part of what a one-row launch costs on the host.
+        global _raw_stream
+        if _raw_stream is None:
+            import torch
+            handle = torch.cuda.current_stream().cuda_stream          # initialises CUDA
+            device, raw = getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
+            if device is None or raw is None:
+                _raw_stream = lambda: torch.cuda.current_stream().cuda_stream
+            else:
+                _raw_stream = lambda: raw(device())
+            return handle
+        return _raw_stream()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
