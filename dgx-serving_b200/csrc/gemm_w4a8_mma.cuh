@@ -75,7 +75,15 @@ struct Cfg {
     static constexpr int RB = (BN + THREADS - 1) / THREADS, RA = (BM + THREADS - 1) / THREADS;   // scale rows per thread
 };
 
-using gemm::GroupList;
+// Grouped experts: the activation rows are sorted by expert, item i of the list says "expert x, sorted rows [y, y + z)" with
+// z <= ITEM_ROWS (one item per 64-row tile of an expert, written on the device by moe_sort_kernel), the weights are the
+// flat [experts * N][K/2] tensor of the reference (kernels/moe_fused.cuh:21-24: expert e starts e * N rows in), and one
+// unit of work is (item, 128 of the expert's N outputs).
+constexpr int ITEM_ROWS = 64;
+struct GroupList {
+    const int4 *items = nullptr;
+    const int *num_items = nullptr;
+};
 
 template <class C, typename ST, bool GROUPED>
 __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
@@ -352,11 +360,11 @@ inline int launch(const int8_t *X, const float *xs, const uint8_t *Wq, const voi
     return launch_t<float>(X, xs, Wq, (const float *)sw, Y, M, N, K, nsplit, gsplit, st);
 }
 
-// Grouped experts, as gemm::launch_tc_grouped: Y[sorted row, n] for the rows the item list names.
+// Grouped experts: Y[sorted row, n] for the rows and experts the item list names (rows no item covers are not written).
 inline int launch_grouped(const int8_t *X, const float *xs, const uint8_t *Wq, const void *sw, float *Y, int rows, int N, int K,
                           int scale_dtype, const GroupList &gl, int max_items, cudaStream_t st) {
     using C = CfgRows<4>;
-    static_assert(C::BM == gemm::BNG, "an item's rows are one tile");
+    static_assert(C::BM == ITEM_ROWS, "an item's rows are one tile");
     if (scale_dtype == 1) return launch_c<C, __half, true>(X, xs, Wq, (const __half *)sw, Y, rows, N, K, 1, K / QBLK, st, gl, max_items);
     return launch_c<C, float, true>(X, xs, Wq, (const float *)sw, Y, rows, N, K, 1, K / QBLK, st, gl, max_items);
 }

@@ -34,7 +34,6 @@ namespace w4a8 {
 namespace gemm {
 
 constexpr int BM = 128, BN = 128, KT = 128;
-static_assert(BM == BN, "the grouped (transposed) instantiation exchanges the operands' roles");
 constexpr int GPK = KT / QBLK;  // groups (MMAs) per K-tile = 4
 #ifndef W4A8_GEMM_SA
 #define W4A8_GEMM_SA 4
@@ -70,10 +69,7 @@ constexpr int OFF_B8 = OFF_A + SA * A_STAGE;
 constexpr int OFF_BP = OFF_B8 + S8 * B8_STAGE;
 constexpr int OFF_SW = OFF_BP + SB * BP_STAGE;
 constexpr int OFF_BAR = OFF_SW + SS * SW_STAGE;
-constexpr int BNG = 64;          // GROUPED: accumulator columns per group = most rows of an item (MMA N); 8 buffers of 64 columns,
-                                 // i.e. two K-tiles of accumulators in tensor memory: K-tile j+1's MMAs run while j is fetched
-constexpr int KD = 12;           // K-tile-done ring (GROUPED): a multiple of SA and S8, deeper than any role can lag
-constexpr int NUM_BARS = 2 * (SA + SB + S8 + SS + TB) + KD;
+constexpr int NUM_BARS = 2 * (SA + SB + S8 + SS + TB);
 constexpr int OFF_TMEM = OFF_BAR + NUM_BARS * 8;
 constexpr int SMEM_BYTES = OFF_TMEM + 16 + 1024;  // + slack to align the base to 1024 B
 
@@ -156,26 +152,6 @@ __device__ __forceinline__ void epi_chunk(const uint32_t (&d)[NC], float x, cons
         }
     }
 }
-// The same arithmetic with the roles of the two scales exchanged (grouped experts: lane = weight row, column = token):
-// xs[j] belongs to column j, sw16 to the lane.  t = (float)d * xs (rounded), acc = fma(t, sw16, acc): the same operations
-// on the same values as epi_chunk, so the same bits.
-template <int NC>
-__device__ __forceinline__ void epi_chunk_t(const uint32_t (&d)[NC], const float *__restrict__ xs, float sw16, uint64_t (&acc2)[NC / 2]) {
-    // accumulators stay packed two to a 64-bit register across groups; the tokens' scales are read as packed pairs
-    const uint64_t ss = pack_f32x2(sw16, sw16);
-#pragma unroll
-    for (int j4 = 0; j4 < NC / 4; j4++) {
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(xs + j4 * 4);   // {xs[4j4], xs[4j4+1]}, {xs[4j4+2], xs[4j4+3]}
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int j = j4 * 4 + 2 * h;
-            const uint64_t f2 = pack_f32x2(__int2float_rn((int)d[j]), __int2float_rn((int)d[j + 1]));
-            uint64_t t2;
-            asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(t2) : "l"(f2), "l"(h == 0 ? x.x : x.y));
-            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc2[j / 2]) : "l"(t2), "l"(ss));
-        }
-    }
-}
 // Four consecutive scales of one row (one K-tile's worth) with one load; the address must be aligned to the
 // size of the load.
 __device__ __forceinline__ void load_scales4(const float *p, float (&v)[4]) {
@@ -200,43 +176,19 @@ __device__ __forceinline__ void epi_dump(const uint32_t (&d)[NC], int32_t *__res
     }
 }
 
-// Grouped experts (GROUPED instantiation): the activation rows are sorted by expert, item i of the list says
-// "expert x, sorted rows [y, y + z)" with z <= BNG (one item per 64-row tile of an expert, written on the device by
-// moe_sort_kernel), the weights are the flat [experts * N][K/2] tensor of the reference (kernels/moe_fused.cuh:21-24:
-// expert e starts e * N rows in), and one unit of work is (item, 128 of the expert's N outputs).
-struct GroupList {
-    const int4 *items = nullptr;
-    const int *num_items = nullptr;
-};
-
 // One unit of work = (output tile, K split).  Tiles are numbered M-fastest so that CTAs running at the
 // same time share weight tiles in L2; split s covers groups [s*gsplit, min(nb, (s+1)*gsplit)).
-// Rows [m0, mend) of the tile are live; wrow0 is added to a column index to get its row in the weight tensor.
+// Rows [m0, mend) of the tile are live.
 struct Work {
-    int m0, mend, n0, wrow0, g0, g1, nkt, split;
+    int m0, mend, n0, g0, g1, nkt, split;
 };
-template <bool GROUPED>
-__device__ __forceinline__ Work decode_work(int w, int m_tiles, int num_tiles, int nb, int gsplit, int M, int N, int n_tiles,
-                                            const GroupList &gl) {
+__device__ __forceinline__ Work decode_work(int w, int m_tiles, int num_tiles, int nb, int gsplit, int M) {
     Work k;
-    if (GROUPED) {
-        const int4 it = __ldg(gl.items + w / n_tiles);
-        k.split = 0;
-        k.m0 = it.y;
-        k.mend = it.y + it.z;
-        k.n0 = (w % n_tiles) * BN;      // consecutive units share an item: its activation tile stays in L2
-        k.wrow0 = it.x * N;
-        k.g0 = 0;
-        k.g1 = nb;
-        k.nkt = (nb + GPK - 1) / GPK;
-        return k;
-    }
     const int tile = w % num_tiles;
     k.split = w / num_tiles;
     k.m0 = (tile % m_tiles) * BM;
     k.mend = M;
     k.n0 = (tile / m_tiles) * BN;
-    k.wrow0 = 0;
     k.g0 = k.split * gsplit;
     k.g1 = min(nb, k.g0 + gsplit);
     const int ng = max(0, k.g1 - k.g0);
@@ -247,11 +199,11 @@ __device__ __forceinline__ Work decode_work(int w, int m_tiles, int num_tiles, i
 // PEER (N-sharded weights, no split-K): every output tile is stored straight into EVERY rank's Y[M, ld] at its final
 // columns (oa.col0 + n: plain 16-byte peer stores over NVLink) and the last CTA publishes the step's epoch, so the
 // all-gather costs no extra pass over the outputs (peer_allgather.cuh).
-template <typename ST, bool DUMP, int EPI, bool PEER = false, bool GROUPED = false>
+template <typename ST, bool DUMP, int EPI, bool PEER = false>
 __global__ void __launch_bounds__(THREADS, 1) gemm_w4a8_tc_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     const float *__restrict__ xs, const ST *__restrict__ sw, float *__restrict__ Y, int32_t *__restrict__ Dout,
-    int M, int N, int K, int nsplit, int gsplit, const OutArgs oa, const GroupList gl) {
+    int M, int N, int K, int nsplit, int gsplit, const OutArgs oa) {
     extern __shared__ unsigned char smem_dyn[];
     const uint32_t raw = ptx::smem_u32(smem_dyn);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -262,14 +214,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_w4a8_tc_kernel(
     // barrier index map
     constexpr int A_FULL = 0, A_EMPTY = A_FULL + SA, BP_FULL = A_EMPTY + SA, BP_EMPTY = BP_FULL + SB,
                   B8_FULL = BP_EMPTY + SB, B8_EMPTY = B8_FULL + S8, SW_FULL = B8_EMPTY + S8, SW_EMPTY = SW_FULL + SS,
-                  TM_FULL = SW_EMPTY + SS, TM_EMPTY = TM_FULL + TB, KT_DONE = TM_EMPTY + TB;
-    // GROUPED: ONE tcgen05.commit per K-tile instead of six (accumulator ready x 4, activation stage free, operand stage
-    // free).  K-tile j of the CTA (counted across work units, the same in every role) commits to KT_DONE[j % KD]; whoever
-    // needs "the MMAs of K-tile j have completed" waits for parity (j / KD) & 1 — the epilogue for its accumulators, the
-    // producer and the expansion warps for the stages K-tile j read.  The epilogue then fetches all of a K-tile's live
-    // columns in one go and hands the four accumulator buffers back together (MoE block at M = 512: 555 -> 530 us).
-    constexpr bool KT_COMMIT = GROUPED;
-    auto kt_done_wait = [&](int j) { return ptx::mbar_wait(BAR(KT_DONE + j % KD), (uint32_t)(j / KD) & 1u); };
+                  TM_FULL = SW_EMPTY + SS, TM_EMPTY = TM_FULL + TB;
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(base_ptr + OFF_TMEM);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -277,7 +222,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_w4a8_tc_kernel(
     const bool scales_aligned = ((reinterpret_cast<uintptr_t>(xs) & 15) == 0) && ((reinterpret_cast<uintptr_t>(sw) & (4 * sizeof(ST) - 1)) == 0);
     const int m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
     const int num_tiles = m_tiles * n_tiles;
-    const int num_work = GROUPED ? *gl.num_items * n_tiles : num_tiles * nsplit;
+    const int num_work = num_tiles * nsplit;
 
     if (tid == 0) {
         for (int i = 0; i < SA; i++) { ptx::mbar_init(BAR(A_FULL + i), 1); ptx::mbar_init(BAR(A_EMPTY + i), 1); }
@@ -285,7 +230,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_w4a8_tc_kernel(
         for (int i = 0; i < S8; i++) { ptx::mbar_init(BAR(B8_FULL + i), DEQ_WARPS); ptx::mbar_init(BAR(B8_EMPTY + i), 1); }
         for (int i = 0; i < SS; i++) { ptx::mbar_init(BAR(SW_FULL + i), DEQ_WARPS); ptx::mbar_init(BAR(SW_EMPTY + i), EPI_WARPS); }
         for (int i = 0; i < TB; i++) { ptx::mbar_init(BAR(TM_FULL + i), 1); ptx::mbar_init(BAR(TM_EMPTY + i), EPI_WARPS); }
-        for (int i = 0; i < KD; i++) ptx::mbar_init(BAR(KT_DONE + i), 1);
         ptx::mbar_fence_init();
         ptx::tma_prefetch_desc(&tmA);
         ptx::tma_prefetch_desc(&tmB);
@@ -304,19 +248,18 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_w4a8_tc_kernel(
         if (lane == 0) {
             Ring ra(SA), rb(SB);
             bool ok = true;
-            int kc = 0;
             for (int wi = blockIdx.x; wi < num_work && ok; wi += gridDim.x) {
-                const Work wk = decode_work<GROUPED>(wi, m_tiles, num_tiles, nb, gsplit, M, N, n_tiles, gl);
+                const Work wk = decode_work(wi, m_tiles, num_tiles, nb, gsplit, M);
                 const int m0 = wk.m0, n0 = wk.n0;
-                for (int kt = 0; kt < wk.nkt && ok; kt++, kc++) {
+                for (int kt = 0; kt < wk.nkt && ok; kt++) {
                     const int kbyte = (wk.g0 + kt * GPK) * QBLK;   // first K element of this K-tile (multiple of 32)
-                    if (KT_COMMIT ? (kc >= SA && !kt_done_wait(kc - SA)) : !ptx::mbar_wait(BAR(A_EMPTY + ra.stage), ra.phase ^ 1u)) { dev_set_error(ERR_PRODUCER | 1); ok = false; break; }
+                    if (!ptx::mbar_wait(BAR(A_EMPTY + ra.stage), ra.phase ^ 1u)) { dev_set_error(ERR_PRODUCER | 1); ok = false; break; }
                     ptx::mbar_arrive_expect_tx(BAR(A_FULL + ra.stage), A_STAGE);
                     ptx::tma_load_2d(base + OFF_A + ra.stage * A_STAGE, &tmA, kbyte, m0, BAR(A_FULL + ra.stage));
                     ra.advance();
                     if (!ptx::mbar_wait(BAR(BP_EMPTY + rb.stage), rb.phase ^ 1u)) { dev_set_error(ERR_PRODUCER | 2); ok = false; break; }
                     ptx::mbar_arrive_expect_tx(BAR(BP_FULL + rb.stage), BP_STAGE);
-                    ptx::tma_load_2d(base + OFF_BP + rb.stage * BP_STAGE, &tmB, kbyte / 2, wk.wrow0 + n0, BAR(BP_FULL + rb.stage));
+                    ptx::tma_load_2d(base + OFF_BP + rb.stage * BP_STAGE, &tmB, kbyte / 2, n0, BAR(BP_FULL + rb.stage));
                     rb.advance();
                 }
             }
@@ -329,35 +272,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_w4a8_tc_kernel(
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
             Ring ra(SA), r8(S8), rt(TB);
-            const uint32_t idesc = ptx::umma_idesc_s8(BM, BN), idesc_g = ptx::umma_idesc_s8(BN, BNG);
+            const uint32_t idesc = ptx::umma_idesc_s8(BM, BN);
             bool ok = true;
-            int kc = 0;
             for (int wi = blockIdx.x; wi < num_work && ok; wi += gridDim.x) {
-                const Work wk = decode_work<GROUPED>(wi, m_tiles, num_tiles, nb, gsplit, M, N, n_tiles, gl);
-                for (int kt = 0; kt < wk.nkt && ok; kt++, kc++) {
+                const Work wk = decode_work(wi, m_tiles, num_tiles, nb, gsplit, M);
+                for (int kt = 0; kt < wk.nkt && ok; kt++) {
                     if (!ptx::mbar_wait(BAR(A_FULL + ra.stage), ra.phase)) { dev_set_error(ERR_MMA | 1); ok = false; break; }
                     if (!ptx::mbar_wait(BAR(B8_FULL + r8.stage), r8.phase)) { dev_set_error(ERR_MMA | 2); ok = false; break; }
                     ptx::tc_fence_after_sync();
                     const uint64_t adesc = ptx::umma_desc_k_sw128(base + OFF_A + ra.stage * A_STAGE);
                     const uint64_t bdesc = ptx::umma_desc_k_sw128(base + OFF_B8 + r8.stage * B8_STAGE);
                     const int ng = min(GPK, wk.g1 - (wk.g0 + kt * GPK));
-                    if (KT_COMMIT) {
-                        // K-tile kc uses the accumulator half kc & 1 (GPK buffers of BNG columns); wait until the epilogue has
-                        // fetched the K-tile that used it before (kc - 2), then the K-tile's MMAs back to back and ONE commit
-                        const int half = kc & 1;
-                        if (!ptx::mbar_wait(BAR(TM_EMPTY + half), ((uint32_t)(kc >> 1) & 1u) ^ 1u)) { dev_set_error(ERR_MMA | 3); ok = false; break; }
-                        ptx::tc_fence_after_sync();
-                        for (int g = 0; g < ng; g++) {
-                            // the expanded weights are the MMA's A operand (accumulator lanes = weight rows), the activations
-                            // its B operand (columns = tokens, BNG of them): an expert's tile has few live tokens, and the
-                            // epilogue's work follows the live COLUMNS while all 128 lanes stay busy
-                            ptx::umma_i8(tmem_base + (half * GPK + g) * BNG, bdesc + (uint64_t)(g * 2), adesc + (uint64_t)(g * 2), idesc_g, 0u);
-                        }
-                        ptx::umma_commit(BAR(KT_DONE + kc % KD));
-                        ra.advance();
-                        r8.advance();
-                        continue;
-                    }
                     for (int g = 0; g < ng; g++) {
                         if (!ptx::mbar_wait(BAR(TM_EMPTY + rt.stage), rt.phase ^ 1u)) { dev_set_error(ERR_MMA | 3); ok = false; break; }
                         ptx::tc_fence_after_sync();
@@ -378,26 +303,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_w4a8_tc_kernel(
         const int dt = tid - 64;  // 0..DEQ_WARPS*32-1
         Ring rb(SB), r8(S8), rs(SS);
         bool ok = true;
-        int kc = 0;
         for (int wi = blockIdx.x; wi < num_work && ok; wi += gridDim.x) {
-            const Work wk = decode_work<GROUPED>(wi, m_tiles, num_tiles, nb, gsplit, M, N, n_tiles, gl);
+            const Work wk = decode_work(wi, m_tiles, num_tiles, nb, gsplit, M);
             const int n0 = wk.n0;
-            if (GROUPED && dt == 0 && scales_aligned) {
-                // An expert's scales are touched by this CTA only, so every K-tile's scale loads would wait for HBM (with
-                // dense weights another CTA has usually brought them into L2).  The scale rows of a unit are one contiguous
-                // block each: ask for the NEXT unit's blocks now (and for this CTA's first unit at its start).
-                auto prefetch_unit = [&](const Work &u) {
-                    const int nrows = min(BN, N - u.n0), mrows = u.mend - u.m0;
-                    const uint32_t wbytes = (uint32_t)((size_t)nrows * nb * sizeof(ST)) & ~15u, xbytes = (uint32_t)((size_t)mrows * nb * 4) & ~15u;
-                    const ST *wp = sw + (size_t)(u.wrow0 + u.n0) * nb;
-                    const float *xp = xs + (size_t)u.m0 * nb;
-                    if (wbytes && (reinterpret_cast<uintptr_t>(wp) & 15) == 0) ptx::prefetch_l2_bulk(wp, wbytes);
-                    if (xbytes && (reinterpret_cast<uintptr_t>(xp) & 15) == 0) ptx::prefetch_l2_bulk(xp, xbytes);
-                };
-                if (wi == (int)blockIdx.x) prefetch_unit(wk);
-                if (wi + (int)gridDim.x < num_work) prefetch_unit(decode_work<GROUPED>(wi + gridDim.x, m_tiles, num_tiles, nb, gsplit, M, N, n_tiles, gl));
-            }
-            for (int kt = 0; kt < wk.nkt && ok; kt++, kc++) {
+            for (int kt = 0; kt < wk.nkt && ok; kt++) {
                 // ---- this K-tile's scales: issue the loads first, they complete behind the expansion below.
                 // A row's GPK scales are contiguous in memory: one 16-byte (fp32) or 8-byte (fp16) load per row
                 // when the K-tile is complete and the addresses line up, else element by element.
@@ -411,7 +320,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_w4a8_tc_kernel(
 #pragma unroll
                     for (int g = 0; g < GPK; g++) vw[r][g] = 0.f;
                     if (!DUMP && n < N) {
-                        const ST *swrow = sw + (size_t)(wk.wrow0 + n) * nb;
+                        const ST *swrow = sw + (size_t)n * nb;
                         if (vec) load_scales4(swrow + b0, vw[r]);
                         else {
 #pragma unroll
@@ -436,8 +345,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_w4a8_tc_kernel(
                 }
 
                 // ---- expansion of the packed stage into the operand stage
-                bool w = ptx::mbar_wait_warp(BAR(BP_FULL + rb.stage), rb.phase) && (KT_COMMIT ? (kc < S8 || ptx::mbar_wait_warp(BAR(KT_DONE + (kc - S8) % KD), (uint32_t)((kc - S8) / KD) & 1u))
-                                                                                                   : ptx::mbar_wait_warp(BAR(B8_EMPTY + r8.stage), r8.phase ^ 1u));
+                bool w = ptx::mbar_wait_warp(BAR(BP_FULL + rb.stage), rb.phase) && ptx::mbar_wait_warp(BAR(B8_EMPTY + r8.stage), r8.phase ^ 1u);
                 if (!w) { dev_set_error(ERR_DEQUANT | 1); ok = false; break; }
                 const unsigned char *src = base_ptr + OFF_BP + rb.stage * BP_STAGE;
                 unsigned char *dst = base_ptr + OFF_B8 + r8.stage * B8_STAGE;
@@ -492,99 +400,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_w4a8_tc_kernel(
         const int col0 = (ew >> 2) * EPI_COLS;  // this warp's accumulator columns [col0, col0 + EPI_COLS)
         Ring rs(SS), rt(TB);
         bool ok = true;
-        if (GROUPED) {
-            // Transposed accumulator: lanes are weight rows (all 128 live), columns are the item's tokens (z <= BNG live, 32
-            // on average).  The 4 warps that share a quad of lanes deal the live columns out in chunks of CW: warp group cg
-            // takes chunks cg and cg + 4, so that at z = 32 every one of the 16 warps converts and scales 8 columns per
-            // group.  A K-tile's accumulators (one half of tensor memory) are handed back once all of its groups have been
-            // fetched; the other half is being written by the next K-tile's MMAs meanwhile.
-            constexpr int CW = 8, CK = BNG / (4 * CW);     // 2 chunks of 8 columns per warp at most
-            const int cg = ew >> 2;
-            int kce = 0;                                   // K-tiles of this CTA so far (the index every role counts)
-            for (int wi = blockIdx.x; wi < num_work && ok; wi += gridDim.x) {
-                const Work wk = decode_work<GROUPED>(wi, m_tiles, num_tiles, nb, gsplit, M, N, n_tiles, gl);
-                const int z = wk.mend - wk.m0;
-                const int nlive = z > CW * cg ? (z - CW * cg - 1) / (4 * CW) + 1 : 0;   // chunk k covers columns CW*(cg + 4k) ...
-                const int n = wk.n0 + quad * 32 + lane;
-                uint64_t acc[CK][CW / 2];                              // packed pairs of fp32 accumulators
-#pragma unroll
-                for (int k = 0; k < CK; k++)
-#pragma unroll
-                    for (int j = 0; j < CW / 2; j++) acc[k][j] = 0ull;
-                const int ngroups = wk.g1 - wk.g0;
-                for (int gi = 0; gi < ngroups; gi += GPK) {             // one K-tile = up to GPK groups = one commit
-                    const int ngk = min(GPK, ngroups - gi);
-                    if (!ptx::mbar_wait_warp(BAR(SW_FULL + rs.stage), rs.phase)) { dev_set_error(ERR_EPILOGUE | 1); ok = false; break; }
-                    const float *stage = reinterpret_cast<const float *>(base_ptr + OFF_SW + rs.stage * SW_STAGE);
-                    if (!ptx::mbar_wait_warp(BAR(KT_DONE + kce % KD), (uint32_t)(kce / KD) & 1u)) { dev_set_error(ERR_EPILOGUE | 2); ok = false; break; }
-                    ptx::tc_fence_after_sync();
-                    const int half = kce & 1;
-                    kce++;
-                    const uint32_t tl = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * GPK * BNG + CW * cg);
-                    // Fetches are issued in batches of four chunks (32 registers) with one wait per batch, the K-tile's half of
-                    // tensor memory is handed back after the last fetch, and the loops are fully unrolled per case (one or two
-                    // chunks per group): the epilogue is bound by its instruction count, not by the arithmetic in it.
-                    auto release = [&]() {
-                        ptx::tc_fence_before_sync();
-                        __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive(BAR(TM_EMPTY + half));
-                    };
-                    const float *xs0 = stage + GPK * BN + CW * cg;          // + g * BM (+ 4 * CW for the second chunk)
-                    const float *sw0 = stage + quad * 32 + lane;            // + g * BN
-                    uint32_t d[4][CW];
-                    if (nlive == 0) {
-                        release();
-                    } else if (nlive == 1) {
-#pragma unroll
-                        for (int g = 0; g < GPK; g++)
-                            if (g < ngk) ptx::tmem_ld(tl + g * BNG, d[g]);
-                        ptx::tmem_ld_wait();
-                        release();
-#pragma unroll
-                        for (int g = 0; g < GPK; g++)
-                            if (g < ngk) epi_chunk_t<CW>(d[g], xs0 + g * BM, sw0[g * BN], acc[0]);
-                    } else {
-#pragma unroll
-                        for (int h = 0; h < GPK / 2; h++) {                 // groups 2h and 2h + 1, both chunks of each
-                            const int g0 = 2 * h, g1 = 2 * h + 1;
-                            if (g0 < ngk) { ptx::tmem_ld(tl + g0 * BNG, d[0]); ptx::tmem_ld(tl + g0 * BNG + 4 * CW, d[1]); }
-                            if (g1 < ngk) { ptx::tmem_ld(tl + g1 * BNG, d[2]); ptx::tmem_ld(tl + g1 * BNG + 4 * CW, d[3]); }
-                            ptx::tmem_ld_wait();
-                            if (h == GPK / 2 - 1) release();
-                            if (g0 < ngk) {
-                                const float swl = sw0[g0 * BN];
-                                epi_chunk_t<CW>(d[0], xs0 + g0 * BM, swl, acc[0]);
-                                epi_chunk_t<CW>(d[1], xs0 + g0 * BM + 4 * CW, swl, acc[1]);
-                            }
-                            if (g1 < ngk) {
-                                const float swl = sw0[g1 * BN];
-                                epi_chunk_t<CW>(d[2], xs0 + g1 * BM, swl, acc[0]);
-                                epi_chunk_t<CW>(d[3], xs0 + g1 * BM + 4 * CW, swl, acc[1]);
-                            }
-                            if (h == 0) ptx::tc_fence_after_sync();
-                        }
-                    }
-                    __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(BAR(SW_EMPTY + rs.stage));
-                    rs.advance();
-                }
-                if (!ok) break;
-                if (n < N) {   // consecutive lanes write consecutive floats of a row of Y
-#pragma unroll
-                    for (int k = 0; k < CK; k++)
-#pragma unroll
-                        for (int j = 0; j < CW; j += 2) {
-                            const int col = CW * (cg + 4 * k) + j;
-                            float lo, hi;
-                            unpack_f32x2(acc[k][j / 2], lo, hi);
-                            if (k < nlive && col < z) Y[(size_t)(wk.m0 + col) * N + n] = lo;
-                            if (k < nlive && col + 1 < z) Y[(size_t)(wk.m0 + col + 1) * N + n] = hi;
-                        }
-                }
-            }
-        }
-        for (int wi = blockIdx.x; !GROUPED && wi < num_work && ok; wi += gridDim.x) {
-            const Work wk = decode_work<GROUPED>(wi, m_tiles, num_tiles, nb, gsplit, M, N, n_tiles, gl);
+        for (int wi = blockIdx.x; wi < num_work && ok; wi += gridDim.x) {
+            const Work wk = decode_work(wi, m_tiles, num_tiles, nb, gsplit, M);
             const int m0 = wk.m0, n0 = wk.n0;
             const int m = m0 + quad * 32 + lane;
             // a warp whose 32 rows all lie beyond M only keeps the barriers moving
@@ -693,18 +510,15 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restr
 }
 
 // ---- host side ------------------------------------------------------------------------------------
-// experts > 0: grouped launch (GROUPED instantiation): M = sorted activation rows, N = outputs per expert, Wq / sw the
-// flat tensors of `experts` experts, gl the item list; max_items bounds the list's length (grid size only).
-template <typename ST, bool DUMP, int EPI, bool PEER = false, bool GROUPED = false>
+template <typename ST, bool DUMP, int EPI, bool PEER = false>
 inline int launch_tc_e(const int8_t *X, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int32_t *D,
-                       int M, int N, int K, int nsplit, int gsplit, cudaStream_t st, const OutArgs &oa,
-                       const GroupList &gl = GroupList(), int experts = 0, int max_items = 0) {
+                       int M, int N, int K, int nsplit, int gsplit, cudaStream_t st, const OutArgs &oa) {
     CUtensorMap tmA, tmB;
     int rc = make_tmap_u8(&tmA, X, (uint64_t)K, (uint64_t)M, KT, BM, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != W4A8_OK) return rc;
-    rc = make_tmap_u8(&tmB, Wq, (uint64_t)K / 2, (uint64_t)N * (GROUPED ? experts : 1), KT / 2, BN, CU_TENSOR_MAP_SWIZZLE_NONE);
+    rc = make_tmap_u8(&tmB, Wq, (uint64_t)K / 2, (uint64_t)N, KT / 2, BN, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc != W4A8_OK) return rc;
-    auto kern = gemm_w4a8_tc_kernel<ST, DUMP, EPI, PEER, GROUPED>;
+    auto kern = gemm_w4a8_tc_kernel<ST, DUMP, EPI, PEER>;
     static PerDevice<bool> configured_dev;              // the opt-in is a per-device function attribute
     bool &configured = configured_dev.get();
     if (!configured) {
@@ -712,10 +526,10 @@ inline int launch_tc_e(const int8_t *X, const float *xs, const uint8_t *Wq, cons
         if (e != cudaSuccess) return cuda_fail(e, "gemm smem opt-in");
         configured = true;
     }
-    const long tiles = GROUPED ? (long)max_items * ((N + BN - 1) / BN) : (long)((M + BM - 1) / BM) * ((N + BN - 1) / BN) * nsplit;
+    const long tiles = (long)((M + BM - 1) / BM) * ((N + BN - 1) / BN) * nsplit;
     const int sms = sm_count();
     const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
-    kern<<<grid, THREADS, SMEM_BYTES, st>>>(tmA, tmB, xs, sw, Y, D, M, N, K, nsplit, gsplit, PEER ? oa : OutArgs(), gl);
+    kern<<<grid, THREADS, SMEM_BYTES, st>>>(tmA, tmB, xs, sw, Y, D, M, N, K, nsplit, gsplit, PEER ? oa : OutArgs());
     return launch_status("gemm_w4a8_tc");
 }
 

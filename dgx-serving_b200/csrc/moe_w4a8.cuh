@@ -24,7 +24,7 @@ namespace w4a8 {
 namespace moe {
 
 constexpr int MAX_EXPERTS = 1024;
-constexpr int TILE_ROWS = gemm::BNG;   // rows per item of the grouped GEMM = its accumulator's columns
+constexpr int TILE_ROWS = gemm_mma::ITEM_ROWS;   // rows per item of the grouped GEMM
 
 // Byte offsets of the block's intermediates inside the caller's workspace (all 256-byte aligned).
 struct Layout {
@@ -364,7 +364,7 @@ inline int launch_experts(const BlockArgs &a, const Buffers &b, bool use_gemm, l
         moe_gather_rows_kernel<<<gg, 128, 0, st>>>(b.xq, b.xs, b.perm, b.offsets + a.experts, a.topk, a.H, b.xq_g, b.xs_g);
         rc = launch_status("moe_gather_rows");
         if (rc != W4A8_OK) return rc;
-        gemm::GroupList gl;
+        gemm_mma::GroupList gl;
         gl.items = b.items; gl.num_items = b.num_items;
         rc = gemm_mma::launch_grouped(b.xq_g, b.xs_g, a.gu_wq, a.gu_sc, b.gu, nslots, 2 * a.MI, a.H, a.scale_dtype, gl, b.max_items, st);
         if (rc != W4A8_OK) return rc;
