@@ -116,15 +116,17 @@ __device__ __forceinline__ float quant_scale(float amax) {
     return amax / 127.0f;
 }
 // Four quantized activations of one float4: q = rintf(x / d) clamped to +-127 (kernels/quantize_x.cuh:36-37), packed into
-// one word (byte i = q_i), and their sum.  The quotient is at most 127 * (1 + 2^-23) in magnitude because |x| <= amax
-// and d = amax / 127 rounded, so the clamp never changes a finite value: one cvt.rni.sat.s8.f32 per element does
-// round-to-nearest-even, the conversion and the saturation (a NaN quotient — amax infinite — gives 0 either way).
+// one word (byte i = q_i).  cvt.rni.sat.s8.f32 rounds to nearest even, converts and saturates (a NaN quotient — amax
+// infinite, or 0 / 0 — gives 0 either way); the saturation stops at -128 and the definition at -127.  While d is a normal
+// number the quotient is at most 127 * (1 + 2^-23) in magnitude, because |x| <= amax and d = amax / 127 rounded; a subnormal
+// d is rounded so coarsely that it reaches 190, so the lower bound is taken here, on the path that all such d take.
+__device__ __forceinline__ int quantize1_div(float x, float d) {
+    int q;
+    asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(q) : "f"(x / d));
+    return max(q, -127);
+}
 __device__ __noinline__ uint32_t quantize4_div(float4 v, float d) {
-    int q0, q1, q2, q3;
-    asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(q0) : "f"(v.x / d));
-    asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(q1) : "f"(v.y / d));
-    asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(q2) : "f"(v.z / d));
-    asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(q3) : "f"(v.w / d));
+    const int q0 = quantize1_div(v.x, d), q1 = quantize1_div(v.y, d), q2 = quantize1_div(v.z, d), q3 = quantize1_div(v.w, d);
     const uint32_t lo = __byte_perm((uint32_t)q0, (uint32_t)q1, 0x0040), hi = __byte_perm((uint32_t)q2, (uint32_t)q3, 0x0040);
     return __byte_perm(lo, hi, 0x5410);
 }
@@ -132,8 +134,8 @@ __device__ __noinline__ uint32_t quantize4_div(float4 v, float d) {
 // r = 1/d to one ulp (rcp.approx: relative error at most 2^-23), m = fma(x, r, 1.5 * 2^23) holds the integer nearest to x*r
 // in its low byte, and t = x*r - q is its distance.  |x*r - x/d| <= 127 * 2^-23 = 1.6e-5 and the fp32 quotient is within
 // 2^-18 = 3.8e-6 of x/d, so where |t| <= 0.5 - 2^-15 no half-integer lies between x*r and the fp32 quotient and both
-// round to the same q.  The other elements (about 6 in 10^5), d outside the range in which r keeps its accuracy, and
-// anything that is not finite take the divisions.
+// round to the same q, at most 127 in magnitude.  The other elements (about 6 in 10^5), d outside the range in which r keeps
+// its accuracy, and anything that is not finite take the divisions.
 __device__ __forceinline__ uint32_t quantize4_pack(float4 v, float d, int &sum) {
     constexpr float MAGIC = 12582912.0f, TIE = 0.5f - 0x1p-15f;
     float r;
