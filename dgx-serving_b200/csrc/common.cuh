@@ -22,13 +22,16 @@ inline int fail(int code, const char *fmt, ...) {
     va_end(ap);
     return code;
 }
+// The caller learns of e from the return code, so it must not stay behind as the thread's last error, where the next
+// call's launch_status would report it for a launch that succeeded.
 inline int cuda_fail(cudaError_t e, const char *what) {
+    cudaGetLastError();
     return fail(W4A8_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 // After a kernel launch: reports launch-configuration errors without synchronising.
 inline int launch_status(const char *what) {
     cudaError_t e = cudaPeekAtLastError();
-    if (e != cudaSuccess) { cudaGetLastError(); return cuda_fail(e, what); }
+    if (e != cudaSuccess) return cuda_fail(e, what);
     return W4A8_OK;
 }
 inline bool aligned(const void *p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
