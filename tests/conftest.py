@@ -56,3 +56,28 @@ def cuda():
 def to_dev(a, dev):
     import torch
     return torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+
+
+def launched_kernels(call):
+    """Mangled names of the kernels that call(stream) launches, in launch order: the call is captured, not run."""
+    import torch
+    from cuda.bindings import driver as D
+
+    def ok(r):
+        assert r[0] == D.CUresult.CUDA_SUCCESS, r[0]
+        return r[1] if len(r) == 2 else r[1:]
+
+    stream = torch.cuda.Stream()
+    ok(D.cuStreamBeginCapture(stream.cuda_stream, D.CUstreamCaptureMode.CU_STREAM_CAPTURE_MODE_THREAD_LOCAL))
+    try:
+        call(stream.cuda_stream)
+    finally:
+        graph = ok(D.cuStreamEndCapture(stream.cuda_stream))
+    names = []
+    count = ok(D.cuGraphGetNodes(graph, 0))[1]
+    for node in ok(D.cuGraphGetNodes(graph, count))[0]:
+        if ok(D.cuGraphNodeGetType(node)) == D.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            p = ok(D.cuGraphKernelNodeGetParams(node))
+            names.append(ok(D.cuFuncGetName(p.func) if int(p.func) else D.cuKernelGetName(p.kern)).decode())
+    ok(D.cuGraphDestroy(graph))
+    return names
