@@ -1,7 +1,8 @@
 // W4A8 prefill / verify / grouped-expert GEMM whose group dots never leave the register file.
 //   Y[m,n] = sum_b ((float)D[m,n,b] * xs[m,b]) * sw[n,b],   D[m,n,b] = sum_{k in group b} X[m,k]*(Wq[n,k]-8)
 // Same semantics and fp32 order as gemm_w4a8_tc.cuh (t = (float)D*xs rounded, acc = fma(t, sw, acc), groups ascending:
-// the reference's kernels/gemm_mmq.cuh:104-105), hence the same bits.
+// the reference's kernels/gemm_mmq.cuh:104-105), hence the same bits.  The dots come out 16 times too large (unpack8_x16);
+// the 1/16 goes into the weight scale, as there, where it is exact from 2^-122 up whatever the activation scale is.
 //
 // What bounds it.  Both operands carry a scale per 32-element group, so whatever computes the dots, every (m, n, group)
 // costs a conversion, a multiply and an fma on the CUDA cores.  On tcgen05 the dots come out in tensor memory and every
@@ -203,8 +204,8 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
                     const uint2 v0 = *reinterpret_cast<const uint2 *>(As + bg * C::A_GROUP + i * 512), v1 = *reinterpret_cast<const uint2 *>(As + bg * C::A_GROUP + i * 512 + 256);
                     split_even_odd(v0.x, v0.y, a[i][0], a[i][2]);
                     split_even_odd(v1.x, v1.y, a[i][1], a[i][3]);
-                    xx[bg & 1][i][0] = *reinterpret_cast<const float *>(sx + bg * 4 + (16 * i) * (GPK * 4)) * 0.0625f;         // exact 1/16
-                    xx[bg & 1][i][1] = *reinterpret_cast<const float *>(sx + bg * 4 + (16 * i + 8) * (GPK * 4)) * 0.0625f;
+                    xx[bg & 1][i][0] = *reinterpret_cast<const float *>(sx + bg * 4 + (16 * i) * (GPK * 4));
+                    xx[bg & 1][i][1] = *reinterpret_cast<const float *>(sx + bg * 4 + (16 * i + 8) * (GPK * 4));
                 }
             }
             uint32_t b0, b1;
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
         for (int q = 0; q < NG * TN; q++) {
             if (q + 1 < NG * TN) start(q + 1);
             const int bg = q / TN, j = q % TN;
-            const uint64_t s2 = pack2(sv[q & 1][0], sv[q & 1][1]);
+            const uint64_t s2 = mul2(pack2(sv[q & 1][0], sv[q & 1][1]), pack2(0.0625f, 0.0625f));
 #pragma unroll
             for (int i = 0; i < L; i++) {
                 const int (&d)[4] = c[q & 1][i];

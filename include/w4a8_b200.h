@@ -78,7 +78,10 @@ int w4a8_device_status(uint32_t *detail);
  *                  kind::i8, whichever the sizes make faster; 0 = operands converted to fp16 on the way into shared
  *                  memory (every int4 and int8 value is exact in fp16), tcgen05.mma kind::f16 with fp32
  *                  accumulation of one 32-element group, which is exact as well (|sum| <= 32*127*8 < 2^24).
- *                  Both give the same bits.
+ *                  Both give the same bits.  (This and every other equality of bits between kernels and with the
+ *                  reference holds for fp32 weight scales that are zero or between 2^-122 and 2^108 in magnitude, and where
+ *                  a GEMV takes part for activation scales in that range too: the kernels that expand a weight to 16
+ *                  times its value fold the 1/16 into one of the scales.)
  *   "moe_kernel":  w4a8_moe_block's expert products: 0 = by slot count (default), 1 = grouped GEMV, 2 = sorted grouped
  *                  tensor-core GEMM. */
 int w4a8_config(const char *key, int value);

@@ -85,3 +85,29 @@ def test_gemm_tiles_split_k(w4a8, oracle, cuda, sms148, M, N, K, splitk, rows, s
     torch.cuda.synchronize()
     assert tile_rows(launched_kernels(call)) == rows
     assert np.array_equal(Y.cpu().numpy().view(np.uint32), oracle.gemm_splitk_w4a8(*host, splitk).view(np.uint32))
+
+
+@pytest.mark.parametrize("scale_dtype", [0, 1])
+@pytest.mark.parametrize("kernel", [0, 1])
+@pytest.mark.parametrize("M,N,K,rows", [(16, 130, 256, 16), (17, 130, 640, 32), (48, 130, 256, 48), (64, 130, 512, 64), (49, 131, 544, 0),
+                                        (193, 7700, 128, 0), (2048, 2047, 128, 128)])
+def test_tiny_activation_scales(w4a8, oracle, cuda, sms148, M, N, K, rows, kernel, scale_dtype):
+    """Activation scales down to a few multiples of the smallest subnormal: a factor folded into them would lose bits, and the
+    tile that M and N select would show in the result."""
+    import torch
+    (xq, xs, Wq, sw), _ = operands(oracle, cuda, M, N, K, 0, 17)
+    rng = np.random.default_rng(18)
+    xs = np.ldexp(rng.uniform(1, 4, xs.shape), rng.integers(-146, -115, (M, 1))).astype(np.float32)
+    sw = (sw * 1000).astype(np.float16 if scale_dtype else np.float32)
+    d = [torch.from_numpy(np.ascontiguousarray(a)).to(cuda) for a in (xq, xs, Wq, sw)]
+    Y = torch.empty((M, N), dtype=torch.float32, device=cuda)
+    w4a8.config("gemm_kernel", kernel)
+    try:
+        def call(stream):
+            w4a8.launch_gemm_mmq_w4a8(d[0], d[1], d[2], d[3], Y, M, N, K, scale_dtype, stream)
+        call(None)
+        w4a8.device_status()
+        assert kernel == 0 or tile_rows(launched_kernels(call)) == rows
+    finally:
+        w4a8.config("gemm_kernel", 1)
+    assert np.array_equal(Y.cpu().numpy().view(np.uint32), oracle.gemm_mmq_w4a8(xq, xs, Wq, sw).view(np.uint32))
