@@ -74,6 +74,7 @@ struct Cfg {
     static constexpr int OFF_SX = GPK * (A_GROUP + B_GROUP), OFF_SW = OFF_SX + BM * GPK * 4;      // scales: [row][group]
     static constexpr int STAGE = OFF_SW + BN * GPK * 4, SMEM = STAGES * STAGE;
     static constexpr int RB = (BN + THREADS - 1) / THREADS, RA = (BM + THREADS - 1) / THREADS;   // scale rows per thread
+    static_assert(CTAS * (SMEM + 1024) <= 228 * 1024, "CTAS of these do not fit an SM's shared memory (1 KB each is the system's)");
 };
 
 // Grouped experts: the activation rows are sorted by expert, item i of the list says "expert x, sorted rows [y, y + z)" with
@@ -304,22 +305,26 @@ inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const S
 }
 
 using Cfg128 = Cfg<4, 8, 2, 2, 4, 2>;                       // 128 x 128, four warps of 64 x 64, two CTAs per SM
+// 16 TM x 128, four warps side by side, three (four) CTAs per SM.  64 rows: three stages instead of four, with which only two
+// CTAs would fit (expert block, 128 experts, 512 rows 308 us with four, 283 with three; 128 rows 239 and 204; dense
+// 160 x 17408 x 5120 183 and 135).  A grid that leaves one CTA to an SM has nothing but the ring to cover its loads: four.
 template <int TM>
-using CfgRows = Cfg<TM, 4, 1, 4, 4, TM == 1 ? 4 : 3>;       // 16 TM x 128, four warps side by side, three (four) CTAs per SM
+using CfgRows = Cfg<TM, 4, 1, 4, TM == 4 ? 3 : 4, TM == 1 ? 4 : 3>;
+using Cfg64Deep = Cfg<4, 4, 1, 4, 4, 2>;                    // 112 x 7000 x 3840: 43.2 us, with three stages 45.1
 
 // Which kernel and tile a dense product takes.  Up to 64 rows always a tile of the rows rounded up to 16 (a 128-row tile
 // computes its dead rows too: 5120 x 17408, 40 rows, 51.8 us against 83.2 on tcgen05 and 123 with 128 x 128 tiles here).
 // Above that the padding of the last row tile, the number of CTAs left over for the last wave and the rate of each kind
 // of tile decide; all three follow from the counts and the time a tile needs per group of K with 1, 2, 3 of its kind on
 // an SM, measured over nine shapes between 96 x 4096 x 4096 and 2048 x 17408 x 5120 (ns):
-//   tcgen05 128 x 128  505 (one per SM)      here 128 x 128  570, 920      48 x 128  320, 500, 700      64 x 128  380, 620, 970
+//   tcgen05 128 x 128  505 (one per SM)      here 128 x 128  570, 920      48 x 128  320, 500, 700      64 x 128  370, 590, 820
 // The sum over waves reproduces those nine to 6 % and picks the fastest of the four on each of them, for example 333 x 15360:
 // 48 rows (165 us; tcgen05 192), 333 x 6000: tcgen05 (69; 48 rows 87), 512 x 17408: 128 x 128 (310; tcgen05 333).
 enum class Tile { TC, T128, R48, R64 };
 inline Tile pick(long M, long N, int nsplit) {
     struct Kind { Tile tile; int rows, per_sm; long ns[3]; };
     static const Kind kinds[4] = {{Tile::TC, 128, 1, {505, 0, 0}}, {Tile::T128, 128, 2, {570, 920, 0}},
-                                  {Tile::R48, 48, 3, {320, 500, 700}}, {Tile::R64, 64, 3, {380, 620, 970}}};
+                                  {Tile::R48, 48, 3, {320, 500, 700}}, {Tile::R64, 64, 3, {370, 590, 820}}};
     const long sms = sm_count(), n_tiles = (N + 127) / 128 * nsplit;
     Tile best = Tile::TC;
     long best_ns = 0;
@@ -343,11 +348,16 @@ inline int launch_t(const int8_t *X, const float *xs, const uint8_t *Wq, const S
     if (M <= 16) return launch_c<CfgRows<1>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
     if (M <= 32) return launch_c<CfgRows<2>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
     if (M <= 48) return launch_c<CfgRows<3>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
-    if (M <= 64) return launch_c<CfgRows<4>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+    const auto rows64 = [&]() {
+        if ((long)((M + 63) / 64) * ((N + 127) / 128) * nsplit <= sm_count())
+            return launch_c<Cfg64Deep, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+        return launch_c<CfgRows<4>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+    };
+    if (M <= 64) return rows64();
     switch (pick(M, N, nsplit)) {
         case Tile::T128: return launch_c<Cfg128, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
         case Tile::R48: return launch_c<CfgRows<3>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
-        case Tile::R64: return launch_c<CfgRows<4>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+        case Tile::R64: return rows64();
         default: break;
     }
     return gemm::launch_tc_t<ST, false>(X, xs, Wq, sw, Y, nullptr, M, N, K, nsplit, gsplit, st, OutArgs());

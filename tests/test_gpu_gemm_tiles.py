@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 # (M, N, K, rows of the tile, 0: tcgen05).  K / 32 is a multiple of four in the first list: scales copied 16 (8) bytes at a time.
 LINED_UP = [(1, 8, 128, 16), (16, 129, 256, 16), (17, 130, 640, 32), (32, 300, 512, 32), (33, 128, 1152, 48), (48, 257, 256, 48),
-            (49, 131, 640, 64), (64, 384, 2048, 64), (65, 200, 128, 48), (100, 130, 640, 48), (193, 4095, 256, 64), (130, 1000, 128, 48),
+            (49, 131, 640, 64), (64, 384, 2048, 64), (65, 200, 128, 48), (100, 130, 640, 48), (193, 4095, 256, 64), (150, 17401, 384, 64), (130, 1000, 128, 48),
             (193, 7700, 128, 0), (2047, 2046, 128, 128), (2048, 2047, 640, 128)]
 # ... and not here: element by element, wherever more than two CTAs per SM cover those loads
 ELEMENTWISE = [(1, 8, 32, 16), (16, 129, 96, 16), (9, 40, 1120, 16), (17, 37889, 288, 32), (33, 37889, 544, 48), (49, 37890, 544, 64),
@@ -23,7 +23,7 @@ ELEMENTWISE = [(1, 8, 32, 16), (16, 129, 96, 16), (9, 40, 1120, 16), (17, 37889,
                (17, 40, 160, 0), (33, 128, 1120, 0), (49, 131, 544, 0), (64, 384, 2080, 0), (96, 520, 288, 0)]
 # (M, N, K, splits, rows of the tile)
 SPLIT_K = [(64, 1, 2048, 8, 64), (24, 258, 1024, 3, 32), (48, 12801, 960, 3, 48), (20, 9600, 288, 4, 32), (64, 5000, 1120, 8, 64), (3, 130, 1120, 3, 16),
-           (100, 8000, 480, 3, 128), (48, 130, 1120, 3, 0), (20, 300, 160, 4, 0), (70, 256, 480, 2, 0)]
+           (100, 8000, 480, 3, 64), (48, 130, 1120, 3, 0), (20, 300, 160, 4, 0), (70, 256, 480, 2, 0)]
 
 
 def tile_rows(names):
