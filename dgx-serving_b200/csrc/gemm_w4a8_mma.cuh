@@ -21,9 +21,11 @@
 // LDS.32, no conflicts); groups are 32 bytes further apart than they need, which makes the copies' writes conflict-free
 // too.  A lane's word of weights expands to its two B registers with three logic operations (unpack8_x16: even and odd
 // elements), the matching A registers are two byte permutes of eight activations.  Any order of K inside a group gives
-// the same integer.  Scales travel with their K-tile, [row][group], one 16-byte
-// piece per row (element by element where rows of scales are not a multiple of four or not aligned).  One __syncthreads per
-// K-tile; two or three CTAs per SM cover each other's.
+// the same integer.  Scales travel with their K-tile, [row][group], one 16-byte (fp16: 8-byte) piece per row where they line
+// up, that is where K / 32 and every range of a split K are multiples of four and the pointers aligned (VEC); 4 bytes at a
+// time otherwise, and fp16 scales of an odd K / 32, whose rows start between two words, by plain loads.  Plain loads of all
+// scales stall their warp once per K-tile, which cost more than the kernel gains over tcgen05: 700 x 9000 x 5024 321 us with
+// them, 246 on tcgen05.  One __syncthreads per K-tile; two or three CTAs per SM cover each other's.
 #pragma once
 #include <type_traits>
 #include "common.cuh"
@@ -39,6 +41,9 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool l
 }
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -87,12 +92,15 @@ struct GroupList {
     const int *num_items = nullptr;
 };
 
-template <class C, typename ST, bool GROUPED>
+template <class C, typename ST, bool GROUPED, bool VEC>
 __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     const int8_t *__restrict__ X, const float *__restrict__ xs, const uint8_t *__restrict__ Wq, const ST *__restrict__ sw,
-    float *__restrict__ Y, int M, int N, int K, int m_tiles, int n_tiles, int gsplit, bool vec_scales, const GroupList gl) {
+    float *__restrict__ Y, int M, int N, int K, int m_tiles, int n_tiles, int gsplit, bool pairs, const GroupList gl) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int TM = C::TM, TN = C::TN, BM = C::BM, BN = C::BN, NT = C::THREADS, STAGES = C::STAGES;
+    // Scales that line up make every K-tile complete.  Known at compile time that is worth 1 to 10 % (fewer instructions), except
+    // where ptxas then spills: 64 rows at three CTAs per SM, 28 bytes and 6 % slower.
+    constexpr bool FULL = VEC && !(TM * TN == 16 && C::CTAS == 3);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int wm = warp % C::WM, wn = warp / C::WM;
     const int nb = K / QBLK;
@@ -115,7 +123,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     const int nkt = (g1 - g0 + GPK - 1) / GPK;
 
     // ---- copies: thread -> 16-byte chunk of a row (8 of 128 bytes of activations, 4 of 64 bytes of weights).  Rows past
-    // the end re-read the last one and are never stored; chunks past the last group are skipped and never read.
+    // the end are filled with zeros (their scales are the last row's) and never stored; chunks past the last group are skipped.
     constexpr int AI = (BM * 8 + NT - 1) / NT, BI = (BN * 4 + NT - 1) / NT;
     static_assert(BM * 8 % NT == 0 && BN * 4 % NT == 0, "whole copy instructions");
     const uint32_t smem_u = (uint32_t)__cvta_generic_to_shared(smem);
@@ -127,8 +135,45 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     const uint32_t bdst = smem_u + GPK * C::A_GROUP + cb * C::B_GROUP + (tid >> 2) * 16;
     auto copy = [&](int kt) {
         if (kt < nkt) {
-            const int b0 = g0 + kt * GPK, ng = g1 - b0;          // groups left
+            const int b0 = g0 + kt * GPK, ng = FULL ? GPK : g1 - b0;          // groups left
             const uint32_t so = (uint32_t)(kt % STAGES) * C::STAGE;
+            // scales: a row's GPK of them are one 16-byte (fp16: 8-byte) piece when they line up, else 4 bytes at a time.  Ahead of
+            // the operands, so that fewer addresses are live at once: 333 x 15360 x 3840, fp16, 163 us, behind them 169.
+#pragma unroll
+            for (int r = 0; r < C::RA; r++) {
+                const int m = tid + r * NT;
+                if (BM % NT == 0 || m < BM) {
+                    const float *p = xs + (size_t)min(m0 + m, mend - 1) * nb + b0;
+                    const uint32_t o = so + C::OFF_SX + m * (GPK * 4);
+                    if (VEC) cp_async16(smem_u + o, p, true);
+                    else {
+#pragma unroll
+                        for (int q = 0; q < GPK; q++)
+                            if (q < ng) cp_async4(smem_u + o + 4 * q, p + q);
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < C::RB; r++) {
+                const int n = tid + r * NT;
+                if (BN % NT == 0 || n < BN) {
+                    const ST *p = sw + (wrow0 + min(n0 + n, N - 1)) * (size_t)nb + b0;
+                    const uint32_t o = so + C::OFF_SW + n * (GPK * 4);
+                    if (VEC) {
+                        if (sizeof(ST) == 4) cp_async16(smem_u + o, p, true);
+                        else cp_async8(smem_u + o, p);
+                    } else if (sizeof(ST) == 4 || pairs) {               // pairs: the number of groups is even, so words never straddle the end
+                        constexpr int PER = 4 / sizeof(ST);
+#pragma unroll
+                        for (int q = 0; q < GPK; q += PER)
+                            if (q < ng) cp_async4(smem_u + o + sizeof(ST) * q, p + q);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < GPK; q++)
+                            if (q < ng) *reinterpret_cast<ST *>(smem + o + sizeof(ST) * q) = p[q];
+                    }
+                }
+            }
             if ((ca >> 1) < ng) {
                 const int8_t *src = Xb + (size_t)b0 * 32;
 #pragma unroll
@@ -143,34 +188,6 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
                 for (int i = 0; i < BI; i++) {
                     const bool live = i * (NT / 4) < rows_b;
                     cp_async16(bdst + so + i * (NT / 4) * 16, live ? src + (size_t)i * (NT / 4) * (K / 2) : Wq, live);
-                }
-            }
-            // scales: a row's GPK of them are one 16-byte (fp16: 8-byte) piece when they line up, else element by element
-            const bool vec = vec_scales && ng >= GPK;
-#pragma unroll
-            for (int r = 0; r < C::RA; r++) {
-                const int m = tid + r * NT;
-                if (BM % NT == 0 || m < BM) {
-                    const float *p = xs + (size_t)min(m0 + m, mend - 1) * nb + b0;
-                    const uint32_t o = so + C::OFF_SX + m * (GPK * 4);
-                    if (vec) cp_async16(smem_u + o, p, true);
-                    else
-                        for (int q = 0; q < GPK; q++)
-                            if (q < ng) *reinterpret_cast<float *>(smem + o + 4 * q) = p[q];
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < C::RB; r++) {
-                const int n = tid + r * NT;
-                if (BN % NT == 0 || n < BN) {
-                    const ST *p = sw + (wrow0 + min(n0 + n, N - 1)) * (size_t)nb + b0;
-                    const uint32_t o = so + C::OFF_SW + n * (GPK * 4);
-                    if (vec) {
-                        if (sizeof(ST) == 4) cp_async16(smem_u + o, p, true);
-                        else cp_async8(smem_u + o, p);
-                    } else
-                        for (int q = 0; q < GPK; q++)
-                            if (q < ng) *reinterpret_cast<ST *>(smem + o + sizeof(ST) * q) = p[q];
                 }
             }
         }
@@ -240,9 +257,9 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
         __syncthreads();                              // ... and everybody's; K-tile kt - 1 is done with
         copy(kt + STAGES - 1);                        // into the slot K-tile kt - 1 used
         const unsigned char *stage = smem + (kt % STAGES) * C::STAGE;
-        const int ng = min(GPK, g1 - (g0 + kt * GPK));
+        const int ng = FULL ? GPK : min(GPK, g1 - (g0 + kt * GPK));
         auto ktile = [&](auto LT) {
-            if (ng == GPK) groups(LT, std::integral_constant<int, GPK>(), stage, 0);
+            if (FULL || ng == GPK) groups(LT, std::integral_constant<int, GPK>(), stage, 0);
             else {
 #pragma unroll 1
                 for (int b = 0; b < ng; b++) groups(LT, std::integral_constant<int, 1>(), stage, b);
@@ -285,10 +302,20 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
 }
 
 // ---- host side ------------------------------------------------------------------------------------
-template <class C, typename ST, bool GROUPED>
+// A K-tile's scales are one aligned piece of each row.
+template <typename ST>
+inline bool scales_line_up(const float *xs, const ST *sw, int K, int nsplit, int gsplit) {
+    return (K / QBLK) % GPK == 0 && (nsplit == 1 || gsplit % GPK == 0) && aligned(xs, 16) && aligned(sw, 4 * sizeof(ST));
+}
+// The number of groups and every range of them is even, so that two fp16 scales are one aligned word.
+template <typename ST>
+inline bool scales_pair_up(const ST *sw, int K, int nsplit, int gsplit) {
+    return (K / QBLK) % 2 == 0 && (nsplit == 1 || gsplit % 2 == 0) && aligned(sw, 4);
+}
+template <class C, typename ST, bool GROUPED, bool VEC>
 inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int M, int N, int K, int nsplit,
                     int gsplit, cudaStream_t st, const GroupList &gl = GroupList(), int max_items = 0) {
-    auto kern = gemm_w4a8_mma_kernel<C, ST, GROUPED>;
+    auto kern = gemm_w4a8_mma_kernel<C, ST, GROUPED, VEC>;
     static PerDevice<bool> configured_dev;              // the opt-in is a per-device function attribute
     bool &configured = configured_dev.get();
     if (!configured) {
@@ -296,11 +323,11 @@ inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const S
         if (e != cudaSuccess) return cuda_fail(e, "gemm_mma smem opt-in");
         configured = true;
     }
-    const int m_tiles = (M + C::BM - 1) / C::BM, n_tiles = (N + C::BN - 1) / C::BN, nb = K / QBLK;
-    const bool vec = nb % GPK == 0 && (GROUPED || gsplit % GPK == 0 || nsplit == 1) && aligned(xs, 16) && aligned(sw, 4 * sizeof(ST));
+    const int m_tiles = (M + C::BM - 1) / C::BM, n_tiles = (N + C::BN - 1) / C::BN;
+    const bool pairs = scales_pair_up(sw, K, nsplit, gsplit);
     const long units = GROUPED ? (long)max_items * n_tiles : (long)m_tiles * n_tiles * nsplit;
     if (units > 0x7FFFFFFFL) return fail(W4A8_ERR_UNSUPPORTED, "gemm: %ld work units", units);
-    kern<<<(unsigned)units, C::THREADS, C::SMEM, st>>>(X, xs, Wq, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, vec, gl);
+    kern<<<(unsigned)units, C::THREADS, C::SMEM, st>>>(X, xs, Wq, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs, gl);
     return launch_status("gemm_w4a8_mma");
 }
 
@@ -310,28 +337,41 @@ using Cfg128 = Cfg<4, 8, 2, 2, 4, 2>;                       // 128 x 128, four w
 // 160 x 17408 x 5120 183 and 135).  A grid that leaves one CTA to an SM has nothing but the ring to cover its loads: four.
 template <int TM>
 using CfgRows = Cfg<TM, 4, 1, 4, TM == 4 ? 3 : 4, TM == 1 ? 4 : 3>;
-using Cfg64Deep = Cfg<4, 4, 1, 4, 4, 2>;                    // 112 x 7000 x 3840: 43.2 us, with three stages 45.1
+using Cfg64Deep = Cfg<4, 4, 1, 4, 4, 2>;                    // 112 x 7000 x 3840: 41.1 us, with three stages 43.1
 
-// Which kernel and tile a dense product takes.  Up to 64 rows always a tile of the rows rounded up to 16 (a 128-row tile
-// computes its dead rows too: 5120 x 17408, 40 rows, 51.8 us against 83.2 on tcgen05 and 123 with 128 x 128 tiles here).
-// Above that the padding of the last row tile, the number of CTAs left over for the last wave and the rate of each kind
-// of tile decide; all three follow from the counts and the time a tile needs per group of K with 1, 2, 3 of its kind on
-// an SM, measured over nine shapes between 96 x 4096 x 4096 and 2048 x 17408 x 5120 (ns):
-//   tcgen05 128 x 128  505 (one per SM)      here 128 x 128  570, 920      48 x 128  320, 500, 700      64 x 128  370, 590, 820
-// The sum over waves reproduces those nine to 6 % and picks the fastest of the four on each of them, for example 333 x 15360:
-// 48 rows (165 us; tcgen05 192), 333 x 6000: tcgen05 (69; 48 rows 87), 512 x 17408: 128 x 128 (310; tcgen05 333).
-enum class Tile { TC, T128, R48, R64 };
-inline Tile pick(long M, long N, int nsplit) {
-    struct Kind { Tile tile; int rows, per_sm; long ns[3]; };
-    static const Kind kinds[4] = {{Tile::TC, 128, 1, {505, 0, 0}}, {Tile::T128, 128, 2, {570, 920, 0}},
-                                  {Tile::R48, 48, 3, {320, 500, 700}}, {Tile::R64, 64, 3, {370, 590, 820}}};
-    const long sms = sm_count(), n_tiles = (N + 127) / 128 * nsplit;
+// Which kernel and tile a dense product takes.  The padding of the last row tile, the number of CTAs left over for the last
+// wave and the rate of each kind of tile decide; all three follow from the counts and the time a tile needs per group of K
+// with 1, 2, 3, 4 of its kind on an SM.  ns: those times, fitted to 13700 timings over M = 8 .. 2048, N = 256 .. 40000 and
+// K = 2048 .. 17408, for scales that line up, fp32 scales that are copied 4 bytes at a time, pairs of fp16 scales, and fp16
+// scales of an odd K / 32 (plain loads, a latency per K-tile that company on the SM hides).  tcgen05 adds 4 us a wave where N
+// is not a multiple of four: its rows are then stored 4 bytes at a time, lane by lane in different rows; 3 us a wave separate it
+// from the other kinds' fit for fp32 scales that do not line up.  The sum over waves reproduces the timings to 2 to 8 %.  On
+// average over the four the choice is 0.1 to 0.5 % slower than the fastest kind (9 % at most); it is slower than tcgen05 by more than 3 % at one point of the 13700 (65 x 15360 x 2048, 48-row tiles, 4 %).
+// Measured, us, chosen kind / tcgen05: 40 x 17408 x 5120 47 / 80, 160 x 17408 x 5120 131 / 166, 333 x 15360 x 3840 158 / 187,
+// 512 x 17408 x 5120 296 / 327, 24 x 20000 x 4128 53 / 122; tcgen05 / 64 rows: 700 x 9000 x 5024 240 / 254, 128 x 17408 x 5120
+// 87 / 91.  16 and 32 rows were not timed above max_rows.  128 x 128 tiles with scales 4 bytes at a time were never the fastest
+// kind for fp32 scales and at most 7 % ahead for fp16, so there are none.
+enum class Tile { TC, T128, R16, R32, R48, R64 };
+enum Scales { LINED_UP, WORDS, PAIRS, HALVES };
+inline Tile pick(long M, long N, int K, int nsplit, int gsplit, Scales scales) {
+    struct Kind { Tile tile; int rows, per_sm; long ns[4][4], max_rows; };
+    static const Kind kinds[6] = {
+        {Tile::TC, 128, 1, {{485}, {475}, {560}, {570}}, 1L << 31},
+        {Tile::T128, 128, 2, {{510, 935}, {0}, {0}, {0}}, 1L << 31},
+        {Tile::R16, 16, 4, {{155, 295, 470, 630}, {180, 435, 555, 720}, {175, 390, 480, 640}, {350, 475, 655, 850}}, 16},
+        {Tile::R32, 32, 3, {{200, 375, 525}, {225, 390, 530}, {220, 370, 515}, {405, 510, 600}}, 128},
+        {Tile::R48, 48, 3, {{255, 460, 635}, {275, 490, 725}, {260, 500, 690}, {410, 585, 735}}, 1L << 31},
+        {Tile::R64, 64, 3, {{295, 535, 760}, {320, 545, 795}, {315, 545, 790}, {430, 625, 820}}, 1L << 31}};
+    const long sms = sm_count(), n_tiles = (N + 127) / 128 * nsplit, groups = nsplit > 1 ? gsplit : K / QBLK;
     Tile best = Tile::TC;
     long best_ns = 0;
     for (const Kind &k : kinds) {
+        const long *ns = k.ns[scales];
+        if (M > k.max_rows || ns[0] == 0) continue;
         const long ctas = (M + k.rows - 1) / k.rows * n_tiles, wave = sms * k.per_sm, rest = ctas % wave;
-        const long ns = ctas / wave * k.ns[k.per_sm - 1] + (rest ? k.ns[(rest + sms - 1) / sms - 1] : 0);
-        if (best_ns == 0 || ns < best_ns) { best = k.tile; best_ns = ns; }
+        long t = (ctas / wave * ns[k.per_sm - 1] + (rest ? ns[(rest + sms - 1) / sms - 1] : 0)) * groups;
+        if (k.tile == Tile::TC) t += (ctas + sms - 1) / sms * ((scales == WORDS ? 3000 : 0) + (N % 4 != 0 ? 4000 : 0));
+        if (best_ns == 0 || t < best_ns) { best = k.tile; best_ns = t; }
     }
     return best;
 }
@@ -339,26 +379,23 @@ inline Tile pick(long M, long N, int nsplit) {
 template <typename ST>
 inline int launch_t(const int8_t *X, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int M, int N, int K, int nsplit,
                     int gsplit, cudaStream_t st) {
-    // Rows of scales that are not a multiple of four groups (or not aligned) are staged element by element here, and with one
-    // or two tiles on an SM nothing covers those loads: 19 x 4484 x 4192 69.8 us against 69.4 on tcgen05, other such shapes up
-    // to 5 % slower.  With more tiles they are covered (478 x 5630 x 2400: 74 against 102).
-    const bool lines_up = (K / QBLK) % GPK == 0 && (nsplit == 1 || gsplit % GPK == 0) && aligned(xs, 16) && aligned(sw, 4 * sizeof(ST));
-    if (!lines_up && M > 16 && (long)((M + 63) / 64) * ((N + 127) / 128) * nsplit <= 2L * sm_count())
-        return gemm::launch_tc_t<ST, false>(X, xs, Wq, sw, Y, nullptr, M, N, K, nsplit, gsplit, st, OutArgs());
-    if (M <= 16) return launch_c<CfgRows<1>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
-    if (M <= 32) return launch_c<CfgRows<2>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
-    if (M <= 48) return launch_c<CfgRows<3>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
-    const auto rows64 = [&]() {
-        if ((long)((M + 63) / 64) * ((N + 127) / 128) * nsplit <= sm_count())
-            return launch_c<Cfg64Deep, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
-        return launch_c<CfgRows<4>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+    const bool lines_up = scales_line_up(xs, sw, K, nsplit, gsplit);
+    const Scales scales = lines_up ? LINED_UP : sizeof(ST) == 4 ? WORDS : scales_pair_up(sw, K, nsplit, gsplit) ? PAIRS : HALVES;
+    const auto run = [&](auto c) {
+        using C = decltype(c);
+        if (lines_up) return launch_c<C, ST, false, true>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+        return launch_c<C, ST, false, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
     };
-    if (M <= 64) return rows64();
-    switch (pick(M, N, nsplit)) {
-        case Tile::T128: return launch_c<Cfg128, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
-        case Tile::R48: return launch_c<CfgRows<3>, ST, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
-        case Tile::R64: return rows64();
-        default: break;
+    switch (pick(M, N, K, nsplit, gsplit, scales)) {
+        case Tile::T128: return launch_c<Cfg128, ST, false, true>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+        case Tile::R16: return run(CfgRows<1>());
+        case Tile::R32: return run(CfgRows<2>());
+        case Tile::R48: return run(CfgRows<3>());
+        case Tile::R64:
+            if (lines_up && (long)((M + 63) / 64) * ((N + 127) / 128) * nsplit <= sm_count())
+                return launch_c<Cfg64Deep, ST, false, true>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
+            return run(CfgRows<4>());
+        case Tile::TC: break;
     }
     return gemm::launch_tc_t<ST, false>(X, xs, Wq, sw, Y, nullptr, M, N, K, nsplit, gsplit, st, OutArgs());
 }
@@ -376,8 +413,13 @@ inline int launch_grouped(const int8_t *X, const float *xs, const uint8_t *Wq, c
                           int scale_dtype, const GroupList &gl, int max_items, cudaStream_t st) {
     using C = CfgRows<4>;
     static_assert(C::BM == ITEM_ROWS, "an item's rows are one tile");
-    if (scale_dtype == 1) return launch_c<C, __half, true>(X, xs, Wq, (const __half *)sw, Y, rows, N, K, 1, K / QBLK, st, gl, max_items);
-    return launch_c<C, float, true>(X, xs, Wq, (const float *)sw, Y, rows, N, K, 1, K / QBLK, st, gl, max_items);
+    const int gsplit = K / QBLK;
+    const auto run = [&](auto *w) {
+        using ST = std::remove_const_t<std::remove_pointer_t<decltype(w)>>;
+        if (scales_line_up(xs, w, K, 1, gsplit)) return launch_c<C, ST, true, true>(X, xs, Wq, w, Y, rows, N, K, 1, gsplit, st, gl, max_items);
+        return launch_c<C, ST, true, false>(X, xs, Wq, w, Y, rows, N, K, 1, gsplit, st, gl, max_items);
+    };
+    return scale_dtype == 1 ? run((const __half *)sw) : run((const float *)sw);
 }
 
 }  // namespace gemm_mma

@@ -1,9 +1,9 @@
 """Every tile of the register-resident GEMM (csrc/gemm_w4a8_mma.cuh) at the edges of its rows, columns and K, bit for bit
-against the oracle's MMQ order: 16- to 64-row tiles, 48- and 64-row tiles repeated, 128 x 128 tiles, rows, columns and K-tiles
-that end ragged, odd N (unpaired stores), rows of scales that are not a multiple of four through more K-tiles than the ring
-has stages, split K with ranges that are not, and with an empty last range; the few tiles with such scales that stay on the
-tcgen05 kernel too.  Each case names the kernel and tile the dispatch has to choose for it on 148 SMs, so that no later rule
-can leave one of them untested."""
+against the oracle's MMQ order: 16- to 64-row tiles alone and repeated, 128 x 128 tiles, rows, columns and K-tiles that end
+ragged, odd N (unpaired stores), the three ways of copying scales (K / 32 and the ranges of a split K multiples of four,
+even, odd) through more K-tiles than the ring has stages, split K with an empty last range, and shapes that stay on the
+tcgen05 kernel.  Each case names the kernel that the dispatch has to choose for it on 148 SMs, so that no later rule can
+leave one of them untested."""
 import re
 
 import numpy as np
@@ -13,28 +13,35 @@ from conftest import launched_kernels
 
 pytestmark = pytest.mark.gpu
 
-# (M, N, K, rows of the tile, 0: tcgen05).  K / 32 is a multiple of four in the first list: scales copied 16 (8) bytes at a time.
-LINED_UP = [(1, 8, 128, 16), (16, 129, 256, 16), (17, 130, 640, 32), (32, 300, 512, 32), (33, 128, 1152, 48), (48, 257, 256, 48),
-            (49, 131, 640, 64), (64, 384, 2048, 64), (65, 200, 128, 48), (100, 130, 640, 48), (193, 4095, 256, 64), (150, 17401, 384, 64), (130, 1000, 128, 48),
-            (193, 7700, 128, 0), (2047, 2046, 128, 128), (2048, 2047, 640, 128)]
-# ... and not here: element by element, wherever more than two CTAs per SM cover those loads
-ELEMENTWISE = [(1, 8, 32, 16), (16, 129, 96, 16), (9, 40, 1120, 16), (17, 37889, 288, 32), (33, 37889, 544, 48), (49, 37890, 544, 64),
-               (64, 38000, 672, 64), (129, 17408, 64, 48), (145, 23809, 288, 64), (2048, 2048, 160, 128), (2040, 2047, 544, 128),
-               (17, 40, 160, 0), (33, 128, 1120, 0), (49, 131, 544, 0), (64, 384, 2080, 0), (96, 520, 288, 0)]
-# (M, N, K, splits, rows of the tile)
-SPLIT_K = [(64, 1, 2048, 8, 64), (24, 258, 1024, 3, 32), (48, 12801, 960, 3, 48), (20, 9600, 288, 4, 32), (64, 5000, 1120, 8, 64), (3, 130, 1120, 3, 16),
-           (100, 8000, 480, 3, 64), (48, 130, 1120, 3, 0), (20, 300, 160, 4, 0), (70, 256, 480, 2, 0)]
+# The kernels: rows of the tile / stages of its ring, "e" where scales do not line up (VEC = false), "tc" for tcgen05.  A pair
+# where fp32 and fp16 scales differ.
+# (M, N, K, kernel); K / 32 is a multiple of four
+LINED_UP = [(1, 8, 128, "16/4"), (16, 129, 256, "16/4"), (17, 130, 640, "32/4"), (32, 300, 512, "32/4"),
+            (65, 200, 128, "32/4"), (100, 130, 640, "32/4"), (33, 9601, 1152, "48/4"), (48, 15001, 256, "48/4"),
+            (130, 1000, 128, "48/4"), (64, 15001, 640, "64/4"), (193, 4095, 256, "64/4"), (150, 17401, 384, "64/3"),
+            (64, 20001, 512, "32/4"), (2047, 2046, 128, "128/4"), (2048, 2047, 640, "128/4"), (193, 7700, 128, "tc")]
+# ... even, or odd
+OTHERS = [(1, 8, 32, "16/4e"), (16, 129, 96, "16/4e"), (9, 40, 1120, "16/4e"), (17, 40, 160, "32/4e"),
+          (32, 300, 1120, "32/4e"), (64, 384, 2080, "32/4e"), (33, 140, 1600, "32/4e"), (33, 37889, 544, "48/4e"),
+          (48, 12001, 704, "48/4e"), (129, 17408, 64, "48/4e"), (200, 3001, 320, "48/4e"), (333, 5001, 352, "48/4e"),
+          (49, 37890, 544, "64/3e"), (64, 9601, 704, "64/3e"), (145, 23809, 288, "64/3e"), (64, 15001, 736, "64/3e"),
+          (2040, 2047, 544, "64/3e"), (250, 6000, 544, ("48/4e", "tc")), (104, 14336, 1600, ("tc", "64/3e"))]
+# (M, N, K, splits, kernel)
+SPLIT_K = [(64, 1, 2048, 8, "32/4"), (24, 258, 1024, 3, "32/4"), (48, 3840, 1536, 3, "48/4"), (64, 4000, 1024, 3, "64/4"),
+           (48, 12801, 960, 3, "48/4e"), (20, 9600, 288, 4, "32/4e"), (64, 5000, 1120, 8, "64/3e"), (3, 130, 1120, 3, "16/4e"),
+           (100, 8000, 480, 3, "64/3e"), (48, 130, 1120, 3, "32/4e"), (20, 300, 160, 4, "32/4e"), (70, 256, 480, 2, "32/4e"),
+           (300, 7000, 1024, 2, "64/3"), (96, 1500, 992, 2, "32/4e")]
 
 
-def tile_rows(names):
-    """Rows of the one GEMM launch's tile, 0 for the tcgen05 kernel."""
+def tile_name(names):
+    """Which kernel the one GEMM launch among the names is."""
     gemm = [n for n in names if "gemm_w4a8" in n]
     assert len(gemm) == 1, names
-    m = re.search(r"gemm_w4a8_mma_kernelI.*?3CfgILi(\d+)ELi\d+ELi(\d+)E", gemm[0])
+    m = re.search(r"gemm_w4a8_mma_kernelI.*?3CfgILi(\d+)ELi\d+ELi(\d+)ELi\d+ELi(\d+)ELi\d+EE.*?Lb0ELb([01])E", gemm[0])
     if m is None:
         assert "gemm_w4a8_tc_kernel" in gemm[0], gemm
-        return 0
-    return 16 * int(m.group(1)) * int(m.group(2))
+        return "tc"
+    return "%d/%s%s" % (16 * int(m.group(1)) * int(m.group(2)), m.group(3), "" if m.group(4) == "1" else "e")
 
 
 def operands(oracle, cuda, M, N, K, scale_dtype, seed):
@@ -53,8 +60,8 @@ def sms148(cuda):
 
 
 @pytest.mark.parametrize("scale_dtype", [0, 1])
-@pytest.mark.parametrize("M,N,K,rows", LINED_UP + ELEMENTWISE)
-def test_gemm_tiles(w4a8, oracle, cuda, sms148, M, N, K, rows, scale_dtype):
+@pytest.mark.parametrize("M,N,K,kernel", LINED_UP + OTHERS)
+def test_gemm_tiles(w4a8, oracle, cuda, sms148, M, N, K, kernel, scale_dtype):
     import torch
     host, d = operands(oracle, cuda, M, N, K, scale_dtype, M + N + K)
     Y = torch.full((M + 1, N), 7.0, dtype=torch.float32, device=cuda)            # the last row is a canary
@@ -64,15 +71,15 @@ def test_gemm_tiles(w4a8, oracle, cuda, sms148, M, N, K, rows, scale_dtype):
 
     call(None)
     w4a8.device_status()
-    assert tile_rows(launched_kernels(call)) == rows
+    assert tile_name(launched_kernels(call)) == (kernel if isinstance(kernel, str) else kernel[scale_dtype])
     y = Y.cpu().numpy()
     assert np.array_equal(y[:M].view(np.uint32), oracle.gemm_mmq_w4a8(*host).view(np.uint32))
     assert np.all(y[M] == 7.0)
 
 
 @pytest.mark.parametrize("scale_dtype", [0, 1])
-@pytest.mark.parametrize("M,N,K,splitk,rows", SPLIT_K)
-def test_gemm_tiles_split_k(w4a8, oracle, cuda, sms148, M, N, K, splitk, rows, scale_dtype):
+@pytest.mark.parametrize("M,N,K,splitk,kernel", SPLIT_K)
+def test_gemm_tiles_split_k(w4a8, oracle, cuda, sms148, M, N, K, splitk, kernel, scale_dtype):
     import torch
     host, d = operands(oracle, cuda, M, N, K, scale_dtype, 3)
     Y = torch.empty((M, N), dtype=torch.float32, device=cuda)
@@ -83,15 +90,38 @@ def test_gemm_tiles_split_k(w4a8, oracle, cuda, sms148, M, N, K, splitk, rows, s
 
     call(None)
     torch.cuda.synchronize()
-    assert tile_rows(launched_kernels(call)) == rows
+    assert tile_name(launched_kernels(call)) == (kernel if isinstance(kernel, str) else kernel[scale_dtype])
     assert np.array_equal(Y.cpu().numpy().view(np.uint32), oracle.gemm_splitk_w4a8(*host, splitk).view(np.uint32))
 
 
+@pytest.mark.parametrize("shift_xs,shift_sw", [(1, 0), (0, 1), (0, 2)])
 @pytest.mark.parametrize("scale_dtype", [0, 1])
-@pytest.mark.parametrize("kernel", [0, 1])
-@pytest.mark.parametrize("M,N,K,rows", [(16, 130, 256, 16), (17, 130, 640, 32), (48, 130, 256, 48), (64, 130, 512, 64), (49, 131, 544, 0),
-                                        (193, 7700, 128, 0), (2048, 2047, 128, 128)])
-def test_tiny_activation_scales(w4a8, oracle, cuda, sms148, M, N, K, rows, kernel, scale_dtype):
+def test_unaligned_scales(w4a8, oracle, cuda, sms148, scale_dtype, shift_xs, shift_sw):
+    """Scales whose rows would line up, at addresses that do not: fp16 ones at odd multiples of two bytes among them."""
+    import torch
+    M, N, K = 32, 300, 768
+    host, d = operands(oracle, cuda, M, N, K, scale_dtype, 5)
+    for i, shift in ((1, shift_xs), (3, shift_sw)):
+        flat = torch.zeros(d[i].numel() + 8, dtype=d[i].dtype, device=cuda)
+        flat[shift:shift + d[i].numel()] = d[i].reshape(-1)
+        d[i] = flat[shift:]
+    Y = torch.empty((M, N), dtype=torch.float32, device=cuda)
+
+    def call(stream):
+        w4a8.launch_gemm_mmq_w4a8(d[0], d[1], d[2], d[3], Y, M, N, K, scale_dtype, stream)
+
+    call(None)
+    w4a8.device_status()
+    assert tile_name(launched_kernels(call)) == "32/4e"
+    assert np.array_equal(Y.cpu().numpy().view(np.uint32), oracle.gemm_mmq_w4a8(*host).view(np.uint32))
+
+
+@pytest.mark.parametrize("scale_dtype", [0, 1])
+@pytest.mark.parametrize("policy", [0, 1])
+@pytest.mark.parametrize("M,N,K,kernel", [(16, 130, 256, "16/4"), (17, 130, 640, "32/4"), (48, 15001, 256, "48/4"), (64, 15001, 256, "64/4"),
+                                          (150, 17401, 128, "64/3"), (49, 131, 544, "32/4e"), (64, 9601, 224, "64/3e"), (193, 7700, 128, "tc"),
+                                          (2048, 2047, 128, "128/4")])
+def test_tiny_activation_scales(w4a8, oracle, cuda, sms148, M, N, K, kernel, policy, scale_dtype):
     """Activation scales down to a few multiples of the smallest subnormal: a factor folded into them would lose bits, and the
     tile that M and N select would show in the result."""
     import torch
@@ -101,13 +131,13 @@ def test_tiny_activation_scales(w4a8, oracle, cuda, sms148, M, N, K, rows, kerne
     sw = (sw * 1000).astype(np.float16 if scale_dtype else np.float32)
     d = [torch.from_numpy(np.ascontiguousarray(a)).to(cuda) for a in (xq, xs, Wq, sw)]
     Y = torch.empty((M, N), dtype=torch.float32, device=cuda)
-    w4a8.config("gemm_kernel", kernel)
+    w4a8.config("gemm_kernel", policy)
     try:
         def call(stream):
             w4a8.launch_gemm_mmq_w4a8(d[0], d[1], d[2], d[3], Y, M, N, K, scale_dtype, stream)
         call(None)
         w4a8.device_status()
-        assert kernel == 0 or tile_rows(launched_kernels(call)) == rows
+        assert policy == 0 or tile_name(launched_kernels(call)) == (kernel if isinstance(kernel, str) else kernel[scale_dtype])
     finally:
         w4a8.config("gemm_kernel", 1)
     assert np.array_equal(Y.cpu().numpy().view(np.uint32), oracle.gemm_mmq_w4a8(xq, xs, Wq, sw).view(np.uint32))
