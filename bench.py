@@ -609,7 +609,7 @@ def run_ours(args):
             blk["m%d" % tok_] = {"us": us_b, "reference_w4a32_fused_path_sm100a_us": us_ref,
                                  "experts_touched": touched, "weight_bytes": touched * per_expert,
                                  "gbps_weights": touched * per_expert / (us_b * 1e-6) / 1e9, "int8_tops": ops / (us_b * 1e-6) / 1e12,
-                                 "kernel": "grouped GEMV per slot" if tok_ * topk <= 128 else "sorted grouped tcgen05 GEMM"}
+                                 "kernel": "grouped GEMV per slot" if tok_ * topk <= 128 else "sorted grouped GEMM"}
         extra["moe_block_128e_top8"] = blk
         del gu_w, gu_s, dn_w, dn_s
         # ---- the reference's own kernels rebuilt for sm_100a, same buffers (not part of the library) -------

@@ -10,11 +10,12 @@
 // cycles per 128 x 128 outputs and group, at 6 % tensor-pipe use, and always for 128 rows.  mma.sync m16n8k32 leaves the
 // dots in the registers that the epilogue reads: no hand-off, and a tile has as many rows as there are, in steps of 16.
 // Alone (a loop without loads) MMA 314, I2F 337 and packed mul + fma 370 cycles per 128 x 128 group, together about 500;
-// with the operand and scale traffic the kernel needs 864 with 128 x 128 tiles.  It issues on 44 % of the cycles with two
-// warps per scheduler; the rest are waits on loads from shared memory, on MMA results and on the register file.
-// Measured: 2048 x 17408 x 5120 1118 us (tcgen05 1218), 512 rows 310 (333), 333 x 15360 x 3840 165 (192), 48 x 3840 x 15360 in three
-// K ranges 52 (87).  Slower here: integer-to-float through a preset accumulator (1.5 * 2^23) instead of I2F (1133 against 989
-// cycles), scalar instead of packed fp32 (1044 against 864), scales through registers (977 against 864; they spill).
+// with the operand and scale traffic the kernel needs about 840 with 128 x 128 tiles.  It issues on 52 % of the cycles with two
+// warps per scheduler; the rest are waits on the register file, the pipes, loads from shared memory and MMA results.
+// Measured, us: 2048 x 17408 x 5120 1086 (tcgen05 1213), 512 rows 296 (327), 333 x 15360 x 3840 158 (187), 48 x 3840 x 15360 in
+// three K ranges, twice, with the quantizer, 106 (174).  Slower in the first versions, in cycles per 128 x 128 group:
+// integer-to-float through a preset accumulator (1.5 * 2^23) instead of I2F (1133 against 989), scalar instead of packed fp32
+// (1044 against 864), scales through registers (977 against 864; they spill).
 //
 // Data flow.  cp.async brings K-tiles of 4 groups into a STAGES-deep ring, laid out [group][row][32 B] for the int8
 // activations and [group][row][16 B] for the packed weights, so that a warp's fragment reads are contiguous (LDS.64 and

@@ -314,7 +314,11 @@ struct BlockArgs {
                                                                  //               2 wait + combine only
 };
 
-constexpr int GEMV_MAX_SLOTS = 128;   // auto: up to this many slots one CTA column per slot, above it the sorted GEMM
+// auto: up to this many slots one CTA column per slot, above it the sorted GEMM.  At 128 slots, H = 2048, MI = 768, fp32 scales,
+// us, GEMV / GEMM: 128 experts 77 / 147, 64 experts 73 / 114, 16 experts 71 / 58; at 512 slots 239 / 194, 237 / 122, 232 / 73.
+// With many experts the GEMV stays ahead up to about 400 slots.  The line is where it is because the two give a slot's row
+// different fp32 orders (the single-row GEMV's, the MMQ kernels'), and moving it changes the bits of calls on the way.
+constexpr int GEMV_MAX_SLOTS = 128;
 
 struct Buffers {
     int *perm, *pos, *offsets, *num_items;

@@ -133,7 +133,7 @@ int w4a8_gemv_multi(const int8_t *xq, const float *xs, int count, const uint8_t 
  * (kernels/gemm_mmq.cuh:222-233, gemm_mmq_tmpl.cuh:100-119), launch_gemm_mmq_raster_w4a8
  * (kernels/gemm_mmq_raster.cuh:115-130), launch_gemm_mma_w4a8 / _bm<BM> (kernels/gemm_mma.cuh:119-132)
  * and launch_gemm_mmq_ms (kernels/gemm_mmq_ms.cuh).  Note the (M,N,K) argument order of this family.
- * Y[M,N] fp32 row-major.  Integer group dots come from tcgen05 kind::i8 MMAs and are exact; the fp32
+ * Y[M,N] fp32 row-major.  Integer group dots come from int8 MMAs (mma.sync or tcgen05, see "gemm_kernel") and are exact; the fp32
  * epilogue evaluates t = (float)D*xs[m,b]; acc = fma(t, sw[n,b], acc) for b ascending, the order of
  * kernels/gemm_mmq.cuh:104-105, so results match the reference MMQ kernels bit for bit.
  * Needs X and Wq 16-byte aligned (TMA); M, N arbitrary. */
