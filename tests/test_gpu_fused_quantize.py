@@ -85,6 +85,18 @@ def test_rmsnorm_quantize(w4a8, oracle, cuda, request, rows, hh, variant):
     assert torch.equal(xqr, xq) and torch.equal(xsr.view(torch.int32), xs.view(torch.int32)) and torch.equal(xsumr, xsum)
 
 
+# rows shorter than one trip of the CTA's loads, exactly one trip, a ragged second and third one, and the many-row variant
+@pytest.mark.parametrize("rows,hh,variant", [(2, 32, 0), (1, 8192, 1), (2, 8224, 0), (1, 17408, 2), (320, 1056, 1)])
+def test_rmsnorm_quantize_row_lengths(w4a8, oracle, cuda, rows, hh, variant):
+    rng = np.random.default_rng(7 + rows + hh)
+    X = rng.normal(0, 1.5, size=(rows, hh)).astype(np.float32)
+    W = rng.normal(0.0 if variant == 1 else 1.0, 0.2, size=hh).astype(np.float32)
+    got = outputs(rows, hh, cuda)
+    w4a8.launch_rmsnorm_quantize_x_q8(to_dev(X, cuda), None if variant == 2 else to_dev(W, cuda), 1e-6, variant, *got, hh, rows)
+    torch.cuda.synchronize()
+    check_against_oracle(oracle, oracle.rmsnorm(X, W, 1e-6, variant), tuple(t.cpu().numpy() for t in got))
+
+
 @pytest.mark.parametrize("act", [0, 1])
 @pytest.mark.parametrize("S,IN", [(1, 17408), (4, 768), (9, 96), (16, 15360)])
 def test_glu_quantize(w4a8, oracle, cuda, request, S, IN, act):
