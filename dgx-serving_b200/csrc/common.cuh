@@ -78,6 +78,20 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
     return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
+// While a kernel waits for the one before it, HBM is idle: about 3 us in a chain of decode steps.  One thread of a CTA asks, ahead of
+// its wait, for the first `budget` bytes of the CTA's contiguous rows of weights (and their scales) to be brought to L2.  Nothing
+// is read into the SM, so this is safe whatever the kernels before write: their stores meet the lines in L2.
+__device__ __forceinline__ void prefetch_rows_l2(const uint8_t *w, const void *s, int rows, uint32_t wrow, uint32_t srow, uint32_t budget) {
+    const int fit = (int)(budget / (wrow + srow)), n = rows < fit ? rows : fit;
+    if (n <= 0) return;
+    const auto range = [](const void *p, uint64_t bytes) {                // the 16-byte pieces inside [p, p + bytes)
+        const uint64_t a = (reinterpret_cast<uint64_t>(p) + 15) & ~15ull, e = (reinterpret_cast<uint64_t>(p) + bytes) & ~15ull;
+        if (e > a) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((uint32_t)(e - a)) : "memory");
+    };
+    range(w, (uint64_t)n * wrow);
+    range(s, (uint64_t)n * srow);
+}
+
 // ---- device-side error word (set when a bounded wait runs out) ---------------------------------
 __device__ unsigned int g_dev_error = 0u;  // one translation unit: w4a8_b200.cu includes every kernel file
 __device__ __forceinline__ void dev_set_error(unsigned int code) { atomicCAS(&g_dev_error, 0u, code); }

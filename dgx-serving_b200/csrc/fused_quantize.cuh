@@ -55,6 +55,61 @@ __device__ __forceinline__ void quantize_row_vec4(float4 v, int i, bool live, ui
     }
 }
 
+// An fp32 row that a GEMV quantizes itself instead of waiting for a launch of quantize_x: every CTA quantizes the whole row for
+// its own shared memory, the first one also stores xq / xs / xsum (null: skipped) for the caller.
+struct RowSrc {
+    const float *x = nullptr;
+    uint32_t *xq = nullptr;
+    float *xs = nullptr;
+    int32_t *xsum = nullptr;
+};
+// The float4s i = tid, tid + NT, ... of the row.  load() asks for the first UB of them (ahead of the weights, so that they do not
+// queue behind them); quantize() calls put(i, word, d, live) with four quantized elements and the scale of their block.  Every lane
+// of a warp reaches put together, live == false past the end.  nvec = row length / 4, a multiple of 8.
+template <int NT, int UB>
+struct RowQuantizer {
+    float4 v[UB];
+    __device__ __forceinline__ void load(const RowSrc &src, int nvec, int i0) {
+        const float4 *x4 = reinterpret_cast<const float4 *>(src.x);
+#pragma unroll
+        for (int u = 0; u < UB; u++) v[u] = i0 + u * NT < nvec ? x4[i0 + u * NT] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    template <class F>
+    __device__ __forceinline__ void quantize(const RowSrc &src, int nvec, int tid, bool store, F &&put) {
+        const int lane = tid & 31;
+        for (int i0 = tid; i0 - lane < nvec; i0 += NT * UB) {
+            if (i0 != tid) load(src, nvec, i0);
+#pragma unroll
+            for (int u = 0; u < UB; u++) {
+                const int i = i0 + u * NT;
+                if (i - lane < nvec) {                                              // the same for the whole warp
+                    const bool live = i < nvec;
+                    float amax = fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w)));
+                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+                    const float d = quant_scale(amax);
+                    int sum = 0;
+                    const uint32_t packed = amax != 0.0f ? quantize4_pack(v[u], d, sum) : 0u;
+                    put(i, packed, d, live);
+                    if (store) {
+                        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                        sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                        if (live) {
+                            src.xq[i] = packed;
+                            if ((i & 7) == 0) {
+                                src.xs[i >> 3] = d;
+                                if (src.xsum) src.xsum[i >> 3] = sum;
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+};
+
 // VARIANT 0: y = x * inv * W (launch_rmsnorm); 1: y = x * inv * (1 + W) (launch_rmsnorm_zc); 2: y = x * inv
 // (launch_rmsnorm_noscale).  One CTA of 256 threads per row, as in the reference (the reduction order depends on it).
 // Bound by latency: a decode step has a few rows, each on one SM, and every dependent trip to L2 costs about 0.4 us.  So both

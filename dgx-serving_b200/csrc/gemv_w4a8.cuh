@@ -116,13 +116,23 @@ __device__ __forceinline__ void gemv_compute_batch(const GemvBatch<U, ST> &bt, f
     }
 }
 
-template <int MT, int U, typename ST, bool PEER>
-__global__ void __launch_bounds__(GEMV_WARPS * 32) gemv_w4a8_dp4a_kernel(
+// WARPS = FUSE_WARPS: the CTA quantizes its (one) activation row itself from src.x (RowSrc) instead of reading xq / xs.  That takes
+// every CTA about 70 warp instructions per 128 elements, so there is one CTA per SM with all the SM's warps instead of three.
+// It saves the quantizer's launch, about 4 us of every 15 in a chain of linears of one row.  Nothing is read before the wait for
+// the kernel before this one: the quantizer, which stood between that kernel and the early weight loads, is gone.  Instead
+// FUSE_PREFETCH bytes of the CTA's rows go to L2 meanwhile (four 15360 -> 3840 linears 58.0 us without, 53.9 with 64 KB, 54.1 with
+// 112, 57 with 160; four 3840 -> 4096: 18.9, 16.4, 16.3, 16.3; start 56.1 and 23.7).
+constexpr int FUSE_WARPS = 24;
+constexpr uint32_t FUSE_PREFETCH = 96 * 1024;
+template <int MT, int U, typename ST, bool PEER, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) gemv_w4a8_dp4a_kernel(
     const int8_t *__restrict__ xq, const float *__restrict__ xs, const uint8_t *__restrict__ Wq,
-    const ST *__restrict__ sw, float *__restrict__ Y, int IN, int OUT, int S, bool w_a16, GroupedArgs ga, OutArgs oa) {
+    const ST *__restrict__ sw, float *__restrict__ Y, int IN, int OUT, int S, bool w_a16, GroupedArgs ga, OutArgs oa, RowSrc src) {
+    constexpr bool FUSE = WARPS != GEMV_WARPS;
+    static_assert(!FUSE || (MT == 1 && !PEER), "one row, ordinary outputs");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int nb = IN / QBLK;
-    if (ga.idx) {  // grouped experts: blockIdx.y = slot, one activation row against that slot's expert
+    if (!FUSE && ga.idx) {  // grouped experts: blockIdx.y = slot, one activation row against that slot's expert
         const int slot = blockIdx.y;
         pdl_wait();   // the routing indices are written by an earlier kernel of the stream (router / top-k): wait first
         const int e = ga.idx[slot] - ga.expert_base;
@@ -142,24 +152,43 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32) gemv_w4a8_dp4a_kernel(
     // rows [r0, r1) of this CTA: a balanced contiguous partition of OUT over gridDim.x
     const int r0 = (int)(((long)OUT * blockIdx.x) / gridDim.x), r1 = (int)(((long)OUT * (blockIdx.x + 1)) / gridDim.x);
     const int nbatch = ((nb + 31) / 32 + U - 1) / U;                // batches per row
-    const int nrows_w = (r1 - r0 - warp + GEMV_WARPS - 1) / GEMV_WARPS;   // rows of this warp (may be <= 0)
+    const int nrows_w = (r1 - r0 - warp + WARPS - 1) / WARPS;   // rows of this warp (may be <= 0)
     const int nitems = nrows_w > 0 ? nrows_w * nbatch : 0;
     const size_t wpitch = (size_t)(IN / 2);
 
     // The first batch of weight loads goes out before the activations are staged.
     GemvBatch<U, ST> ba, bb;
+    RowQuantizer<WARPS * 32, 6> rq;
+    if constexpr (FUSE) {
+        if (tid == 0) prefetch_rows_l2(Wq + (size_t)r0 * wpitch, sw + (size_t)r0 * nb, r1 - r0, (uint32_t)wpitch, nb * sizeof(ST), FUSE_PREFETCH);
+        pdl_wait();
+        rq.load(src, IN / 4, tid);
+    }
     pdl_launch_dependents();
     if (nitems > 0) gemv_load_batch<U, ST>(ba, Wq + (size_t)(r0 + warp) * wpitch, sw + (size_t)(r0 + warp) * nb, 0, lane, nb, w_a16);
     // Everything above read only the weights and their scales.  The activations (written by the quantize kernel
     // that precedes this launch in the stream) and Y may only be touched once the previous kernel is complete.
-    pdl_wait();
+    if (!FUSE) pdl_wait();
 
+    if constexpr (FUSE) {
+        // word i = elements 4 i .. 4 i + 3; the even lane of a pair writes the 8-element chunk i / 2
+        rq.quantize(src, IN / 4, tid, blockIdx.x == 0, [&](int i, uint32_t word, float d, bool live) {
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, word, 1);
+            if (live && (i & 1) == 0) {
+                uint32_t e, od;
+                split_even_odd(word, other, e, od);
+                const int b = i >> 3, w = (i >> 1) & 3;
+                *(reinterpret_cast<uint2 *>((w < 2 ? plane0 : plane1) + b) + (w & 1)) = make_uint2(e, od);
+                if ((i & 7) == 0) sxs[b] = d;
+            }
+        });
+    } else
     // Stage activations: one task = one 8-element chunk (two 4-byte loads, like the reference's x0/x1).
 #pragma unroll
     for (int m = 0; m < MT; m++) {
         // loads in batches of UB ahead of the stores: the compiler cannot tell that the shared-memory stores do not
         // alias the loads, and a long row would otherwise pay one L2 round trip per chunk
-        constexpr int NT = GEMV_WARPS * 32, UB = 8;
+        constexpr int NT = WARPS * 32, UB = 8;
         for (int c0 = tid; c0 < IN / 8; c0 += NT * UB) {
             uint32_t x0[UB], x1[UB];
 #pragma unroll
@@ -200,7 +229,7 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32) gemv_w4a8_dp4a_kernel(
     // item i: row = r0 + warp + 8*(i / nbatch), batch = i % nbatch.  Two items per trip so that the two
     // register buffers alternate without copies.
     int row = r0 + warp, batch = 0;
-    auto advance = [&](int &r, int &bi) { if (++bi == nbatch) { bi = 0; r += GEMV_WARPS; } };
+    auto advance = [&](int &r, int &bi) { if (++bi == nbatch) { bi = 0; r += WARPS; } };
     auto finish_row = [&](int r) {
 #pragma unroll
         for (int m = 0; m < MT; m++) {
@@ -228,12 +257,12 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32) gemv_w4a8_dp4a_kernel(
     publish_out<PEER>(oa, lane == 0);
 }
 
-template <int MT, int U, typename ST, bool PEER>
+template <int MT, int U, typename ST, bool PEER, int WARPS = GEMV_WARPS>
 inline int launch_gemv_dp4a_p(const int8_t *xq, const float *xs, const uint8_t *Wq, const ST *sw, float *Y,
-                              int IN, int OUT, int S, cudaStream_t st, const GroupedArgs &ga, const OutArgs &oa) {
+                              int IN, int OUT, int S, cudaStream_t st, const GroupedArgs &ga, const OutArgs &oa, const RowSrc &src = RowSrc()) {
     const int nb = IN / QBLK;
     const size_t smem = (size_t)MT * IN + (size_t)MT * nb * sizeof(float);
-    auto kern = gemv_w4a8_dp4a_kernel<MT, U, ST, PEER>;
+    auto kern = gemv_w4a8_dp4a_kernel<MT, U, ST, PEER, WARPS>;
     if (smem > 48 * 1024) {
         static PerDevice<size_t> configured_dev;        // grow-only; the opt-in is a per-device function attribute
         size_t &configured = configured_dev.get();
@@ -252,18 +281,18 @@ inline int launch_gemv_dp4a_p(const int8_t *xq, const float *xs, const uint8_t *
     int occ = oc.occ > 0 ? oc.occ : 1;
     if (oc.smem_plus1 == 0 || occ_smem != smem) {
         int n = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, GEMV_WARPS * 32, smem);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, WARPS * 32, smem);
         if (e != cudaSuccess) return cuda_fail(e, "gemv occupancy query");
         occ = n > 0 ? n : 1;
         oc.occ = occ;
         oc.smem_plus1 = smem + 1;
     }
-    long want = (OUT + GEMV_WARPS - 1) / GEMV_WARPS;
+    long want = WARPS == GEMV_WARPS ? (OUT + WARPS - 1) / WARPS : OUT;     // one CTA per SM: every SM takes part in a narrow matrix
     long cap = (long)sm_count() * occ;
     if (ga.idx) cap = cap * ga.shard_world / ga.nslots > 1 ? cap * ga.shard_world / ga.nslots : 1;   // CTAs per slot
     const dim3 grid((unsigned)(want < cap ? want : cap), (unsigned)(ga.idx ? ga.nslots : 1));
     // every expert's base stays 16-byte aligned when Wq is, because OUT*IN/2 is a multiple of 16
-    cudaError_t le = launch_pdl(kern, grid, dim3(GEMV_WARPS * 32), smem, st, xq, xs, Wq, sw, Y, IN, OUT, S, aligned(Wq, 16), ga, oa);
+    cudaError_t le = launch_pdl(kern, grid, dim3(WARPS * 32), smem, st, xq, xs, Wq, sw, Y, IN, OUT, S, aligned(Wq, 16), ga, oa, src);
     if (le != cudaSuccess) return cuda_fail(le, "gemv_w4a8 launch");
     return launch_status("gemv_w4a8");
 }
@@ -275,15 +304,32 @@ inline int launch_gemv_dp4a_t(const int8_t *xq, const float *xs, const uint8_t *
     return launch_gemv_dp4a_p<MT, U, ST, false>(xq, xs, Wq, sw, Y, IN, OUT, S, st, ga, oa);
 }
 
+// Loads in flight per lane: the whole row when it has at most 5 slots, else the divisor of the slot
+// count that wastes no predicated slot (5 for K = 15360), else 4.
+inline int gemv_batch_of(int IN) {
+    const int nslots = (IN / QBLK + 31) / 32;
+    return nslots <= 5 ? nslots : (nslots % 5 == 0 ? 5 : (nslots % 3 == 0 ? 3 : 4));
+}
+
+// One row that the kernel quantizes itself.
+template <typename ST>
+inline int launch_gemv_row(const uint8_t *Wq, const ST *sw, float *Y, int IN, int OUT, cudaStream_t st, const RowSrc &src) {
+    const GroupedArgs ga;
+    const OutArgs oa;
+    switch (gemv_batch_of(IN)) {
+        case 1: return launch_gemv_dp4a_p<1, 1, ST, false, FUSE_WARPS>(nullptr, nullptr, Wq, sw, Y, IN, OUT, 1, st, ga, oa, src);
+        case 2: return launch_gemv_dp4a_p<1, 2, ST, false, FUSE_WARPS>(nullptr, nullptr, Wq, sw, Y, IN, OUT, 1, st, ga, oa, src);
+        case 3: return launch_gemv_dp4a_p<1, 3, ST, false, FUSE_WARPS>(nullptr, nullptr, Wq, sw, Y, IN, OUT, 1, st, ga, oa, src);
+        case 4: return launch_gemv_dp4a_p<1, 4, ST, false, FUSE_WARPS>(nullptr, nullptr, Wq, sw, Y, IN, OUT, 1, st, ga, oa, src);
+        default: return launch_gemv_dp4a_p<1, 5, ST, false, FUSE_WARPS>(nullptr, nullptr, Wq, sw, Y, IN, OUT, 1, st, ga, oa, src);
+    }
+}
+
 template <int MT, typename ST>
 inline int launch_gemv_dp4a_u(const int8_t *xq, const float *xs, const uint8_t *Wq, const ST *sw, float *Y,
                               int IN, int OUT, int S, cudaStream_t st, const GroupedArgs &ga = GroupedArgs(),
                               const OutArgs &oa = OutArgs()) {
-    const int nslots = (IN / QBLK + 31) / 32;
-    // Loads in flight per lane: the whole row when it has at most 5 slots, else the divisor of the slot
-    // count that wastes no predicated slot (5 for K = 15360), else 4.
-    int u = nslots <= 5 ? nslots : (nslots % 5 == 0 ? 5 : (nslots % 3 == 0 ? 3 : 4));
-    switch (u) {
+    switch (gemv_batch_of(IN)) {
         case 1: return launch_gemv_dp4a_t<MT, 1, ST>(xq, xs, Wq, sw, Y, IN, OUT, S, st, ga, oa);
         case 2: return launch_gemv_dp4a_t<MT, 2, ST>(xq, xs, Wq, sw, Y, IN, OUT, S, st, ga, oa);
         case 3: return launch_gemv_dp4a_t<MT, 3, ST>(xq, xs, Wq, sw, Y, IN, OUT, S, st, ga, oa);

@@ -17,6 +17,7 @@
 // are multiples of 16 bytes), K <= 8192, Wq and sw 16-byte aligned.  No expert grouping.
 #pragma once
 #include "common.cuh"
+#include "fused_quantize.cuh"
 #include "ptx_sm100.cuh"
 #include "peer_allgather.cuh"
 
@@ -71,9 +72,15 @@ struct Mats {
 
 // NG = groups per lane = ceil(K / 1024).
 // PEER: outputs go to every rank's arena and the last CTA publishes the step's epoch (peer_allgather.cuh); single matrix.
-template <int NG, typename ST, bool PEER>
+// FUSE: the consumers quantize the activation row themselves from src.x (fused_quantize.cuh) into row_bytes(IN) of shared memory
+// behind the ring; nothing is read before the wait for the kernel before this one, but FUSE_PREFETCH bytes of the CTA's rows go to
+// L2 meanwhile (see the dp4a kernel).  Four 5120 x 17408 linears, fp32 scales 47.1 us without, 45.7 with 64 KB, 47.0 with 128 KB;
+// fp16 scales 45.2, 43.9, 45.5.
+__host__ __device__ inline uint32_t row_bytes(int IN) { return (uint32_t)IN + (uint32_t)(IN / QBLK) * 4u; }
+constexpr uint32_t FUSE_PREFETCH = 64 * 1024;
+template <int NG, typename ST, bool PEER, bool FUSE>
 __global__ void __launch_bounds__(THREADS) gemv_w4a8_bulk_kernel(
-    const int8_t *__restrict__ xq, const float *__restrict__ xs, const Mats mats, int IN, int nstages, int G, OutArgs oa) {
+    const int8_t *__restrict__ xq, const float *__restrict__ xs, const Mats mats, int IN, int nstages, int G, OutArgs oa, RowSrc src) {
     int mi = 0;
     while (mi + 1 < mats.count && (int)blockIdx.x >= mats.cta0[mi + 1]) mi++;
     const uint8_t *__restrict__ Wq = mats.Wq[mi];
@@ -101,6 +108,10 @@ __global__ void __launch_bounds__(THREADS) gemv_w4a8_bulk_kernel(
         ptx::mbar_fence_init();
     }
     __syncthreads();
+    if (FUSE) {
+        if (tid == 0) prefetch_rows_l2(Wq + (size_t)r0 * wrow, sw + (size_t)r0 * nb, r1 - r0, wrow, srow, FUSE_PREFETCH);
+        pdl_wait();
+    }
     pdl_launch_dependents();
 
     if (warp == G * CW) {
@@ -125,8 +136,26 @@ __global__ void __launch_bounds__(THREADS) gemv_w4a8_bulk_kernel(
         }
     } else {
         // ---------------- consumers: warp w owns row w of every stage --------------------------------------------
-        pdl_wait();   // the activations come from the kernel before this one
-        const bool x16 = (reinterpret_cast<uintptr_t>(xq) & 15) == 0;
+        if (!FUSE) pdl_wait();   // the activations come from the kernel before this one
+        if constexpr (FUSE) {
+            uint32_t *xrow = reinterpret_cast<uint32_t *>(ring + (size_t)nstages * stage_bytes);
+            float *xrow_s = reinterpret_cast<float *>(xrow + IN / 4);
+            const auto run = [&](auto rq) {
+                rq.load(src, IN / 4, tid);
+                rq.quantize(src, IN / 4, tid, blockIdx.x == 0, [&](int i, uint32_t word, float d, bool live) {
+                    if (live) {
+                        xrow[i] = word;
+                        if ((i & 7) == 0) xrow_s[i >> 3] = d;
+                    }
+                });
+            };
+            if (G == 2) run(RowQuantizer<2 * CW * 32, 3>());
+            else run(RowQuantizer<CW * 32, 3>());
+            asm volatile("bar.sync 1, %0;" ::"r"(G * CW * 32) : "memory");
+            xq = reinterpret_cast<const int8_t *>(xrow);
+            xs = xrow_s;
+        }
+        const bool x16 = FUSE || (reinterpret_cast<uintptr_t>(xq) & 15) == 0;
         uint32_t xe[NG][4], xo[NG][4];
         float xsr[NG];
 #pragma unroll
@@ -229,9 +258,10 @@ inline bool plan_for(const void *xq, const void *Wq, const void *sw, int IN, int
     return true;
 }
 
-template <int NG, typename ST, bool PEER>
-inline int launch_p(const int8_t *xq, const float *xs, const Mats &mats_in, int IN, const Plan &p, cudaStream_t st, const OutArgs &oa) {
-    auto kern = gemv_w4a8_bulk_kernel<NG, ST, PEER>;
+template <int NG, typename ST, bool PEER, bool FUSE = false>
+inline int launch_p(const int8_t *xq, const float *xs, const Mats &mats_in, int IN, const Plan &p, cudaStream_t st, const OutArgs &oa,
+                    const RowSrc &src = RowSrc()) {
+    auto kern = gemv_w4a8_bulk_kernel<NG, ST, PEER, FUSE>;
     static PerDevice<size_t> configured_dev;            // grow-only; the opt-in is a per-device function attribute
     size_t &configured = configured_dev.get();
     if (p.smem > configured) {
@@ -258,43 +288,44 @@ inline int launch_p(const int8_t *xq, const float *xs, const Mats &mats_in, int 
         m.cta0[i + 1] = (int)end;
     }
     m.cta0[m.count] = (int)grid;
-    cudaError_t le = launch_pdl(kern, dim3((unsigned)grid), dim3((p.groups * CW + 1) * 32), p.smem, st, xq, xs, m, IN, p.stages, p.groups, oa);
+    cudaError_t le = launch_pdl(kern, dim3((unsigned)grid), dim3((p.groups * CW + 1) * 32), p.smem, st, xq, xs, m, IN, p.stages, p.groups, oa, src);
     if (le != cudaSuccess) return cuda_fail(le, "gemv_w4a8_bulk launch");
     return launch_status("gemv_w4a8_bulk");
 }
 
 template <int NG, typename ST>
-inline int launch_t(const int8_t *xq, const float *xs, const Mats &m, int IN, const Plan &p, cudaStream_t st, const OutArgs &oa) {
+inline int launch_t(const int8_t *xq, const float *xs, const Mats &m, int IN, const Plan &p, cudaStream_t st, const OutArgs &oa, const RowSrc &src) {
+    if (src.x) return launch_p<NG, ST, false, true>(xq, xs, m, IN, p, st, oa, src);
     if (oa.peers) return launch_p<NG, ST, true>(xq, xs, m, IN, p, st, oa);
     return launch_p<NG, ST, false>(xq, xs, m, IN, p, st, oa);
 }
 
 template <typename ST>
-inline int launch_st(const int8_t *xq, const float *xs, const Mats &m, int IN, const Plan &p, cudaStream_t st, const OutArgs &oa) {
+inline int launch_st(const int8_t *xq, const float *xs, const Mats &m, int IN, const Plan &p, cudaStream_t st, const OutArgs &oa, const RowSrc &src) {
     switch (p.NG) {
-        case 1: return launch_t<1, ST>(xq, xs, m, IN, p, st, oa);
-        case 2: return launch_t<2, ST>(xq, xs, m, IN, p, st, oa);
-        case 3: return launch_t<3, ST>(xq, xs, m, IN, p, st, oa);
-        case 4: return launch_t<4, ST>(xq, xs, m, IN, p, st, oa);
-        case 5: return launch_t<5, ST>(xq, xs, m, IN, p, st, oa);
-        case 6: return launch_t<6, ST>(xq, xs, m, IN, p, st, oa);
-        case 7: return launch_t<7, ST>(xq, xs, m, IN, p, st, oa);
-        case 8: return launch_t<8, ST>(xq, xs, m, IN, p, st, oa);
+        case 1: return launch_t<1, ST>(xq, xs, m, IN, p, st, oa, src);
+        case 2: return launch_t<2, ST>(xq, xs, m, IN, p, st, oa, src);
+        case 3: return launch_t<3, ST>(xq, xs, m, IN, p, st, oa, src);
+        case 4: return launch_t<4, ST>(xq, xs, m, IN, p, st, oa, src);
+        case 5: return launch_t<5, ST>(xq, xs, m, IN, p, st, oa, src);
+        case 6: return launch_t<6, ST>(xq, xs, m, IN, p, st, oa, src);
+        case 7: return launch_t<7, ST>(xq, xs, m, IN, p, st, oa, src);
+        case 8: return launch_t<8, ST>(xq, xs, m, IN, p, st, oa, src);
     }
     return fail(W4A8_ERR_UNSUPPORTED, "gemv_bulk: no kernel for %d groups per lane", p.NG);
 }
 
 inline int launch_multi(const int8_t *xq, const float *xs, const Mats &m, int IN, int scale_dtype, const Plan &p, cudaStream_t st,
-                        const OutArgs &oa = OutArgs()) {
-    if (scale_dtype == 1) return launch_st<__half>(xq, xs, m, IN, p, st, oa);
-    return launch_st<float>(xq, xs, m, IN, p, st, oa);
+                        const OutArgs &oa = OutArgs(), const RowSrc &src = RowSrc()) {
+    if (scale_dtype == 1) return launch_st<__half>(xq, xs, m, IN, p, st, oa, src);
+    return launch_st<float>(xq, xs, m, IN, p, st, oa, src);
 }
 
 inline int launch(const int8_t *xq, const float *xs, const uint8_t *Wq, const void *sw, float *Y, int IN, int OUT,
-                  int scale_dtype, const Plan &p, cudaStream_t st, const OutArgs &oa = OutArgs()) {
+                  int scale_dtype, const Plan &p, cudaStream_t st, const OutArgs &oa = OutArgs(), const RowSrc &src = RowSrc()) {
     Mats m = {};
     m.Wq[0] = Wq; m.sw[0] = sw; m.Y[0] = Y; m.OUT[0] = OUT; m.count = 1;
-    return launch_multi(xq, xs, m, IN, scale_dtype, p, st, oa);
+    return launch_multi(xq, xs, m, IN, scale_dtype, p, st, oa, src);
 }
 
 }  // namespace gemv_bulk

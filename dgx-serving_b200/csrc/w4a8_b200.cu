@@ -481,8 +481,64 @@ W4A8_API int w4a8_group_dots(const int8_t *xq, const uint8_t *Wq, int32_t *D, in
     return launch_status("group_dots");
 }
 
+// One row of a linear in one launch: a streaming GEMV that quantizes the row itself, same bits in Y, xq, xs and xsum as the two
+// launches (the dp4a and the bulk-copy kernel agree bit for bit).  Sets *done when it launched (or failed to); calls it does not
+// serve, all invalid ones among them, go the general way: those of the tensor-path kernels, rows of at most 1024 elements,
+// unaligned X, buffers that overlap (Y may replace X: two launches finish with the row before the first output is stored), and an X
+// in host or another GPU's memory, which every CTA would read over the bus.  us per linear in a chain, two launches / this:
+// 2048 x 2048 4.7 / 2.3, 3840 x 8192 8.1 / 6.4, 5120 x 16384 14.9 / 11.3, fp16 14.4 / 10.9, 7680 x 16384 19.9 / 16.7.
+static int linear_row(const float *X, int8_t *xq, float *xs, int32_t *xsum, const uint8_t *Wq, const void *sw, float *Y, int N, int K,
+                      int scale_dtype, cudaStream_t st, bool *done) {
+    *done = false;
+    const int pol = gemv_policy();
+    if ((pol != 0 && pol != 1 && pol != 3) || !X || !xq || !xs || !Wq || !sw || !Y || N <= 0 || K <= 32 * QBLK || K > 65536 || K % QBLK != 0 ||
+        (scale_dtype != 0 && scale_dtype != 1) || !aligned(X, 16) || !aligned(xq, 4) || !aligned(Wq, 4)) return W4A8_OK;
+    gemv_mma::Plan mp;
+    gemv_bulk::Plan bp;
+    const bool bulk_plan = pol != 1 && gemv_bulk::plan_for(xq, Wq, sw, K, scale_dtype, &bp);
+    // fp16 scales: where the general way takes the tensor path for one row, its fp32 order is another one
+    if (pol == 0 && scale_dtype == 1 && !(K >= 2048 && bulk_plan) && gemv_mma::plan_for(Wq, sw, K, 1, &mp)) return W4A8_OK;
+    const bool bulk_fits = bulk_plan && bp.smem + gemv_bulk::row_bytes(K) <= 227 * 1024;
+    const size_t wbytes = (size_t)N * ((size_t)K / 2 + (size_t)(K / QBLK) * (scale_dtype == 1 ? 2 : 4));
+    // Which of the two streams, us per linear of one row, dp4a / bulk.  fp32 scales: the bulk copies win where a lane has five or six
+    // groups (its registers hold the row, no lane idles) and the matrix is large enough for their fixed cost: 5120 x 4096 5.3 / 5.8,
+    // x 6144 6.5 / 6.3, x 16384 13.2 / 11.3; 6144 x 8192 9.1 / 9.4, x 12288 11.6 / 11.3; 3840 x 16384 10.0 / 10.1; 7680 x 16384
+    // 16.7 / 24.5 (two stages only); and for a vocabulary.  fp16 scales: the dp4a kernel's two-byte loads lose from a few MB up:
+    // 2560 x 3072 3.5 / 3.7, x 4096 4.8 / 4.4, 5120 x 16384 19.9 / 10.9, 7680 x 16384 29.8 / 23.7.
+    const int nb = K / QBLK;
+    const size_t mb32 = nb > 192 ? (size_t)-1 >> 20 : nb > 160 ? 32 : nb > 128 ? 18 : 96;
+    const bool bulk = bulk_fits && (pol == 3 || (K >= 2048 && wbytes >= ((scale_dtype == 1 ? 5 : mb32) << 20)));
+    const auto overlap = [](const void *a, size_t na, const void *b, size_t nb) {
+        const char *pa = static_cast<const char *>(a), *pb = static_cast<const char *>(b);
+        return a && b && pa < pb + nb && pb < pa + na;
+    };
+    const size_t xb = (size_t)K * 4, sb = (size_t)(K / QBLK) * 4, yb = (size_t)N * 4;
+    if (overlap(X, xb, Y, yb) || overlap(xq, K, Y, yb) || overlap(xs, sb, Y, yb) || overlap(xsum, sb, Y, yb) || overlap(X, xb, xq, K) ||
+        overlap(X, xb, xs, sb) || overlap(X, xb, xsum, sb)) return W4A8_OK;
+    cudaPointerAttributes at;
+    int dev = -1;
+    if (cudaPointerGetAttributes(&at, X) != cudaSuccess) { cudaGetLastError(); return W4A8_OK; }
+    if (at.type != cudaMemoryTypeDevice || cudaGetDevice(&dev) != cudaSuccess || at.device != dev) return W4A8_OK;
+    const int rc = require_sm100();
+    *done = true;
+    if (rc != W4A8_OK) return rc;
+    RowSrc src;
+    src.x = X; src.xq = reinterpret_cast<uint32_t *>(xq); src.xs = xs; src.xsum = xsum;
+    if (bulk) {
+        bp.smem += gemv_bulk::row_bytes(K);
+        return gemv_bulk::launch(xq, xs, Wq, sw, Y, K, N, scale_dtype, bp, st, OutArgs(), src);
+    }
+    if (scale_dtype == 1) return launch_gemv_row<__half>(Wq, (const __half *)sw, Y, K, N, st, src);
+    return launch_gemv_row<float>(Wq, (const float *)sw, Y, K, N, st, src);
+}
+
 W4A8_API int w4a8_linear(const float *X, int8_t *xq, float *xs, int32_t *xsum, const uint8_t *Wq, const void *sw, float *Y,
                          int S, int N, int K, int scale_dtype, int skip_quantize, void *stream) {
+    if (!skip_quantize && S == 1) {
+        bool done;
+        const int rc = linear_row(X, xq, xs, xsum, Wq, sw, Y, N, K, scale_dtype, (cudaStream_t)stream, &done);
+        if (done) return rc;
+    }
     if (!skip_quantize) {
         int rc = w4a8_quantize_x_q8(X, xq, xs, xsum, K, S, stream);
         if (rc != W4A8_OK) return rc;
