@@ -9,25 +9,28 @@
 // group pays, on top of that, a commit, a barrier, tcgen05.ld and a release through four accumulator buffers: about 950 SM
 // cycles per 128 x 128 outputs and group, at 6 % tensor-pipe use, and always for 128 rows.  mma.sync m16n8k32 leaves the
 // dots in the registers that the epilogue reads: no hand-off, and a tile has as many rows as there are, in steps of 16.
-// Alone (a loop without loads) MMA 314, I2F 337 and packed mul + fma 370 cycles per 128 x 128 group, together about 500;
-// with the operand and scale traffic the kernel needs about 840 with 128 x 128 tiles.  It issues on 52 % of the cycles with two
-// warps per scheduler; the rest are waits on the register file, the pipes, loads from shared memory and MMA results.
-// Measured, us: 2048 x 17408 x 5120 1086 (tcgen05 1213), 512 rows 296 (327), 333 x 15360 x 3840 158 (187), 48 x 3840 x 15360 in
-// three K ranges, twice, with the quantizer, 106 (174).  Slower in the first versions, in cycles per 128 x 128 group:
-// integer-to-float through a preset accumulator (1.5 * 2^23) instead of I2F (1133 against 989), scalar instead of packed fp32
-// (1044 against 864), scales through registers (977 against 864; they spill).
+// Alone (a loop without loads) MMA 270, I2F 256 (on the ALU pipe) and packed mul + fma 278 cycles per 128 x 128 group; together
+// 630, because the legacy tensor path and the packed fp32 pipe take turns: that is the floor of this kernel.  It needs about 700
+// at 80 and 96 rows, two CTAs per SM.  Measured, us, with cp.async operands / with TMA: 2048 x 17408 x 5120 1088 / 947,
+// 333 x 15360 x 3840 164 / 124, 48 x 3840 x 15360 in three K ranges, twice, with the quantizer, 106 / 88.  Slower in the first
+// versions, in cycles per 128 x 128 group: integer-to-float through a preset accumulator (1.5 * 2^23) instead of I2F (1133 against
+// 989), scalar instead of packed fp32 (1044 against 864), scales through registers (977 against 864; they spill).  Thin tiles with
+// cp.async operands, 32 x 3840 x 15360 in three ranges: 41 us; 8 and 16 warps per CTA 45 and 49, K-tiles of 8 groups 43, rows
+// prefetched to L2 47 to 61.
 //
-// Data flow.  cp.async brings K-tiles of 4 groups into a STAGES-deep ring, laid out [group][row][32 B] for the int8
-// activations and [group][row][16 B] for the packed weights, so that a warp's fragment reads are contiguous (LDS.64 and
-// LDS.32, no conflicts); groups are 32 bytes further apart than they need, which makes the copies' writes conflict-free
-// too.  A lane's word of weights expands to its two B registers with three logic operations (unpack8_x16: even and odd
-// elements), the matching A registers are two byte permutes of eight activations.  Any order of K inside a group gives
-// the same integer.  Scales travel with their K-tile, [row][group], one 16-byte (fp16: 8-byte) piece per row where they line
-// up, that is where K / 32 and every range of a split K are multiples of four and the pointers aligned (VEC); 4 bytes at a
-// time otherwise, and fp16 scales of an odd K / 32, whose rows start between two words, by plain loads.  Plain loads of all
-// scales stall their warp once per K-tile, which cost more than the kernel gains over tcgen05: 700 x 9000 x 5024 321 us with
-// them, 246 on tcgen05.  One __syncthreads per K-tile; two or three CTAs per SM cover each other's.
+// Data flow.  TMA brings K-tiles of 4 groups into a STAGES-deep ring, one barrier per stage: activations in the 128-byte swizzle
+// (a row's 4 groups), packed weights in the 64-byte one.  With cp.async the same copies, 16 bytes a lane, ran at 13 bytes per cycle
+// and SM and took the issue slots of the warps that multiply: without any copies 333 x 15360 x 3840 took 119 us instead of 164.
+// Fragment reads are contiguous up to the swizzle (LDS.64 and LDS.32, no conflicts).  A lane's word of weights expands to its two B
+// registers with three logic operations (unpack8_x16: even and odd elements), the matching A registers are two byte permutes of
+// eight activations.  Any order of K inside a group gives the same integer.  Scales travel with their K-tile by cp.async,
+// [row][group], one 16-byte (fp16: 8-byte) piece per row where they line up, that is where K / 32 and every range of a split K are
+// multiples of four and the pointers aligned (VEC); 4 bytes at a time otherwise, and fp16 scales of an odd K / 32, whose rows start
+// between two words, by plain loads.  Plain loads of all scales stall their warp once per K-tile, which cost more than the kernel
+// gains over tcgen05: 700 x 9000 x 5024 321 us with them, 246 on tcgen05.  One __syncthreads per K-tile; two or three CTAs per SM
+// cover each other.
 #pragma once
+#include <cuda.h>
 #include <type_traits>
 #include "common.cuh"
 #include "gemm_w4a8_tc.cuh"
@@ -36,10 +39,7 @@ namespace w4a8 {
 namespace gemm_mma {
 
 constexpr int GPK = 4;                    // groups per K-tile
-// live = false writes zeros and reads nothing
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool live) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
-}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -76,9 +76,10 @@ template <int TM_, int TN_, int WM_, int WN_, int STAGES_, int CTAS_>
 struct Cfg {
     static constexpr int TM = TM_, TN = TN_, WM = WM_, WN = WN_, STAGES = STAGES_, CTAS = CTAS_;
     static constexpr int BM = 16 * TM * WM, BN = 8 * TN * WN, THREADS = 32 * WM * WN;
-    static constexpr int A_GROUP = BM * 32 + 32, B_GROUP = BN * 16 + 32;      // bytes; + 32 keeps the copies' writes conflict-free
-    static constexpr int OFF_SX = GPK * (A_GROUP + B_GROUP), OFF_SW = OFF_SX + BM * GPK * 4;      // scales: [row][group]
-    static constexpr int STAGE = OFF_SW + BN * GPK * 4, SMEM = STAGES * STAGE;
+    static constexpr int A_STAGE = BM * GPK * 32, B_STAGE = BN * GPK * 16;
+    static constexpr int OFF_SX = A_STAGE + B_STAGE, OFF_SW = OFF_SX + BM * GPK * 4;      // scales: [row][group]
+    static constexpr int STAGE = (OFF_SW + BN * GPK * 4 + 1023) / 1024 * 1024;            // the swizzle repeats every 1024 bytes
+    static constexpr int OFF_BAR = STAGES * STAGE, SMEM = OFF_BAR + STAGES * 8;
     static constexpr int RB = (BN + THREADS - 1) / THREADS, RA = (BM + THREADS - 1) / THREADS;   // scale rows per thread
     static_assert(CTAS * (SMEM + 1024) <= 228 * 1024, "CTAS of these do not fit an SM's shared memory (1 KB each is the system's)");
 };
@@ -95,13 +96,11 @@ struct GroupList {
 
 template <class C, typename ST, bool GROUPED, bool VEC>
 __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
-    const int8_t *__restrict__ X, const float *__restrict__ xs, const uint8_t *__restrict__ Wq, const ST *__restrict__ sw,
+    const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const float *__restrict__ xs, const ST *__restrict__ sw,
     float *__restrict__ Y, int M, int N, int K, int m_tiles, int n_tiles, int gsplit, bool pairs, const GroupList gl) {
-    extern __shared__ __align__(128) unsigned char smem[];
+    extern __shared__ __align__(1024) unsigned char smem[];
     constexpr int TM = C::TM, TN = C::TN, BM = C::BM, BN = C::BN, NT = C::THREADS, STAGES = C::STAGES;
-    // Scales that line up make every K-tile complete.  Known at compile time that is worth 1 to 10 % (fewer instructions), except
-    // where ptxas then spills: 64 rows at three CTAs per SM, 28 bytes and 6 % slower.
-    constexpr bool FULL = VEC && !(TM * TN == 16 && C::CTAS == 3);
+    constexpr bool FULL = VEC;                             // scales that line up make every K-tile complete: 1 to 10 % faster when known here
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int wm = warp % C::WM, wn = warp / C::WM;
     const int nb = K / QBLK;
@@ -123,30 +122,40 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     }
     const int nkt = (g1 - g0 + GPK - 1) / GPK;
 
-    // ---- copies: thread -> 16-byte chunk of a row (8 of 128 bytes of activations, 4 of 64 bytes of weights).  Rows past
-    // the end are filled with zeros (their scales are the last row's) and never stored; chunks past the last group are skipped.
-    constexpr int AI = (BM * 8 + NT - 1) / NT, BI = (BN * 4 + NT - 1) / NT;
-    static_assert(BM * 8 % NT == 0 && BN * 4 % NT == 0, "whole copy instructions");
+    // ---- copies.  Rows past the end come from the next expert or are zeros (their scales are the last row's) and never stored.
     const uint32_t smem_u = (uint32_t)__cvta_generic_to_shared(smem);
-    const int ca = tid & 7, cb = tid & 3;
-    const int8_t *Xb = X + (size_t)(m0 + (tid >> 3)) * K + ca * 16;
-    const uint8_t *Wb = Wq + (wrow0 + n0 + (tid >> 2)) * (size_t)(K / 2) + cb * 16;
-    const int rows_a = mend - m0 - (tid >> 3), rows_b = N - n0 - (tid >> 2);      // live rows from this thread's first one on
-    const uint32_t adst = smem_u + (ca >> 1) * C::A_GROUP + (tid >> 3) * 32 + (ca & 1) * 16;
-    const uint32_t bdst = smem_u + GPK * C::A_GROUP + cb * C::B_GROUP + (tid >> 2) * 16;
+    auto FULL_BAR = [&](int i) { return smem_u + C::OFF_BAR + 8u * i; };
+    if (tid == 0) {
+        for (int i = 0; i < STAGES; i++) ptx::mbar_init(FULL_BAR(i), 1);
+        ptx::mbar_fence_init();
+        ptx::tma_prefetch_desc(&tmX);
+        ptx::tma_prefetch_desc(&tmW);
+    }
+    __syncthreads();
+    static_assert(!GROUPED || C::WM == 1, "an item's live tiles are every warp's");
+    const int live = GROUPED ? min(TM, (mend - m0 + 15) / 16) : TM;            // live m16 tiles
     auto copy = [&](int kt) {
         if (kt < nkt) {
             const int b0 = g0 + kt * GPK, ng = FULL ? GPK : g1 - b0;          // groups left
             const uint32_t so = (uint32_t)(kt % STAGES) * C::STAGE;
-            // scales: a row's GPK of them are one 16-byte (fp16: 8-byte) piece when they line up, else 4 bytes at a time.  Ahead of
-            // the operands, so that fewer addresses are live at once: 333 x 15360 x 3840, fp16, 163 us, behind them 169.
+            if (tid == 0) {
+                if (GROUPED) {                                                // only the item's live m16 tiles, 16 rows a copy
+                    ptx::mbar_arrive_expect_tx(FULL_BAR(kt % STAGES), live * 2048 + C::B_STAGE);
+                    for (int i = 0; i < live; i++) ptx::tma_load_2d(smem_u + so + i * 2048, &tmX, b0 * 32, m0 + 16 * i, FULL_BAR(kt % STAGES));
+                } else {
+                    ptx::mbar_arrive_expect_tx(FULL_BAR(kt % STAGES), C::A_STAGE + C::B_STAGE);
+                    ptx::tma_load_2d(smem_u + so, &tmX, b0 * 32, m0, FULL_BAR(kt % STAGES));
+                }
+                ptx::tma_load_2d(smem_u + so + C::A_STAGE, &tmW, b0 * 16, (int)wrow0 + n0, FULL_BAR(kt % STAGES));
+            }
+            // scales: a row's GPK of them are one 16-byte (fp16: 8-byte) piece when they line up, else 4 bytes at a time
 #pragma unroll
             for (int r = 0; r < C::RA; r++) {
                 const int m = tid + r * NT;
                 if (BM % NT == 0 || m < BM) {
                     const float *p = xs + (size_t)min(m0 + m, mend - 1) * nb + b0;
                     const uint32_t o = so + C::OFF_SX + m * (GPK * 4);
-                    if (VEC) cp_async16(smem_u + o, p, true);
+                    if (VEC) cp_async16(smem_u + o, p);
                     else {
 #pragma unroll
                         for (int q = 0; q < GPK; q++)
@@ -161,7 +170,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
                     const ST *p = sw + (wrow0 + min(n0 + n, N - 1)) * (size_t)nb + b0;
                     const uint32_t o = so + C::OFF_SW + n * (GPK * 4);
                     if (VEC) {
-                        if (sizeof(ST) == 4) cp_async16(smem_u + o, p, true);
+                        if (sizeof(ST) == 4) cp_async16(smem_u + o, p);
                         else cp_async8(smem_u + o, p);
                     } else if (sizeof(ST) == 4 || pairs) {               // pairs: the number of groups is even, so words never straddle the end
                         constexpr int PER = 4 / sizeof(ST);
@@ -175,22 +184,6 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
                     }
                 }
             }
-            if ((ca >> 1) < ng) {
-                const int8_t *src = Xb + (size_t)b0 * 32;
-#pragma unroll
-                for (int i = 0; i < AI; i++) {
-                    const bool live = i * (NT / 8) < rows_a;
-                    cp_async16(adst + so + i * (NT / 8) * 32, live ? src + (size_t)i * (NT / 8) * K : X, live);
-                }
-            }
-            if (cb < ng) {
-                const uint8_t *src = Wb + (size_t)b0 * 16;
-#pragma unroll
-                for (int i = 0; i < BI; i++) {
-                    const bool live = i * (NT / 4) < rows_b;
-                    cp_async16(bdst + so + i * (NT / 4) * 16, live ? src + (size_t)i * (NT / 4) * (K / 2) : Wq, live);
-                }
-            }
         }
         cp_async_commit();
     };
@@ -201,17 +194,20 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
 #pragma unroll
         for (int j = 0; j < TN; j++) acc[i][j][0] = acc[i][j][1] = 0ull;
 
-    const int rows_w = mend - m0 - wm * 16 * TM;                               // live rows of this warp (may be <= 0)
-    const int live = GROUPED ? min(TM, (rows_w + 15) / 16) : TM;               // live m16 tiles
+    // Fragment row g is row gr of its eight: with it the eight-byte reads of half a warp (g = 0..3) meet four different pairs of
+    // swizzled chunks.
+    const int gr = ((g & 3) << 1) | (g >> 2);
+    const uint32_t aoff = gr * 128 + (((t >> 1) ^ gr) << 4) + (t & 1) * 8, boff = g * 64 + ((g >> 1) << 4) + t * 4;
     // ng groups of this warp's tile; L = live m16 tiles.  Software pipeline over the columns (n8 tiles) of all groups: the
     // MMAs of the next column are issued before the current one's results are used, because a result takes far longer
     // than the dozen instructions that use it and a warp issues in order.
     auto groups = [&](auto LT, auto NGT, const unsigned char *stage, int bfirst) {
         constexpr int L = decltype(LT)::value, NG = decltype(NGT)::value;
-        const unsigned char *As = stage + bfirst * C::A_GROUP + (wm * 16 * TM + g) * 32 + t * 8;
-        const unsigned char *Bs = stage + GPK * C::A_GROUP + bfirst * C::B_GROUP + (wn * 8 * TN + g) * 16 + t * 4;
-        const unsigned char *sx = stage + C::OFF_SX + (wm * 16 * TM + g) * (GPK * 4) + bfirst * 4;
+        const unsigned char *As = stage + (wm * 16 * TM) * 128, *Bs = stage + C::A_STAGE + (wn * 8 * TN) * 64;
+        const unsigned char *sx = stage + C::OFF_SX + (wm * 16 * TM + gr) * (GPK * 4) + bfirst * 4;
         const unsigned char *ss = stage + C::OFF_SW + (wn * 8 * TN + 2 * t) * (GPK * 4) + bfirst * sizeof(ST);
+        // the swizzles put chunk c of a row where c ^ (row & 7) (activations) and c ^ (row / 2 & 3) (weights) would be: for group b
+        // that is an exclusive or with b on the lane's offset for group 0
         uint32_t a[L][4];
         int c[2][L][4];
         float xx[2][L][2], sv[2][2];
@@ -220,7 +216,8 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
             if (j == 0) {
 #pragma unroll
                 for (int i = 0; i < L; i++) {
-                    const uint2 v0 = *reinterpret_cast<const uint2 *>(As + bg * C::A_GROUP + i * 512), v1 = *reinterpret_cast<const uint2 *>(As + bg * C::A_GROUP + i * 512 + 256);
+                    const unsigned char *pa = As + (aoff ^ ((bfirst + bg) << 5)) + i * 2048;
+                    const uint2 v0 = *reinterpret_cast<const uint2 *>(pa), v1 = *reinterpret_cast<const uint2 *>(pa + 1024);
                     split_even_odd(v0.x, v0.y, a[i][0], a[i][2]);
                     split_even_odd(v1.x, v1.y, a[i][1], a[i][3]);
                     xx[bg & 1][i][0] = *reinterpret_cast<const float *>(sx + bg * 4 + (16 * i) * (GPK * 4));
@@ -228,7 +225,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
                 }
             }
             uint32_t b0, b1;
-            unpack8_x16(*reinterpret_cast<const uint32_t *>(Bs + bg * C::B_GROUP + j * 128), b0, b1);
+            unpack8_x16(*reinterpret_cast<const uint32_t *>(Bs + (boff ^ ((bfirst + bg) << 4)) + j * 512), b0, b1);
             sv[q & 1][0] = sval(*reinterpret_cast<const ST *>(ss + bg * sizeof(ST) + 8 * j * (GPK * 4)));
             sv[q & 1][1] = sval(*reinterpret_cast<const ST *>(ss + bg * sizeof(ST) + (8 * j + 1) * (GPK * 4)));
 #pragma unroll
@@ -251,11 +248,13 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     };
 
     // ---- main loop
+    bool alive = true;                                // a wait that ran out is not repeated; the results are void (device error word)
 #pragma unroll
     for (int s = 0; s < STAGES - 1; s++) copy(s);
     for (int kt = 0; kt < nkt; kt++) {
-        cp_async_wait<STAGES - 2>();                  // K-tile kt has landed (this thread's copies) ...
-        __syncthreads();                              // ... and everybody's; K-tile kt - 1 is done with
+        cp_async_wait<STAGES - 2>();                  // K-tile kt has landed: this thread's scales, ...
+        if (alive && !ptx::mbar_wait(FULL_BAR(kt % STAGES), (uint32_t)(kt / STAGES) & 1u)) { dev_set_error(0x600u); alive = false; }   // the operands, ...
+        __syncthreads();                              // ... and everybody's scales; K-tile kt - 1 is done with
         copy(kt + STAGES - 1);                        // into the slot K-tile kt - 1 used
         const unsigned char *stage = smem + (kt % STAGES) * C::STAGE;
         const int ng = FULL ? GPK : min(GPK, g1 - (g0 + kt * GPK));
@@ -283,7 +282,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     for (int i = 0; i < TM; i++) {
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int m = m0 + wm * 16 * TM + 16 * i + 8 * h + g;
+            const int m = m0 + wm * 16 * TM + 16 * i + 8 * h + gr;
             if (m < mend) {
                 float *yr = Yb + (size_t)m * N;
 #pragma unroll
@@ -315,7 +314,11 @@ inline bool scales_pair_up(const ST *sw, int K, int nsplit, int gsplit) {
 }
 template <class C, typename ST, bool GROUPED, bool VEC>
 inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int M, int N, int K, int nsplit,
-                    int gsplit, cudaStream_t st, const GroupList &gl = GroupList(), int max_items = 0) {
+                    int gsplit, cudaStream_t st, const GroupList &gl = GroupList(), int max_items = 0, long w_rows = 0) {
+    CUtensorMap tmX, tmW;
+    int rc = make_tmap_u8(&tmX, X, (uint64_t)K, (uint64_t)M, GPK * 32, GROUPED ? 16 : C::BM, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc == W4A8_OK) rc = make_tmap_u8(&tmW, Wq, (uint64_t)K / 2, (uint64_t)(GROUPED ? w_rows : N), GPK * 16, C::BN, CU_TENSOR_MAP_SWIZZLE_64B);
+    if (rc != W4A8_OK) return rc;
     auto kern = gemm_w4a8_mma_kernel<C, ST, GROUPED, VEC>;
     static PerDevice<bool> configured_dev;              // the opt-in is a per-device function attribute
     bool &configured = configured_dev.get();
@@ -328,45 +331,55 @@ inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const S
     const bool pairs = scales_pair_up(sw, K, nsplit, gsplit);
     const long units = GROUPED ? (long)max_items * n_tiles : (long)m_tiles * n_tiles * nsplit;
     if (units > 0x7FFFFFFFL) return fail(W4A8_ERR_UNSUPPORTED, "gemm: %ld work units", units);
-    kern<<<(unsigned)units, C::THREADS, C::SMEM, st>>>(X, xs, Wq, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs, gl);
+    kern<<<(unsigned)units, C::THREADS, C::SMEM, st>>>(tmX, tmW, xs, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs, gl);
     return launch_status("gemm_w4a8_mma");
 }
 
 using Cfg128 = Cfg<4, 8, 2, 2, 4, 2>;                       // 128 x 128, four warps of 64 x 64, two CTAs per SM
-// 16 TM x 128, four warps side by side, three (four) CTAs per SM.  64 rows: three stages instead of four, with which only two
-// CTAs would fit (expert block, 128 experts, 512 rows 308 us with four, 283 with three; 128 rows 239 and 204; dense
-// 160 x 17408 x 5120 183 and 135).  A grid that leaves one CTA to an SM has nothing but the ring to cover its loads: four.
+// 16 TM x 128, four warps side by side, three (four) CTAs per SM.  64 rows at three CTAs spill a few registers; they are left for
+// short ranges only.
 template <int TM>
 using CfgRows = Cfg<TM, 4, 1, 4, TM == 4 ? 3 : 4, TM == 1 ? 4 : 3>;
-using Cfg64Deep = Cfg<4, 4, 1, 4, 4, 2>;                    // 112 x 7000 x 3840: 41.1 us, with three stages 43.1
+using Cfg64Deep = Cfg<4, 4, 1, 4, 4, 2>;
 
 // Which kernel and tile a dense product takes.  The padding of the last row tile, the number of CTAs left over for the last
 // wave and the rate of each kind of tile decide; all three follow from the counts and the time a tile needs per group of K
-// with 1, 2, 3, 4 of its kind on an SM.  ns: those times, fitted to 13700 timings over M = 8 .. 2048, N = 256 .. 40000 and
-// K = 2048 .. 17408, for scales that line up, fp32 scales that are copied 4 bytes at a time, pairs of fp16 scales, and fp16
-// scales of an odd K / 32 (plain loads, a latency per K-tile that company on the SM hides).  tcgen05 adds 4 us a wave where N
+// with 1, 2, 3, 4 of its kind on an SM.  ns: those times, for scales that line up, fp32 scales that are copied 4 bytes at a time,
+// pairs of fp16 scales, and fp16 scales of an odd K / 32 (plain loads, a latency per K-tile that company on the SM hides).  tcgen05 adds 4 us a wave where N
 // is not a multiple of four: its rows are then stored 4 bytes at a time, lane by lane in different rows; 3 us a wave separate it
-// from the other kinds' fit for fp32 scales that do not line up.  The sum over waves reproduces the timings to 2 to 8 %.  On
-// average over the four the choice is 0.1 to 0.5 % slower than the fastest kind (9 % at most); it is slower than tcgen05 by more than 3 % at one point of the 13700 (65 x 15360 x 2048, 48-row tiles, 4 %).
-// Measured, us, chosen kind / tcgen05: 40 x 17408 x 5120 47 / 80, 160 x 17408 x 5120 131 / 166, 333 x 15360 x 3840 158 / 187,
-// 512 x 17408 x 5120 296 / 327, 24 x 20000 x 4128 53 / 122; tcgen05 / 64 rows: 700 x 9000 x 5024 240 / 254, 128 x 17408 x 5120
-// 87 / 91.  16 and 32 rows were not timed above max_rows.  128 x 128 tiles with scales 4 bytes at a time were never the fastest
-// kind for fp32 scales and at most 7 % ahead for fp16, so there are none.
-enum class Tile { TC, T128, R16, R32, R48, R64 };
+// from the other kinds' fit for fp32 scales that do not line up.
+// LONG_K: measured with the operands copied by TMA, over 66 to 162 groups of K, four row tiles; with them 96 and 80 rows are the
+// cheapest per row, 48 where they fill the last wave better, and neither 128 x 128 tiles nor three CTAs of 64 rows are ever ahead.
+// us, old choice / this one: 1024 x 17408 x 5120 588 (128 rows) / 477 (80), 333 x 15360 x 3840 164 / 122 (48 rows both).
+// SHORT_K: fitted to 13700 timings of the kernel with cp.async operands; ranges of up to 50 groups keep it (the tests name the tile
+// of many of them, and nothing on such ranges takes longer than it did).
+enum class Tile { TC, T128, R16, R32, R48, R64, R64X3, R80, R96 };
 enum Scales { LINED_UP, WORDS, PAIRS, HALVES };
+struct Kind { Tile tile; int rows, per_sm; long ns[4][4], max_rows; };
+constexpr long ANY = 1L << 31;
+constexpr int SHORT_K_GROUPS = 50;
 inline Tile pick(long M, long N, int K, int nsplit, int gsplit, Scales scales) {
-    struct Kind { Tile tile; int rows, per_sm; long ns[4][4], max_rows; };
-    static const Kind kinds[6] = {
-        {Tile::TC, 128, 1, {{485}, {475}, {560}, {570}}, 1L << 31},
-        {Tile::T128, 128, 2, {{510, 935}, {0}, {0}, {0}}, 1L << 31},
+    static const Kind SHORT_K[6] = {
+        {Tile::TC, 128, 1, {{485}, {475}, {560}, {570}}, ANY},
+        {Tile::T128, 128, 2, {{510, 935}, {0}, {0}, {0}}, ANY},
         {Tile::R16, 16, 4, {{155, 295, 470, 630}, {180, 435, 555, 720}, {175, 390, 480, 640}, {350, 475, 655, 850}}, 16},
         {Tile::R32, 32, 3, {{200, 375, 525}, {225, 390, 530}, {220, 370, 515}, {405, 510, 600}}, 128},
-        {Tile::R48, 48, 3, {{255, 460, 635}, {275, 490, 725}, {260, 500, 690}, {410, 585, 735}}, 1L << 31},
-        {Tile::R64, 64, 3, {{295, 535, 760}, {320, 545, 795}, {315, 545, 790}, {430, 625, 820}}, 1L << 31}};
+        {Tile::R48, 48, 3, {{255, 460, 635}, {275, 490, 725}, {260, 500, 690}, {410, 585, 735}}, ANY},
+        {Tile::R64X3, 64, 3, {{295, 535, 760}, {320, 545, 795}, {315, 545, 790}, {430, 625, 820}}, ANY}};
+    static const Kind LONG_K[7] = {
+        {Tile::TC, 128, 1, {{485}, {475}, {560}, {570}}, ANY},
+        {Tile::R16, 16, 4, {{128, 213, 256, 320}, {190, 405, 547, 608}, {150, 384, 491, 576}, {299, 373, 512, 597}}, 16},
+        {Tile::R32, 32, 3, {{170, 278, 341}, {192, 341, 461}, {192, 320, 385}, {320, 405, 470}}, ANY},
+        {Tile::R48, 48, 3, {{213, 320, 469}, {310, 555, 662}, {246, 545, 619}, {363, 533, 724}}, ANY},
+        {Tile::R64, 64, 2, {{256, 439}, {278, 503}, {277, 480}, {406, 555}}, ANY},
+        {Tile::R80, 80, 2, {{279, 470}, {320, 598}, {311, 534}, {448, 619}}, ANY},
+        {Tile::R96, 96, 2, {{341, 574}, {384, 619}, {362, 640}, {491, 683}}, ANY}};
     const long sms = sm_count(), n_tiles = (N + 127) / 128 * nsplit, groups = nsplit > 1 ? gsplit : K / QBLK;
+    const bool longk = groups > SHORT_K_GROUPS;
     Tile best = Tile::TC;
     long best_ns = 0;
-    for (const Kind &k : kinds) {
+    for (int i = 0; i < (longk ? 7 : 6); i++) {
+        const Kind &k = longk ? LONG_K[i] : SHORT_K[i];
         const long *ns = k.ns[scales];
         if (M > k.max_rows || ns[0] == 0) continue;
         const long ctas = (M + k.rows - 1) / k.rows * n_tiles, wave = sms * k.per_sm, rest = ctas % wave;
@@ -392,7 +405,10 @@ inline int launch_t(const int8_t *X, const float *xs, const uint8_t *Wq, const S
         case Tile::R16: return run(CfgRows<1>());
         case Tile::R32: return run(CfgRows<2>());
         case Tile::R48: return run(CfgRows<3>());
-        case Tile::R64:
+        case Tile::R64: return run(Cfg64Deep());
+        case Tile::R80: return run(Cfg<5, 4, 1, 4, 4, 2>());
+        case Tile::R96: return run(Cfg<6, 4, 1, 4, 4, 2>());
+        case Tile::R64X3:
             if (lines_up && (long)((M + 63) / 64) * ((N + 127) / 128) * nsplit <= sm_count())
                 return launch_c<Cfg64Deep, ST, false, true>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
             return run(CfgRows<4>());
@@ -411,14 +427,14 @@ inline int launch(const int8_t *X, const float *xs, const uint8_t *Wq, const voi
 
 // Grouped experts: Y[sorted row, n] for the rows and experts the item list names (rows no item covers are not written).
 inline int launch_grouped(const int8_t *X, const float *xs, const uint8_t *Wq, const void *sw, float *Y, int rows, int N, int K,
-                          int scale_dtype, const GroupList &gl, int max_items, cudaStream_t st) {
-    using C = CfgRows<4>;
+                          int scale_dtype, const GroupList &gl, int max_items, long w_rows, cudaStream_t st) {
+    using C = Cfg64Deep;        // expert block, 128 experts, 512 rows: 244 us; three CTAs of three stages, which spill, 302
     static_assert(C::BM == ITEM_ROWS, "an item's rows are one tile");
     const int gsplit = K / QBLK;
     const auto run = [&](auto *w) {
         using ST = std::remove_const_t<std::remove_pointer_t<decltype(w)>>;
-        if (scales_line_up(xs, w, K, 1, gsplit)) return launch_c<C, ST, true, true>(X, xs, Wq, w, Y, rows, N, K, 1, gsplit, st, gl, max_items);
-        return launch_c<C, ST, true, false>(X, xs, Wq, w, Y, rows, N, K, 1, gsplit, st, gl, max_items);
+        if (scales_line_up(xs, w, K, 1, gsplit)) return launch_c<C, ST, true, true>(X, xs, Wq, w, Y, rows, N, K, 1, gsplit, st, gl, max_items, w_rows);
+        return launch_c<C, ST, true, false>(X, xs, Wq, w, Y, rows, N, K, 1, gsplit, st, gl, max_items, w_rows);
     };
     return scale_dtype == 1 ? run((const __half *)sw) : run((const float *)sw);
 }

@@ -370,11 +370,11 @@ inline int launch_experts(const BlockArgs &a, const Buffers &b, bool use_gemm, l
         if (rc != W4A8_OK) return rc;
         gemm_mma::GroupList gl;
         gl.items = b.items; gl.num_items = b.num_items;
-        rc = gemm_mma::launch_grouped(b.xq_g, b.xs_g, a.gu_wq, a.gu_sc, b.gu, nslots, 2 * a.MI, a.H, a.scale_dtype, gl, b.max_items, st);
+        rc = gemm_mma::launch_grouped(b.xq_g, b.xs_g, a.gu_wq, a.gu_sc, b.gu, nslots, 2 * a.MI, a.H, a.scale_dtype, gl, b.max_items, (long)a.experts * 2 * a.MI, st);
         if (rc != W4A8_OK) return rc;
         rc = launch_glu_quantize(b.gu, b.gu + a.MI, a.act, nullptr, b.xq_h, b.xs_h, nullptr, a.MI, nslots, st, 2L * a.MI);
         if (rc != W4A8_OK) return rc;
-        rc = gemm_mma::launch_grouped(b.xq_h, b.xs_h, a.dn_wq, a.dn_sc, b.sout, nslots, a.H, a.MI, a.scale_dtype, gl, b.max_items, st);
+        rc = gemm_mma::launch_grouped(b.xq_h, b.xs_h, a.dn_wq, a.dn_sc, b.sout, nslots, a.H, a.MI, a.scale_dtype, gl, b.max_items, (long)a.experts * a.H, st);
         if (rc != W4A8_OK) return rc;
     } else if (fuse_rows) {
         GroupedArgs f1, f2;
