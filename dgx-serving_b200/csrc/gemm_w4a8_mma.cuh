@@ -34,6 +34,7 @@
 #include <type_traits>
 #include "common.cuh"
 #include "gemm_w4a8_tc.cuh"
+#include "tma_ring.cuh"
 
 namespace w4a8 {
 namespace gemm_mma {
@@ -134,11 +135,11 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     __syncthreads();
     static_assert(!GROUPED || C::WM == 1, "an item's live tiles are every warp's");
     const int live = GROUPED ? min(TM, (mend - m0 + 15) / 16) : TM;            // live m16 tiles
-    auto copy = [&](int kt) {
+    auto copy = [&](int kt, bool ok) {
         if (kt < nkt) {
             const int b0 = g0 + kt * GPK, ng = FULL ? GPK : g1 - b0;          // groups left
             const uint32_t so = (uint32_t)(kt % STAGES) * C::STAGE;
-            if (tid == 0) {
+            if (tid == 0 && ok) {
                 if (GROUPED) {                                                // only the item's live m16 tiles, 16 rows a copy
                     ptx::mbar_arrive_expect_tx(FULL_BAR(kt % STAGES), live * 2048 + C::B_STAGE);
                     for (int i = 0; i < live; i++) ptx::tma_load_2d(smem_u + so + i * 2048, &tmX, b0 * 32, m0 + 16 * i, FULL_BAR(kt % STAGES));
@@ -248,14 +249,12 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     };
 
     // ---- main loop
-    bool alive = true;                                // a wait that ran out is not repeated; the results are void (device error word)
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; s++) copy(s);
-    for (int kt = 0; kt < nkt; kt++) {
-        cp_async_wait<STAGES - 2>();                  // K-tile kt has landed: this thread's scales, ...
-        if (alive && !ptx::mbar_wait(FULL_BAR(kt % STAGES), (uint32_t)(kt / STAGES) & 1u)) { dev_set_error(0x600u); alive = false; }   // the operands, ...
-        __syncthreads();                              // ... and everybody's scales; K-tile kt - 1 is done with
-        copy(kt + STAGES - 1);                        // into the slot K-tile kt - 1 used
+    auto landed = [&](int kt) { return ptx::mbar_wait(FULL_BAR(kt % STAGES), (uint32_t)(kt / STAGES) & 1u); };
+    auto sync = [&](int) {
+        cp_async_wait<STAGES - 2>();                  // this thread's scales; everybody's behind the barrier
+        __syncthreads();
+    };
+    auto use = [&](int kt) {
         const unsigned char *stage = smem + (kt % STAGES) * C::STAGE;
         const int ng = FULL ? GPK : min(GPK, g1 - (g0 + kt * GPK));
         auto ktile = [&](auto LT) {
@@ -272,7 +271,13 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
             else if (TM >= 2 && live == 2) ktile(std::integral_constant<int, TM < 2 ? TM : 2>());
             else if (live == 1) ktile(std::integral_constant<int, 1>());
         }
-    }
+    };
+    auto settle = [&]() {
+        dev_set_error(0x600u);                        // the outputs are void
+        const long long t0 = clock64();
+        while (clock64() - t0 < (1ll << 21)) { }
+    };
+    run_ring<STAGES>(nkt, copy, landed, sync, use, settle);
     cp_async_wait<0>();
 
     // ---- store: a fragment row is two consecutive columns per lane, four lanes fill a 32-byte sector
