@@ -112,12 +112,12 @@ struct RowQuantizer {
 
 // VARIANT 0: y = x * inv * W (launch_rmsnorm); 1: y = x * inv * (1 + W) (launch_rmsnorm_zc); 2: y = x * inv
 // (launch_rmsnorm_noscale).  One CTA of 256 threads per row, as in the reference (the reduction order depends on it).
-// Bound by latency: a decode step has a few rows, each on one SM, and every dependent trip to L2 costs about 0.4 us.  So both
-// passes have all loads of a trip in flight at once: UB strided elements for the sum, and UV float4 of x and W, the latter
+// Bound by latency: a decode step has a few rows, each on one SM, and every dependent trip to L2 costs about 0.4 us.  So DEEP has
+// all loads of a trip of both passes in flight at once: UB strided elements for the sum, and UV float4 of x and W, the latter
 // asked for before the sum is reduced (W does not depend on it).  An MLP block of one row, 5120 x 17408: 47.0 -> 43.8 us; 64 rows
-// of 17408 11.0 -> 9.2.  With more than two rows per SM it is CTAs that hide the latency, and the registers of deep batches cost
-// more CTAs than they give (MLP block of 512 rows 967 -> 976 us): those take UB = 4, UV = 1.
-template <int VARIANT, int UB, int UV>
+// of 17408 11.0 -> 9.2.  With more rows it is CTAs that hide the latency, and the registers of deep batches cost more CTAs than
+// they give: see launch_rmsnorm_quantize for the line.
+template <int VARIANT, bool DEEP>
 __global__ void __launch_bounds__(256) rmsnorm_quantize_kernel(const float *__restrict__ X, const float *__restrict__ W, float eps,
                                                                float *__restrict__ Y, uint32_t *__restrict__ xq, float *__restrict__ xs,
                                                                int32_t *__restrict__ xsum, int hh) {
@@ -131,11 +131,13 @@ __global__ void __launch_bounds__(256) rmsnorm_quantize_kernel(const float *__re
     const int n4 = hh >> 2;                      // a multiple of 8: every 8-lane group is one whole block
     const float4 *x4 = reinterpret_cast<const float4 *>(xr);
     const float4 *w4 = reinterpret_cast<const float4 *>(W);
+    constexpr int UB = 32, UV = DEEP ? 8 : 1;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 xv[UV], wv[UV];
     auto fetch = [&](int j) {
 #pragma unroll
         for (int u = 0; u < UV; u++) {
-            xv[u] = wv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            xv[u] = wv[u] = zero;
             if (j + u * 256 < n4) {
                 xv[u] = x4[j + u * 256];
                 if (VARIANT != 2) wv[u] = w4[j + u * 256];
@@ -143,13 +145,17 @@ __global__ void __launch_bounds__(256) rmsnorm_quantize_kernel(const float *__re
         }
     };
     float ss = 0.f;
-    for (int i0 = tid; i0 < hh; i0 += 256 * UB) {
-        float v[UB];
+    if constexpr (DEEP) {
+        for (int i0 = tid; i0 < hh; i0 += 256 * UB) {
+            float v[UB];
 #pragma unroll
-        for (int u = 0; u < UB; u++) v[u] = i0 + u * 256 < hh ? xr[i0 + u * 256] : 0.f;
-        if (i0 == tid) fetch(tid);
+            for (int u = 0; u < UB; u++) v[u] = i0 + u * 256 < hh ? xr[i0 + u * 256] : 0.f;
+            if (i0 == tid) fetch(tid);
 #pragma unroll
-        for (int u = 0; u < UB; u++) ss = i0 + u * 256 < hh ? fmaf(v[u], v[u], ss) : ss;
+            for (int u = 0; u < UB; u++) ss = i0 + u * 256 < hh ? fmaf(v[u], v[u], ss) : ss;
+        }
+    } else {
+        for (int i = tid; i < hh; i += 256) { const float v = xr[i]; ss = fmaf(v, v, ss); }
     }
     // block_reduce_sum of the reference: shfl_down tree per warp, partials through shared memory, warp 0 adds them
 #pragma unroll
@@ -165,19 +171,21 @@ __global__ void __launch_bounds__(256) rmsnorm_quantize_kernel(const float *__re
     __syncthreads();
     const float inv = inv_s;
     for (int j0 = tid; j0 - lane < n4; j0 += 256 * UV) {
-        if (j0 != tid) fetch(j0);
+        if (!DEEP || j0 != tid) fetch(j0);
 #pragma unroll
         for (int u = 0; u < UV; u++) {
             const int j = j0 + u * 256;
             if (j - lane < n4) {                 // the same for the whole warp
                 const bool live = j < n4;
                 const float4 x = xv[u], w = wv[u];
-                float4 y;
-                if (VARIANT == 2) y = make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv);
-                else if (VARIANT == 0) y = make_float4(x.x * inv * w.x, x.y * inv * w.y, x.z * inv * w.z, x.w * inv * w.w);
-                else y = make_float4(x.x * inv * (1.0f + w.x), x.y * inv * (1.0f + w.y), x.z * inv * (1.0f + w.z), x.w * inv * (1.0f + w.w));
-                if (live && Y) reinterpret_cast<float4 *>(Y + row * hh)[j] = y;
-                quantize_store_vec4(live ? y : make_float4(0.f, 0.f, 0.f, 0.f), (long)(row * n4) + j, live, xq, xs, xsum);
+                float4 y = zero;
+                if (live) {
+                    if (VARIANT == 2) y = make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv);
+                    else if (VARIANT == 0) y = make_float4(x.x * inv * w.x, x.y * inv * w.y, x.z * inv * w.z, x.w * inv * w.w);
+                    else y = make_float4(x.x * inv * (1.0f + w.x), x.y * inv * (1.0f + w.y), x.z * inv * (1.0f + w.z), x.w * inv * (1.0f + w.w));
+                    if (Y) reinterpret_cast<float4 *>(Y + row * hh)[j] = y;
+                }
+                quantize_store_vec4(y, (long)(row * n4) + j, live, xq, xs, xsum);
             }
         }
     }
@@ -215,9 +223,14 @@ __global__ void __launch_bounds__(256) glu_quantize_kernel(const float4 *__restr
 inline int launch_rmsnorm_quantize(const float *X, const float *W, float eps, int variant, float *Y, int8_t *xq, float *xs,
                                    int32_t *xsum, int IN, int S, cudaStream_t st) {
     uint32_t *q = reinterpret_cast<uint32_t *>(xq);
-    auto kern = variant == 0 ? rmsnorm_quantize_kernel<0, 32, 8> : variant == 1 ? rmsnorm_quantize_kernel<1, 32, 8> : rmsnorm_quantize_kernel<2, 32, 8>;
-    if (S > 2 * sm_count())
-        kern = variant == 0 ? rmsnorm_quantize_kernel<0, 4, 1> : variant == 1 ? rmsnorm_quantize_kernel<1, 4, 1> : rmsnorm_quantize_kernel<2, 4, 1>;
+    // DEEP while its CTAs (151 registers a thread, 128 without a weight vector: one and two per SM) are one wave and the row is
+    // longer than the four elements a thread that the plain loop has in flight anyway.  us, DEEP / plain, rows x length: 1 x 1024
+    // 1.85 / 1.65, 1 x 1280 2.07 / 2.26, 148 x 5120 3.5 / 4.3, 149 x 5120 5.8 / 4.3, 296 x 17408 17.0 / 11.3, 400 x 5120 9.1 / 4.8;
+    // no weights: 296 x 2048 2.84 / 2.67, 296 x 3008 3.32 / 3.69, 296 x 5120 4.0 / 4.4, 297 x 5120 6.1 / 4.4.
+    const int sms = sm_count();
+    const bool deep = S <= sms ? IN > 1024 : variant == 2 && S <= 2 * sms && IN > 2048;
+    auto kern = variant == 0 ? rmsnorm_quantize_kernel<0, false> : variant == 1 ? rmsnorm_quantize_kernel<1, false> : rmsnorm_quantize_kernel<2, false>;
+    if (deep) kern = variant == 0 ? rmsnorm_quantize_kernel<0, true> : variant == 1 ? rmsnorm_quantize_kernel<1, true> : rmsnorm_quantize_kernel<2, true>;
     cudaError_t e = launch_pdl(kern, dim3((unsigned)S), dim3(256), 0, st, X, W, eps, Y, q, xs, xsum, IN);
     if (e != cudaSuccess) return cuda_fail(e, "rmsnorm_quantize_x_q8 launch");
     return launch_status("rmsnorm_quantize_x_q8");

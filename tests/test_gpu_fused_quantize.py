@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 import torch
 
-from conftest import to_dev
+from conftest import launched_kernels, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -94,6 +94,27 @@ def test_rmsnorm_quantize_row_lengths(w4a8, oracle, cuda, rows, hh, variant):
     got = outputs(rows, hh, cuda)
     w4a8.launch_rmsnorm_quantize_x_q8(to_dev(X, cuda), None if variant == 2 else to_dev(W, cuda), 1e-6, variant, *got, hh, rows)
     torch.cuda.synchronize()
+    check_against_oracle(oracle, oracle.rmsnorm(X, W, 1e-6, variant), tuple(t.cpu().numpy() for t in got))
+
+
+# rows on either side of one (without weights two) CTAs of the kernel with deep batches of loads per SM, and lengths on either side
+# of what is worth them; waves counts SMs
+@pytest.mark.parametrize("waves,extra,hh,variant,deep", [
+    (0, 1, 1024, 0, 0), (0, 1, 1056, 0, 1), (0, 2, 256, 2, 0), (1, 0, 1056, 1, 1), (1, 1, 1056, 1, 0), (1, 1, 2080, 0, 0), (2, 0, 8224, 1, 0),
+    (1, 1, 2048, 2, 0), (1, 1, 2080, 2, 1), (2, 0, 2080, 2, 1), (2, 1, 2080, 2, 0)])
+def test_rmsnorm_quantize_takes_deep_batches_for_one_wave_only(w4a8, oracle, cuda, waves, extra, hh, variant, deep):
+    rows = waves * torch.cuda.get_device_properties(cuda).multi_processor_count + extra
+    rng = np.random.default_rng(11 + rows + hh)
+    X = rng.normal(0, 1.5, size=(rows, hh)).astype(np.float32)
+    W = rng.normal(1.0, 0.2, size=hh).astype(np.float32)
+    x, w, got = to_dev(X, cuda), None if variant == 2 else to_dev(W, cuda), outputs(rows, hh, cuda)
+
+    def call(stream):
+        w4a8.launch_rmsnorm_quantize_x_q8(x, w, 1e-6, variant, *got, hh, rows, stream)
+
+    call(None)
+    torch.cuda.synchronize()
+    assert ["rmsnorm_quantize_kernelILi%dELb%dE" % (variant, deep) in n for n in launched_kernels(call)] == [True]
     check_against_oracle(oracle, oracle.rmsnorm(X, W, 1e-6, variant), tuple(t.cpu().numpy() for t in got))
 
 
