@@ -257,11 +257,30 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_w4a8_dp4a_kernel(
     publish_out<PEER>(oa, lane == 0);
 }
 
+// CTAs that an SM holds at once; asked of the runtime once per kernel variant and smem size.
+template <int MT, int U, typename ST, bool PEER, int WARPS>
+inline cudaError_t gemv_ctas_per_sm(size_t smem, int *ctas) {
+    struct Occ { size_t smem_plus1; int occ; };          // per device: another GPU may answer differently
+    static PerDevice<Occ> occ_dev;
+    Occ &oc = occ_dev.get();
+    size_t occ_smem = oc.smem_plus1 - 1;
+    *ctas = oc.occ > 0 ? oc.occ : 1;
+    if (oc.smem_plus1 == 0 || occ_smem != smem) {
+        int n = 0;
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gemv_w4a8_dp4a_kernel<MT, U, ST, PEER, WARPS>, WARPS * 32, smem);
+        if (e != cudaSuccess) return e;
+        oc.occ = *ctas = n > 0 ? n : 1;
+        oc.smem_plus1 = smem + 1;
+    }
+    return cudaSuccess;
+}
+
+inline size_t gemv_smem_bytes(int MT, int IN) { return (size_t)MT * IN + (size_t)MT * (IN / QBLK) * sizeof(float); }
+
 template <int MT, int U, typename ST, bool PEER, int WARPS = GEMV_WARPS>
 inline int launch_gemv_dp4a_p(const int8_t *xq, const float *xs, const uint8_t *Wq, const ST *sw, float *Y,
                               int IN, int OUT, int S, cudaStream_t st, const GroupedArgs &ga, const OutArgs &oa, const RowSrc &src = RowSrc()) {
-    const int nb = IN / QBLK;
-    const size_t smem = (size_t)MT * IN + (size_t)MT * nb * sizeof(float);
+    const size_t smem = gemv_smem_bytes(MT, IN);
     auto kern = gemv_w4a8_dp4a_kernel<MT, U, ST, PEER, WARPS>;
     if (smem > 48 * 1024) {
         static PerDevice<size_t> configured_dev;        // grow-only; the opt-in is a per-device function attribute
@@ -273,20 +292,10 @@ inline int launch_gemv_dp4a_p(const int8_t *xq, const float *xs, const uint8_t *
         }
     }
     // Persistent: as many CTAs as are resident at once (fewer when there are not enough rows, or when grouped
-    // slots already fill the GPU).  Residency is asked of the runtime once per kernel variant and smem size.
-    struct Occ { size_t smem_plus1; int occ; };          // per device: another GPU may answer differently
-    static PerDevice<Occ> occ_dev;
-    Occ &oc = occ_dev.get();
-    size_t occ_smem = oc.smem_plus1 - 1;
-    int occ = oc.occ > 0 ? oc.occ : 1;
-    if (oc.smem_plus1 == 0 || occ_smem != smem) {
-        int n = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, WARPS * 32, smem);
-        if (e != cudaSuccess) return cuda_fail(e, "gemv occupancy query");
-        occ = n > 0 ? n : 1;
-        oc.occ = occ;
-        oc.smem_plus1 = smem + 1;
-    }
+    // slots already fill the GPU).
+    int occ = 1;
+    cudaError_t oe = gemv_ctas_per_sm<MT, U, ST, PEER, WARPS>(smem, &occ);
+    if (oe != cudaSuccess) return cuda_fail(oe, "gemv occupancy query");
     long want = WARPS == GEMV_WARPS ? (OUT + WARPS - 1) / WARPS : OUT;     // one CTA per SM: every SM takes part in a narrow matrix
     long cap = (long)sm_count() * occ;
     if (ga.idx) cap = cap * ga.shard_world / ga.nslots > 1 ? cap * ga.shard_world / ga.nslots : 1;   // CTAs per slot
@@ -309,6 +318,34 @@ inline int launch_gemv_dp4a_t(const int8_t *xq, const float *xs, const uint8_t *
 inline int gemv_batch_of(int IN) {
     const int nslots = (IN / QBLK + 31) / 32;
     return nslots <= 5 ? nslots : (nslots % 5 == 0 ? 5 : (nslots % 3 == 0 ? 3 : 4));
+}
+
+// Whether the kernel that quantizes its row itself is the faster way to take one row, or a launch of the quantizer before it.
+// Every CTA spends time on the whole row, so there is a length from which the launch is cheaper.  us, two launches / one: fp32
+// scales, 17408 x 3404 11.2 / 8.7, 18976 x 4144 14.0 / 14.2, 20480 x 1776 9.7 / 10.0, 45728 x 1292 17.4 / 19.3, 61152 x 7
+// 17.2 / 20.9; fp16 scales, 14528 x 2664 13.8 / 13.6, 15744 x 4 7.8 / 8.2, 20352 x 1378 11.6 / 13.4.
+// With fp16 scales a round of rows takes as long however many warps share the SM, and up to four rows in flight per lane leave
+// registers for 32 to 48 warps of the plain kernel against FUSE_WARPS: rounds that this costs are worth the launch while rows are
+// short.  Rows per SM 24 / 25 / 40 / 50, us: 9184 elements 9.9 / 10.2 / 16.8 / 17.0 in two launches, 8.9 / 13.8 / 14.1 / 19.6 in
+// one; 25 rows of 4000 6.0 / 6.3, of 3040 5.2 / 4.8; 2016 elements, 75 rows 7.0 / 6.5, 150 rows 10.4 / 11.1.
+template <typename ST>
+inline bool gemv_row_pays(int IN, int OUT) {
+    if (sizeof(ST) == 4) return IN <= 608 * QBLK;
+    if (IN > 480 * QBLK) return false;
+    const size_t smem = gemv_smem_bytes(1, IN);
+    int ctas = 1;
+    cudaError_t e = cudaSuccess;
+    switch (gemv_batch_of(IN)) {
+        case 1: e = gemv_ctas_per_sm<1, 1, ST, false, GEMV_WARPS>(smem, &ctas); break;
+        case 2: e = gemv_ctas_per_sm<1, 2, ST, false, GEMV_WARPS>(smem, &ctas); break;
+        case 3: e = gemv_ctas_per_sm<1, 3, ST, false, GEMV_WARPS>(smem, &ctas); break;
+        case 4: e = gemv_ctas_per_sm<1, 4, ST, false, GEMV_WARPS>(smem, &ctas); break;
+        default: e = gemv_ctas_per_sm<1, 5, ST, false, GEMV_WARPS>(smem, &ctas); break;
+    }
+    if (e != cudaSuccess) { cudaGetLastError(); return false; }
+    const int rows = (OUT + sm_count() - 1) / sm_count(), warps = ctas * GEMV_WARPS;      // per SM
+    const long more = (rows + FUSE_WARPS - 1) / FUSE_WARPS - (rows + warps - 1) / warps;
+    return more <= 0 || (IN <= 96 * QBLK && more * IN <= 132 * QBLK);
 }
 
 // One row that the kernel quantizes itself.

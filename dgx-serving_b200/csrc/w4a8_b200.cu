@@ -483,8 +483,8 @@ W4A8_API int w4a8_group_dots(const int8_t *xq, const uint8_t *Wq, int32_t *D, in
 
 // One row of a linear in one launch: a streaming GEMV that quantizes the row itself, same bits in Y, xq, xs and xsum as the two
 // launches (the dp4a and the bulk-copy kernel agree bit for bit).  Sets *done when it launched (or failed to); calls it does not
-// serve, all invalid ones among them, go the general way: those of the tensor-path kernels, rows of at most 1024 elements,
-// unaligned X, buffers that overlap (Y may replace X: two launches finish with the row before the first output is stored), and an X
+// serve, all invalid ones among them, go the general way: those of the tensor-path kernels, rows of at most 1024 elements, calls
+// that two launches are faster for (gemv_row_pays), unaligned X, buffers that overlap (Y may replace X: two launches finish with the row before the first output is stored), and an X
 // in host or another GPU's memory, which every CTA would read over the bus.  us per linear in a chain, two launches / this:
 // 2048 x 2048 4.7 / 2.3, 3840 x 8192 8.1 / 6.4, 5120 x 16384 14.9 / 11.3, fp16 14.4 / 10.9, 7680 x 16384 19.9 / 16.7.
 static int linear_row(const float *X, int8_t *xq, float *xs, int32_t *xsum, const uint8_t *Wq, const void *sw, float *Y, int N, int K,
@@ -508,6 +508,7 @@ static int linear_row(const float *X, int8_t *xq, float *xs, int32_t *xsum, cons
     const int nb = K / QBLK;
     const size_t mb32 = nb > 192 ? (size_t)-1 >> 20 : nb > 160 ? 32 : nb > 128 ? 18 : 96;
     const bool bulk = bulk_fits && (pol == 3 || (K >= 2048 && wbytes >= ((scale_dtype == 1 ? 5 : mb32) << 20)));
+    if (!bulk && !(scale_dtype == 1 ? gemv_row_pays<__half>(K, N) : gemv_row_pays<float>(K, N))) return W4A8_OK;
     const auto overlap = [](const void *a, size_t na, const void *b, size_t nb) {
         const char *pa = static_cast<const char *>(a), *pb = static_cast<const char *>(b);
         return a && b && pa < pb + nb && pb < pa + na;

@@ -4,6 +4,8 @@ import numpy as np
 import pytest
 import torch
 
+from conftest import launched_kernels
+
 pytestmark = pytest.mark.gpu
 
 
@@ -46,6 +48,19 @@ def _check(w4a8, x, wq, sw, sd, x_call=None):
     (15360, 3840, 0), (17408, 513, 0), (17440, 65, 1)])
 def test_linear_row_equals_two_launches(w4a8, cuda, K, N, sd):
     _check(w4a8, *_case(K, N, sd), sd)
+
+
+# Long rows, and fp16 scales where the plain kernel's 32 to 48 warps per SM take fewer rounds than the 24 of the one that quantizes:
+# either side of each line; rows of the matrix per SM
+@pytest.mark.parametrize("K,per_sm,sd,launches", [
+    (19456, 1, 0, 1), (19488, 1, 0, 2), (30720, 1, 0, 2), (19456, 25, 0, 1), (15328, 2, 1, 1), (15392, 2, 1, 2), (17440, 1, 1, 2), (9184, 24, 1, 1),
+    (9184, 25, 1, 2), (9184, 33, 1, 1), (9184, 49, 1, 2), (3040, 25, 1, 1), (4000, 25, 1, 2), (2016, 75, 1, 1), (2016, 150, 1, 2)])
+def test_linear_row_takes_one_launch_where_that_is_faster(w4a8, cuda, K, per_sm, sd, launches):
+    N = per_sm * torch.cuda.get_device_properties(cuda).multi_processor_count
+    x, wq, sw = _case(K, N, sd)
+    _check(w4a8, x, wq, sw, sd)
+    out = _out(K, N)
+    assert len(launched_kernels(lambda st: w4a8.linear(x, out[0], out[1], out[2], wq, sw, out[3], 1, N, K, sd, 0, st))) == launches
 
 
 @pytest.mark.parametrize("policy", [1, 2, 3, 5])
