@@ -533,6 +533,17 @@ static int linear_row(const float *X, int8_t *xq, float *xs, int32_t *xsum, cons
     return launch_gemv_row<float>(Wq, (const float *)sw, Y, K, N, st, src);
 }
 
+// A linear as two launches: the quantizer, then the product.
+static int linear_general(const float *X, int8_t *xq, float *xs, int32_t *xsum, const uint8_t *Wq, const void *sw, float *Y, int S, int N,
+                          int K, int scale_dtype, int skip_quantize, void *stream) {
+    if (!skip_quantize) {
+        int rc = w4a8_quantize_x_q8(X, xq, xs, xsum, K, S, stream);
+        if (rc != W4A8_OK) return rc;
+    }
+    if (S <= 16 || !aligned(xq, 16) || !aligned(Wq, 16)) return w4a8_gemv(xq, xs, Wq, sw, Y, K, N, S, scale_dtype, stream);
+    return w4a8_gemm(xq, xs, Wq, sw, Y, S, N, K, scale_dtype, stream);
+}
+
 W4A8_API int w4a8_linear(const float *X, int8_t *xq, float *xs, int32_t *xsum, const uint8_t *Wq, const void *sw, float *Y,
                          int S, int N, int K, int scale_dtype, int skip_quantize, void *stream) {
     if (!skip_quantize && S == 1) {
@@ -540,12 +551,7 @@ W4A8_API int w4a8_linear(const float *X, int8_t *xq, float *xs, int32_t *xsum, c
         const int rc = linear_row(X, xq, xs, xsum, Wq, sw, Y, N, K, scale_dtype, (cudaStream_t)stream, &done);
         if (done) return rc;
     }
-    if (!skip_quantize) {
-        int rc = w4a8_quantize_x_q8(X, xq, xs, xsum, K, S, stream);
-        if (rc != W4A8_OK) return rc;
-    }
-    if (S <= 16 || !aligned(xq, 16) || !aligned(Wq, 16)) return w4a8_gemv(xq, xs, Wq, sw, Y, K, N, S, scale_dtype, stream);
-    return w4a8_gemm(xq, xs, Wq, sw, Y, S, N, K, scale_dtype, stream);
+    return linear_general(X, xq, xs, xsum, Wq, sw, Y, S, N, K, scale_dtype, skip_quantize, stream);
 }
 
 // Device alias of a host pointer that the GPU can address directly (pinned and mapped; with unified addressing every
@@ -570,11 +576,15 @@ W4A8_API int w4a8_linear_host(const float *X_host, float *Y_host, float *X_dev, 
     const float *X_in = X_dev;
     if (xbytes <= (1u << 20))
         if (void *xa = mapped_alias(X_host)) X_in = static_cast<const float *>(xa);
+    int rc;
     if (X_in == X_dev) {
         e = cudaMemcpyAsync(X_dev, X_host, xbytes, cudaMemcpyHostToDevice, st);
         if (e != cudaSuccess) return cuda_fail(e, "linear_host: H2D");
+        rc = w4a8_linear(X_in, xq, xs, xsum, Wq, sw, Y_dev, S, N, K, scale_dtype, 0, stream);
+    } else {
+        // one row of host memory is never quantized by every CTA (linear_row): do not pay for finding that out
+        rc = linear_general(X_in, xq, xs, xsum, Wq, sw, Y_dev, S, N, K, scale_dtype, 0, stream);
     }
-    int rc = w4a8_linear(X_in, xq, xs, xsum, Wq, sw, Y_dev, S, N, K, scale_dtype, 0, stream);
     if (rc != W4A8_OK) return rc;
     e = cudaMemcpyAsync(Y_host, Y_dev, ybytes, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
