@@ -26,8 +26,7 @@
 // eight activations.  Any order of K inside a group gives the same integer.  Scales travel with their K-tile by cp.async,
 // [row][group], one 16-byte (fp16: 8-byte) piece per row where they line up, that is where K / 32 and every range of a split K are
 // multiples of four and the pointers aligned (VEC); 4 bytes at a time otherwise, and fp16 scales of an odd K / 32, whose rows start
-// between two words, by plain loads.  Plain loads of all scales stall their warp once per K-tile, which cost more than the kernel
-// gains over tcgen05: 700 x 9000 x 5024 321 us with them, 246 on tcgen05.  One __syncthreads per K-tile; two or three CTAs per SM
+// between two words, by plain loads, which stall their warp once per K-tile.  One __syncthreads per K-tile; two or three CTAs per SM
 // cover each other.
 #pragma once
 #include <cuda.h>
@@ -124,6 +123,10 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     const int nkt = (g1 - g0 + GPK - 1) / GPK;
 
     // ---- copies.  Rows past the end come from the next expert or are zeros (their scales are the last row's) and never stored.
+    // The thread that starts the bulk copies, one of the last warp: the first warps have the activations' scales to copy besides
+    // (16 x 17408 x 5120 24.9 us by thread 0, 23.1 so).  Experts: of the first, the last one is no quicker for five copies a stage
+    // (128 experts, 512 rows 242 us by the last warp, 238 so).
+    constexpr int ISSUER = GROUPED ? 0 : NT - 32;
     const uint32_t smem_u = (uint32_t)__cvta_generic_to_shared(smem);
     auto FULL_BAR = [&](int i) { return smem_u + C::OFF_BAR + 8u * i; };
     if (tid == 0) {
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
         if (kt < nkt) {
             const int b0 = g0 + kt * GPK, ng = FULL ? GPK : g1 - b0;          // groups left
             const uint32_t so = (uint32_t)(kt % STAGES) * C::STAGE;
-            if (tid == 0 && ok) {
+            if (tid == ISSUER && ok) {
                 if (GROUPED) {                                                // only the item's live m16 tiles, 16 rows a copy
                     ptx::mbar_arrive_expect_tx(FULL_BAR(kt % STAGES), live * 2048 + C::B_STAGE);
                     for (int i = 0; i < live; i++) ptx::tma_load_2d(smem_u + so + i * 2048, &tmX, b0 * 32, m0 + 16 * i, FULL_BAR(kt % STAGES));
@@ -149,39 +152,43 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
                 }
                 ptx::tma_load_2d(smem_u + so + C::A_STAGE, &tmW, b0 * 16, (int)wrow0 + n0, FULL_BAR(kt % STAGES));
             }
-            // scales: a row's GPK of them are one 16-byte (fp16: 8-byte) piece when they line up, else 4 bytes at a time
+            // scales: a row's GPK of them are one 16-byte (fp16: 8-byte) piece when they line up, else 4 bytes at a time, neighbours by
+            // neighbouring lanes, so that an instruction touches 8 (pairs: 16) rows and not 32: 4 x 5004 x 4192 27.8 us with a row
+            // per lane, 21.3 so; 300 x 9000 x 4128 fp32 107.5 and 99.8, fp16 118 and 104
+            if (VEC) {
 #pragma unroll
-            for (int r = 0; r < C::RA; r++) {
-                const int m = tid + r * NT;
-                if (BM % NT == 0 || m < BM) {
-                    const float *p = xs + (size_t)min(m0 + m, mend - 1) * nb + b0;
-                    const uint32_t o = so + C::OFF_SX + m * (GPK * 4);
-                    if (VEC) cp_async16(smem_u + o, p);
-                    else {
+                for (int r = 0; r < C::RA; r++) {
+                    const int m = tid + r * NT;
+                    if (BM % NT == 0 || m < BM) cp_async16(smem_u + so + C::OFF_SX + m * (GPK * 4), xs + (size_t)min(m0 + m, mend - 1) * nb + b0);
+                }
 #pragma unroll
-                        for (int q = 0; q < GPK; q++)
-                            if (q < ng) cp_async4(smem_u + o + 4 * q, p + q);
+                for (int r = 0; r < C::RB; r++) {
+                    const int n = tid + r * NT;
+                    if (BN % NT == 0 || n < BN) {
+                        const ST *p = sw + (wrow0 + min(n0 + n, N - 1)) * (size_t)nb + b0;
+                        if (sizeof(ST) == 4) cp_async16(smem_u + so + C::OFF_SW + n * (GPK * 4), p);
+                        else cp_async8(smem_u + so + C::OFF_SW + n * (GPK * 4), p);
                     }
                 }
-            }
+            } else {
+                const int q = tid % GPK;
+                if (q < ng) {
 #pragma unroll
-            for (int r = 0; r < C::RB; r++) {
-                const int n = tid + r * NT;
-                if (BN % NT == 0 || n < BN) {
-                    const ST *p = sw + (wrow0 + min(n0 + n, N - 1)) * (size_t)nb + b0;
-                    const uint32_t o = so + C::OFF_SW + n * (GPK * 4);
-                    if (VEC) {
-                        if (sizeof(ST) == 4) cp_async16(smem_u + o, p);
-                        else cp_async8(smem_u + o, p);
-                    } else if (sizeof(ST) == 4 || pairs) {               // pairs: the number of groups is even, so words never straddle the end
-                        constexpr int PER = 4 / sizeof(ST);
+                    for (int m = tid / GPK; m < BM; m += NT / GPK)
+                        cp_async4(smem_u + so + C::OFF_SX + (m * GPK + q) * 4, xs + (size_t)min(m0 + m, mend - 1) * nb + b0 + q);
+                }
+                auto row = [&](int n) { return sw + (wrow0 + min(n0 + n, N - 1)) * (size_t)nb + b0; };
+                if (sizeof(ST) == 2 && pairs) {                          // the number of groups is even, so words never straddle the end
+                    const int h = tid % (GPK / 2) * 2;
+                    if (h < ng) {
 #pragma unroll
-                        for (int q = 0; q < GPK; q += PER)
-                            if (q < ng) cp_async4(smem_u + o + sizeof(ST) * q, p + q);
-                    } else {
+                        for (int n = tid / (GPK / 2); n < BN; n += NT / (GPK / 2)) cp_async4(smem_u + so + C::OFF_SW + n * (GPK * 4) + h * 2, row(n) + h);
+                    }
+                } else if (q < ng) {
 #pragma unroll
-                        for (int q = 0; q < GPK; q++)
-                            if (q < ng) *reinterpret_cast<ST *>(smem + o + sizeof(ST) * q) = p[q];
+                    for (int n = tid / GPK; n < BN; n += NT / GPK) {
+                        if (sizeof(ST) == 4) cp_async4(smem_u + so + C::OFF_SW + (n * GPK + q) * 4, row(n) + q);
+                        else *reinterpret_cast<ST *>(smem + so + C::OFF_SW + n * (GPK * 4) + q * 2) = row(n)[q];
                     }
                 }
             }
@@ -249,12 +256,16 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     };
 
     // ---- main loop
-    auto landed = [&](int kt) { return ptx::mbar_wait(FULL_BAR(kt % STAGES), (uint32_t)(kt / STAGES) & 1u); };
+    // The next K-tile's operands are asked for ahead of the use of this one: the answer takes 116 cycles, which a lone CTA per SM
+    // would wait for (48 x 3840 x 15360 in three ranges 36.5 us without, 35.7 so).
+    bool early = false;
+    auto landed = [&](int kt) { return early || ptx::mbar_wait(FULL_BAR(kt % STAGES), (uint32_t)(kt / STAGES) & 1u); };
     auto sync = [&](int) {
         cp_async_wait<STAGES - 2>();                  // this thread's scales; everybody's behind the barrier
         __syncthreads();
     };
     auto use = [&](int kt) {
+        early = kt + 1 < nkt && ptx::mbar_test(FULL_BAR((kt + 1) % STAGES), (uint32_t)((kt + 1) / STAGES) & 1u);
         const unsigned char *stage = smem + (kt % STAGES) * C::STAGE;
         const int ng = FULL ? GPK : min(GPK, g1 - (g0 + kt * GPK));
         auto ktile = [&](auto LT) {

@@ -63,5 +63,5 @@ def test_kernel_waits_for_its_operands_in_that_order_only():
     assert "ptx::mbar_wait(" in text[text.index("auto landed = "):text.index("auto sync = ")]
     assert "clock64() - t0 < (1ll << 21)" in text[text.index("auto settle = "):text.index("run_ring<STAGES>")]
     copy = text[text.index("auto copy = "):text.index("cp_async_commit();\n    };")]
-    guarded = copy[copy.index("== 0 && ok) {"):copy.index("// scales:")]
+    guarded = copy[copy.index("== ISSUER && ok) {"):copy.index("// scales:")]
     assert text.count("ptx::tma_load_2d(") == guarded.count("ptx::tma_load_2d(") and "ptx::mbar_arrive_expect_tx(" not in text.replace(guarded, "")
