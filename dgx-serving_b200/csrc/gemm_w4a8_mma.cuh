@@ -123,10 +123,9 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     const int nkt = (g1 - g0 + GPK - 1) / GPK;
 
     // ---- copies.  Rows past the end come from the next expert or are zeros (their scales are the last row's) and never stored.
-    // The thread that starts the bulk copies, one of the last warp: the first warps have the activations' scales to copy besides
-    // (16 x 17408 x 5120 24.9 us by thread 0, 23.1 so).  Experts: of the first, the last one is no quicker for five copies a stage
-    // (128 experts, 512 rows 242 us by the last warp, 238 so).
-    constexpr int ISSUER = GROUPED ? 0 : NT - 32;
+    // The thread that starts the bulk copies.  Where one warp copies all of the activations' scales besides, it is one of the last
+    // warp: 16 x 18944 x 5120 24.8 us by the first thread, 23.1 so; 192 x 9472 x 5120 56.6 and 59.1.
+    constexpr int ISSUER = !GROUPED && BM <= 32 ? NT - 32 : 0;
     const uint32_t smem_u = (uint32_t)__cvta_generic_to_shared(smem);
     auto FULL_BAR = [&](int i) { return smem_u + C::OFF_BAR + 8u * i; };
     if (tid == 0) {
@@ -256,16 +255,12 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     };
 
     // ---- main loop
-    // The next K-tile's operands are asked for ahead of the use of this one: the answer takes 116 cycles, which a lone CTA per SM
-    // would wait for (48 x 3840 x 15360 in three ranges 36.5 us without, 35.7 so).
-    bool early = false;
-    auto landed = [&](int kt) { return early || ptx::mbar_wait(FULL_BAR(kt % STAGES), (uint32_t)(kt / STAGES) & 1u); };
+    auto landed = [&](int kt) { return ptx::mbar_wait(FULL_BAR(kt % STAGES), (uint32_t)(kt / STAGES) & 1u); };
     auto sync = [&](int) {
         cp_async_wait<STAGES - 2>();                  // this thread's scales; everybody's behind the barrier
         __syncthreads();
     };
     auto use = [&](int kt) {
-        early = kt + 1 < nkt && ptx::mbar_test(FULL_BAR((kt + 1) % STAGES), (uint32_t)((kt + 1) / STAGES) & 1u);
         const unsigned char *stage = smem + (kt % STAGES) * C::STAGE;
         const int ng = FULL ? GPK : min(GPK, g1 - (g0 + kt * GPK));
         auto ktile = [&](auto LT) {

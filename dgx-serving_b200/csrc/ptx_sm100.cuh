@@ -36,18 +36,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Whether the phase has completed, without waiting.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 // Polling loop behind the first attempt.  Kept out of line on purpose: inlined, the 64-bit clock read that
 // bounds the loop was scheduled ahead of the first attempt and a wait on a barrier that had ALREADY completed
 // cost about 180 cycles instead of 34, on every hand-off of the pipeline.  The clock is read once per 64
