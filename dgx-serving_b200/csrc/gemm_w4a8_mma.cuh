@@ -10,13 +10,15 @@
 // cycles per 128 x 128 outputs and group, at 6 % tensor-pipe use, and always for 128 rows.  mma.sync m16n8k32 leaves the
 // dots in the registers that the epilogue reads: no hand-off, and a tile has as many rows as there are, in steps of 16.
 // Alone (a loop without loads) MMA 270, I2F 256 (on the ALU pipe) and packed mul + fma 278 cycles per 128 x 128 group; together
-// 630, because the legacy tensor path and the packed fp32 pipe take turns: that is the floor of this kernel.  It needs about 700
-// at 80 and 96 rows, two CTAs per SM.  Measured, us, with cp.async operands / with TMA: 2048 x 17408 x 5120 1088 / 947,
-// 333 x 15360 x 3840 164 / 124, 48 x 3840 x 15360 in three K ranges, twice, with the quantizer, 106 / 88.  Slower in the first
-// versions, in cycles per 128 x 128 group: integer-to-float through a preset accumulator (1.5 * 2^23) instead of I2F (1133 against
-// 989), scalar instead of packed fp32 (1044 against 864), scales through registers (977 against 864; they spill).  Thin tiles with
-// cp.async operands, 32 x 3840 x 15360 in three ranges: 41 us; 8 and 16 warps per CTA 45 and 49, K-tiles of 8 groups 43, rows
-// prefetched to L2 47 to 61.
+// 630, because the legacy tensor path and the packed fp32 pipe take turns: that is the floor of this kernel.  By the times below
+// and at 1965 MHz it needs 750 to 790 with two CTAs of 80 or 96 rows per SM, 860 with three of 48, 1070 with one of 48: a lone
+// CTA has one warp per scheduler, and nothing covers its waits.  Measured, us, with cp.async operands / with TMA:
+// 2048 x 17408 x 5120 1088 / 942, 333 x 15360 x 3840 164 / 123, 48 x 3840 x 15360 in three K ranges, twice, with the quantizer,
+// 106 / 85.  Slower in the first versions, in cycles per 128 x 128 group: integer-to-float through a preset accumulator (1.5 * 2^23)
+// instead of I2F (1133 against 989), scalar instead of packed fp32 (1044 against 864), scales through registers (977 against 864;
+// they spill).  Thin tiles with cp.async operands, 32 x 3840 x 15360 in three ranges: 41 us; 8 and 16 warps per CTA 45 and 49,
+// K-tiles of 8 groups 43, rows prefetched to L2 47 to 61.  A barrier asked ahead of time, so that a CTA does not wait for the answer:
+// 2 % with one CTA per SM, but the CTAs of an SM then keep step and those of a last wave pair up (1208 x 3189 x 3840 98 / 119).
 //
 // Data flow.  TMA brings K-tiles of 4 groups into a STAGES-deep ring, one barrier per stage: activations in the 128-byte swizzle
 // (a row's 4 groups), packed weights in the 64-byte one.  With cp.async the same copies, 16 bytes a lane, ran at 13 bytes per cycle
@@ -346,56 +348,64 @@ inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const S
     return launch_status("gemm_w4a8_mma");
 }
 
-using Cfg128 = Cfg<4, 8, 2, 2, 4, 2>;                       // 128 x 128, four warps of 64 x 64, two CTAs per SM
-// 16 TM x 128, four warps side by side, three (four) CTAs per SM.  64 rows at three CTAs spill a few registers; they are left for
-// short ranges only.
-template <int TM>
-using CfgRows = Cfg<TM, 4, 1, 4, TM == 4 ? 3 : 4, TM == 1 ? 4 : 3>;
-using Cfg64Deep = Cfg<4, 4, 1, 4, 4, 2>;
+// Rows of a tile / CTAs per SM; 128 columns, four warps side by side.  64 rows at two CTAs or three: the deeper ring, or the fuller
+// last wave; three with fp32 scales would spill.
+using Cfg16 = Cfg<1, 4, 1, 4, 4, 4>;
+using Cfg32 = Cfg<2, 4, 1, 4, 4, 3>;
+using Cfg48 = Cfg<3, 4, 1, 4, 4, 3>;
+using Cfg64 = Cfg<4, 4, 1, 4, 4, 2>;
+using Cfg64x3 = Cfg<4, 4, 1, 4, 3, 3>;
+using Cfg80 = Cfg<5, 4, 1, 4, 4, 2>;
+using Cfg96 = Cfg<6, 4, 1, 4, 4, 2>;
 
-// Which kernel and tile a dense product takes.  The padding of the last row tile, the number of CTAs left over for the last
-// wave and the rate of each kind of tile decide; all three follow from the counts and the time a tile needs per group of K
-// with 1, 2, 3, 4 of its kind on an SM.  ns: those times, for scales that line up, fp32 scales that are copied 4 bytes at a time,
-// pairs of fp16 scales, and fp16 scales of an odd K / 32 (plain loads, a latency per K-tile that company on the SM hides).  tcgen05 adds 4 us a wave where N
-// is not a multiple of four: its rows are then stored 4 bytes at a time, lane by lane in different rows; 3 us a wave separate it
-// from the other kinds' fit for fp32 scales that do not line up.
-// LONG_K: measured with the operands copied by TMA, over 66 to 162 groups of K, four row tiles; with them 96 and 80 rows are the
-// cheapest per row, 48 where they fill the last wave better, and neither 128 x 128 tiles nor three CTAs of 64 rows are ever ahead.
-// us, old choice / this one: 1024 x 17408 x 5120 588 (128 rows) / 477 (80), 333 x 15360 x 3840 164 / 122 (48 rows both).
-// SHORT_K: fitted to 13700 timings of the kernel with cp.async operands; ranges of up to 50 groups keep it (the tests name the tile
-// of many of them, and nothing on such ranges takes longer than it did).
-enum class Tile { TC, T128, R16, R32, R48, R64, R64X3, R80, R96 };
-enum Scales { LINED_UP, WORDS, PAIRS, HALVES };
-struct Kind { Tile tile; int rows, per_sm; long ns[4][4], max_rows; };
-constexpr long ANY = 1L << 31;
-constexpr int SHORT_K_GROUPS = 50;
+// Which tile a dense product takes.  The padding of the last row tile, the number of CTAs left over for the last wave and the rate
+// of each kind of tile decide; all three follow from the counts and from times of the tile.  wave_ns: what a wave takes apart from
+// K.  ns: a group of K with 1, 2, 3, 4 of its kind on an SM.  tail_ns: the same in a wave behind full ones, which starts as slots
+// come free.  Five columns each: fp32 scales that line up, fp32 scales copied 4 bytes at a time, pairs of fp16 scales, fp16 scales
+// of an odd K / 32 (plain loads), fp16 scales that line up.  Fitted to 16874 shapes, M = 1 .. 2048, N = 64 .. 20000, one to eight
+// ranges of 1 to 200 groups, on which every tile was timed: the choice is 0.6 to 0.9 % slower than the fastest tile on average, 12 to
+// 15 % at the 99th percentile.  A tile taller than one that holds all rows has only more padding; 16 rows were not timed above
+// max_rows.  Not among them because never or hardly ever ahead: 128 x 128 tiles (fastest for 32 of 15284 shapes, by a few per cent)
+// and the tcgen05 kernel (for none).
+enum class Tile { R16, R32, R48, R64, R64X3, R80, R96 };
+enum Scales { LINED_UP, WORDS, PAIRS, HALVES, LINED_UP_FP16 };
 inline Tile pick(long M, long N, int K, int nsplit, int gsplit, Scales scales) {
-    static const Kind SHORT_K[6] = {
-        {Tile::TC, 128, 1, {{485}, {475}, {560}, {570}}, ANY},
-        {Tile::T128, 128, 2, {{510, 935}, {0}, {0}, {0}}, ANY},
-        {Tile::R16, 16, 4, {{155, 295, 470, 630}, {180, 435, 555, 720}, {175, 390, 480, 640}, {350, 475, 655, 850}}, 16},
-        {Tile::R32, 32, 3, {{200, 375, 525}, {225, 390, 530}, {220, 370, 515}, {405, 510, 600}}, 128},
-        {Tile::R48, 48, 3, {{255, 460, 635}, {275, 490, 725}, {260, 500, 690}, {410, 585, 735}}, ANY},
-        {Tile::R64X3, 64, 3, {{295, 535, 760}, {320, 545, 795}, {315, 545, 790}, {430, 625, 820}}, ANY}};
-    static const Kind LONG_K[7] = {
-        {Tile::TC, 128, 1, {{485}, {475}, {560}, {570}}, ANY},
-        {Tile::R16, 16, 4, {{128, 213, 256, 320}, {190, 405, 547, 608}, {150, 384, 491, 576}, {299, 373, 512, 597}}, 16},
-        {Tile::R32, 32, 3, {{170, 278, 341}, {192, 341, 461}, {192, 320, 385}, {320, 405, 470}}, ANY},
-        {Tile::R48, 48, 3, {{213, 320, 469}, {310, 555, 662}, {246, 545, 619}, {363, 533, 724}}, ANY},
-        {Tile::R64, 64, 2, {{256, 439}, {278, 503}, {277, 480}, {406, 555}}, ANY},
-        {Tile::R80, 80, 2, {{279, 470}, {320, 598}, {311, 534}, {448, 619}}, ANY},
-        {Tile::R96, 96, 2, {{341, 574}, {384, 619}, {362, 640}, {491, 683}}, ANY}};
+    constexpr long ANY = 1L << 31;
+    struct Kind { Tile tile; int rows, per_sm; long max_rows, wave_ns[5], ns[5][4], tail_ns[5][3]; };
+    static const Kind kinds[] = {
+        {Tile::R16, 16, 4, 160, {1935, 1885, 1970, 2110, 1840},
+         {{125, 235, 320, 350}, {145, 265, 365, 390}, {155, 250, 345, 380}, {185, 280, 360, 425}, {130, 235, 340, 370}},
+         {{70, 150, 205}, {75, 165, 275}, {55, 125, 180}, {75, 145, 260}, {30, 125, 200}}},
+        {Tile::R32, 32, 3, ANY, {2255, 2175, 2250, 2520, 2140},
+         {{170, 330, 360}, {190, 325, 380}, {195, 315, 370}, {215, 340, 390}, {170, 310, 345}},
+         {{160, 280}, {170, 300}, {110, 260}, {145, 295}, {105, 240}}},
+        {Tile::R48, 48, 3, ANY, {2755, 2635, 2725, 2985, 2640},
+         {{205, 390, 490}, {230, 445, 530}, {240, 410, 510}, {260, 430, 540}, {200, 395, 485}},
+         {{170, 330}, {175, 365}, {190, 345}, {170, 375}, {170, 335}}},
+        {Tile::R64, 64, 2, ANY, {2935, 2745, 2815, 3130, 2825},
+         {{255, 425}, {270, 450}, {290, 445}, {305, 475}, {255, 420}},
+         {{225}, {285}, {310}, {285}, {275}}},
+        {Tile::R64X3, 64, 3, ANY, {0, 0, 3095, 3520, 3075},
+         {{0}, {0}, {285, 480, 655}, {300, 490, 660}, {250, 475, 635}},
+         {{0}, {0}, {130, 425}, {245, 425}, {145, 415}}},
+        {Tile::R80, 80, 2, ANY, {3450, 3180, 3220, 3635, 3355},
+         {{290, 505}, {345, 520}, {355, 530}, {365, 555}, {290, 485}},
+         {{260}, {390}, {405}, {445}, {355}}},
+        {Tile::R96, 96, 2, ANY, {4080, 3415, 3490, 4075, 3930},
+         {{365, 595}, {400, 610}, {390, 600}, {400, 635}, {360, 575}},
+         {{305}, {400}, {445}, {495}, {420}}}};
     const long sms = sm_count(), n_tiles = (N + 127) / 128 * nsplit, groups = nsplit > 1 ? gsplit : K / QBLK;
-    const bool longk = groups > SHORT_K_GROUPS;
-    Tile best = Tile::TC;
+    Tile best = Tile::R16;
     long best_ns = 0;
-    for (int i = 0; i < (longk ? 7 : 6); i++) {
-        const Kind &k = longk ? LONG_K[i] : SHORT_K[i];
-        const long *ns = k.ns[scales];
-        if (M > k.max_rows || ns[0] == 0) continue;
-        const long ctas = (M + k.rows - 1) / k.rows * n_tiles, wave = sms * k.per_sm, rest = ctas % wave;
-        long t = (ctas / wave * ns[k.per_sm - 1] + (rest ? ns[(rest + sms - 1) / sms - 1] : 0)) * groups;
-        if (k.tile == Tile::TC) t += (ctas + sms - 1) / sms * ((scales == WORDS ? 3000 : 0) + (N % 4 != 0 ? 4000 : 0));
+    int holds_all = 0;                                      // rows of the shortest tile that holds all rows
+    for (const Kind &k : kinds) {
+        if (M > k.max_rows || k.wave_ns[scales] == 0) continue;
+        if (holds_all && k.rows > holds_all) break;
+        if (k.rows >= M) holds_all = k.rows;
+        const long ctas = (M + k.rows - 1) / k.rows * n_tiles, wave = sms * k.per_sm, full = ctas / wave, rest = ctas % wave;
+        const long last = (rest + sms - 1) / sms;           // CTAs per SM in the last wave
+        const long last_ns = last == 0 ? 0 : full == 0 || last == k.per_sm ? k.ns[scales][last - 1] : k.tail_ns[scales][last - 1];
+        const long t = (full + (last != 0)) * k.wave_ns[scales] + (full * k.ns[scales][k.per_sm - 1] + last_ns) * groups;
         if (best_ns == 0 || t < best_ns) { best = k.tile; best_ns = t; }
     }
     return best;
@@ -405,27 +415,24 @@ template <typename ST>
 inline int launch_t(const int8_t *X, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int M, int N, int K, int nsplit,
                     int gsplit, cudaStream_t st) {
     const bool lines_up = scales_line_up(xs, sw, K, nsplit, gsplit);
-    const Scales scales = lines_up ? LINED_UP : sizeof(ST) == 4 ? WORDS : scales_pair_up(sw, K, nsplit, gsplit) ? PAIRS : HALVES;
+    const Scales scales = lines_up ? (sizeof(ST) == 4 ? LINED_UP : LINED_UP_FP16) : sizeof(ST) == 4 ? WORDS : scales_pair_up(sw, K, nsplit, gsplit) ? PAIRS : HALVES;
     const auto run = [&](auto c) {
         using C = decltype(c);
         if (lines_up) return launch_c<C, ST, false, true>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
         return launch_c<C, ST, false, false>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
     };
     switch (pick(M, N, K, nsplit, gsplit, scales)) {
-        case Tile::T128: return launch_c<Cfg128, ST, false, true>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
-        case Tile::R16: return run(CfgRows<1>());
-        case Tile::R32: return run(CfgRows<2>());
-        case Tile::R48: return run(CfgRows<3>());
-        case Tile::R64: return run(Cfg64Deep());
-        case Tile::R80: return run(Cfg<5, 4, 1, 4, 4, 2>());
-        case Tile::R96: return run(Cfg<6, 4, 1, 4, 4, 2>());
+        case Tile::R16: return run(Cfg16());
+        case Tile::R32: return run(Cfg32());
+        case Tile::R48: return run(Cfg48());
+        case Tile::R64: return run(Cfg64());
         case Tile::R64X3:
-            if (lines_up && (long)((M + 63) / 64) * ((N + 127) / 128) * nsplit <= sm_count())
-                return launch_c<Cfg64Deep, ST, false, true>(X, xs, Wq, sw, Y, M, N, K, nsplit, gsplit, st);
-            return run(CfgRows<4>());
-        case Tile::TC: break;
+            if constexpr (sizeof(ST) == 2) return run(Cfg64x3());
+            break;
+        case Tile::R80: return run(Cfg80());
+        case Tile::R96: break;
     }
-    return gemm::launch_tc_t<ST, false>(X, xs, Wq, sw, Y, nullptr, M, N, K, nsplit, gsplit, st, OutArgs());
+    return run(Cfg96());
 }
 
 // nsplit = 1: Y is the output.  nsplit > 1: Y is the [nsplit][M][N] partial-sum workspace and gsplit the number of groups
@@ -439,7 +446,7 @@ inline int launch(const int8_t *X, const float *xs, const uint8_t *Wq, const voi
 // Grouped experts: Y[sorted row, n] for the rows and experts the item list names (rows no item covers are not written).
 inline int launch_grouped(const int8_t *X, const float *xs, const uint8_t *Wq, const void *sw, float *Y, int rows, int N, int K,
                           int scale_dtype, const GroupList &gl, int max_items, long w_rows, cudaStream_t st) {
-    using C = Cfg64Deep;        // expert block, 128 experts, 512 rows: 244 us; three CTAs of three stages, which spill, 302
+    using C = Cfg64;            // expert block, 128 experts, 512 rows: 244 us; three CTAs of three stages, which spill, 302
     static_assert(C::BM == ITEM_ROWS, "an item's rows are one tile");
     const int gsplit = K / QBLK;
     const auto run = [&](auto *w) {

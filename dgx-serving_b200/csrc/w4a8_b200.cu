@@ -239,8 +239,8 @@ static int gemv_dispatch(const int8_t *xq, const float *xs, const uint8_t *Wq, c
     return launch_gemv(xq, xs, Wq, sw, Y, IN, OUT, S, scale_dtype, st, oa_in);
 }
 
-// GEMM kernel policy: 0 = fp16-operand tensor-core kernel (kind::f16, exact float group dots), 1 = int8-operand kernels
-// (int32 group dots; gemm_mma::launch picks mma.sync or tcgen05 kind::i8 by size).  Same results bit for bit.  Environment W4A8_GEMM = f16 | i8.
+// GEMM kernel policy: 0 = fp16-operand tensor-core kernel (kind::f16, exact float group dots), 1 = int8-operand kernel
+// (int32 group dots in registers; gemm_mma::pick chooses the tile by size).  Same results bit for bit.  Environment W4A8_GEMM = f16 | i8.
 static int g_gemm_policy = -1;
 static int gemm_policy() {
     if (g_gemm_policy < 0) {

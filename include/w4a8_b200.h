@@ -74,8 +74,8 @@ int w4a8_device_status(uint32_t *detail);
  *                  batch == single invariant), policy 0 for all S >= 2.
  *   "gemm_kernel": which tensor-core kernel w4a8_gemm / w4a8_gemm_splitk / w4a8_linear use (environment:
  *                  W4A8_GEMM = i8 | f16).  1 = int8 operands, int32 group dots converted in the
- *                  epilogue (default, the faster one): mma.sync tiles whose dots stay in registers, or tcgen05.mma
- *                  kind::i8, whichever the sizes make faster; 0 = operands converted to fp16 on the way into shared
+ *                  epilogue (default, the faster one): mma.sync tiles whose dots stay in registers, in the tile
+ *                  the sizes make fastest; 0 = operands converted to fp16 on the way into shared
  *                  memory (every int4 and int8 value is exact in fp16), tcgen05.mma kind::f16 with fp32
  *                  accumulation of one 32-element group, which is exact as well (|sum| <= 32*127*8 < 2^24).
  *                  Both give the same bits.  (This and every other equality of bits between kernels and with the

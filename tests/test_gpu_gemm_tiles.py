@@ -1,9 +1,8 @@
 """Every tile of the register-resident GEMM (csrc/gemm_w4a8_mma.cuh) at the edges of its rows, columns and K, bit for bit
-against the oracle's MMQ order: 16- to 64-row tiles alone and repeated, 128 x 128 tiles, rows, columns and K-tiles that end
-ragged, odd N (unpaired stores), the three ways of copying scales (K / 32 and the ranges of a split K multiples of four,
-even, odd) through more K-tiles than the ring has stages, split K with an empty last range, and shapes that stay on the
-tcgen05 kernel.  Each case names the kernel that the dispatch has to choose for it on 148 SMs, so that no later rule can
-leave one of them untested."""
+against the oracle's MMQ order: 16- to 96-row tiles alone and repeated, rows, columns and K-tiles that end ragged, odd N
+(unpaired stores), the three ways of copying scales (K / 32 and the ranges of a split K multiples of four, even, odd)
+through more K-tiles than the ring has stages, and split K with an empty last range.  Each case names the tile that the
+dispatch has to choose for it on 148 SMs, so that no later rule can leave one of them untested; the names follow the rule."""
 import re
 
 import numpy as np
@@ -13,24 +12,32 @@ from conftest import launched_kernels
 
 pytestmark = pytest.mark.gpu
 
-# The kernels: rows of the tile / stages of its ring, "e" where scales do not line up (VEC = false), "tc" for tcgen05.  A pair
-# where fp32 and fp16 scales differ.
+# The kernels: rows of the tile / stages of its ring, "e" where scales do not line up (VEC = false).  A pair where fp32 and fp16
+# scales differ.
 # (M, N, K, kernel); K / 32 is a multiple of four
-LINED_UP = [(1, 8, 128, "16/4"), (16, 129, 256, "16/4"), (17, 130, 640, "32/4"), (32, 300, 512, "32/4"),
-            (65, 200, 128, "32/4"), (100, 130, 640, "32/4"), (33, 9601, 1152, "48/4"), (48, 15001, 256, "48/4"),
-            (130, 1000, 128, "48/4"), (64, 15001, 640, "64/4"), (193, 4095, 256, "64/4"), (150, 17401, 384, "64/3"),
-            (64, 20001, 512, "32/4"), (2047, 2046, 128, "128/4"), (2048, 2047, 640, "128/4"), (193, 7700, 128, "tc")]
+LINED_UP = [(1, 8, 128, "16/4"), (16, 129, 256, "16/4"), (17, 130, 640, "16/4"), (32, 300, 512, "16/4"),
+            (65, 200, 128, "16/4"), (100, 130, 640, "16/4"), (33, 9601, 1152, "48/4"), (48, 15001, 256, "48/4"),
+            (130, 1000, 128, "16/4"), (64, 15001, 640, "64/4"), (193, 4095, 256, "32/4"), (150, 17401, 384, "80/4"),
+            (64, 20001, 512, "32/4"), (2047, 2046, 128, "48/4"), (2048, 2047, 640, "48/4"), (193, 7700, 128, "32/4"),
+            (193, 12723, 128, ("32/4", "64/3")), (147, 14287, 128, "80/4"), (262, 11397, 128, "96/4"),
+            (97, 15171, 128, "64/4")]
 # ... even, or odd
-OTHERS = [(1, 8, 32, "16/4e"), (16, 129, 96, "16/4e"), (9, 40, 1120, "16/4e"), (17, 40, 160, "32/4e"),
-          (32, 300, 1120, "32/4e"), (64, 384, 2080, "32/4e"), (33, 140, 1600, "32/4e"), (33, 37889, 544, "48/4e"),
-          (48, 12001, 704, "48/4e"), (129, 17408, 64, "48/4e"), (200, 3001, 320, "48/4e"), (333, 5001, 352, "48/4e"),
-          (49, 37890, 544, "64/3e"), (64, 9601, 704, "64/3e"), (145, 23809, 288, "64/3e"), (64, 15001, 736, "64/3e"),
-          (2040, 2047, 544, "64/3e"), (250, 6000, 544, ("48/4e", "tc")), (104, 14336, 1600, ("tc", "64/3e"))]
+OTHERS = [(1, 8, 32, "16/4e"), (16, 129, 96, "16/4e"), (9, 40, 1120, "16/4e"), (17, 40, 160, "16/4e"),
+          (32, 300, 1120, "16/4e"), (64, 384, 2080, "16/4e"), (33, 140, 1600, "16/4e"), (33, 37889, 544, "48/4e"),
+          (48, 12001, 704, ("48/4e", "16/4e")), (129, 17408, 64, "48/4e"), (200, 3001, 320, "48/4e"),
+          (333, 5001, 352, "32/4e"), (49, 37890, 544, ("32/4e", "64/3e")), (64, 9601, 704, ("64/4e", "32/4e")),
+          (145, 23809, 288, "64/4e"), (64, 15001, 736, "64/4e"), (2040, 2047, 544, "48/4e"),
+          (250, 6000, 544, "32/4e"), (104, 14336, 1600, "64/4e"), (201, 12621, 96, ("32/4e", "64/3e")),
+          (164, 14495, 96, ("96/4e", "64/3e")), (99, 14311, 96, "64/4e"), (149, 14307, 96, "80/4e"),
+          (259, 11493, 96, "96/4e"), (171, 3105, 224, "48/4e"), (149, 14307, 64, "80/4e"),
+          (201, 12621, 64, ("32/4e", "64/3e")), (259, 11493, 64, "96/4e")]
 # (M, N, K, splits, kernel)
-SPLIT_K = [(64, 1, 2048, 8, "32/4"), (24, 258, 1024, 3, "32/4"), (48, 3840, 1536, 3, "48/4"), (64, 4000, 1024, 3, "64/4"),
-           (48, 12801, 960, 3, "48/4e"), (20, 9600, 288, 4, "32/4e"), (64, 5000, 1120, 8, "64/3e"), (3, 130, 1120, 3, "16/4e"),
-           (100, 8000, 480, 3, "64/3e"), (48, 130, 1120, 3, "32/4e"), (20, 300, 160, 4, "32/4e"), (70, 256, 480, 2, "32/4e"),
-           (300, 7000, 1024, 2, "64/3"), (96, 1500, 992, 2, "32/4e")]
+SPLIT_K = [(64, 1, 2048, 8, "16/4"), (24, 258, 1024, 3, "16/4"), (48, 3840, 1536, 3, "16/4"),
+           (64, 4000, 1024, 3, ("16/4", "32/4")), (48, 12801, 960, 3, "48/4e"), (20, 9600, 288, 4, "32/4e"),
+           (64, 5000, 1120, 8, ("32/4e", "64/3e")), (3, 130, 1120, 3, "16/4e"),
+           (100, 8000, 480, 3, ("32/4e", "64/3e")), (48, 130, 1120, 3, "16/4e"), (20, 300, 160, 4, "16/4e"),
+           (70, 256, 480, 2, "16/4e"), (300, 7000, 1024, 2, ("80/4", "64/3")), (96, 1500, 992, 2, "16/4e"),
+           (98, 7049, 512, 2, "64/4"), (195, 6307, 512, 2, ("32/4", "64/3")), (33, 6421, 512, 2, "48/4")]
 
 
 def tile_name(names):
@@ -38,9 +45,7 @@ def tile_name(names):
     gemm = [n for n in names if "gemm_w4a8" in n]
     assert len(gemm) == 1, names
     m = re.search(r"gemm_w4a8_mma_kernelI.*?3CfgILi(\d+)ELi\d+ELi(\d+)ELi\d+ELi(\d+)ELi\d+EE.*?Lb0ELb([01])E", gemm[0])
-    if m is None:
-        assert "gemm_w4a8_tc_kernel" in gemm[0], gemm
-        return "tc"
+    assert m, gemm
     return "%d/%s%s" % (16 * int(m.group(1)) * int(m.group(2)), m.group(3), "" if m.group(4) == "1" else "e")
 
 
@@ -112,15 +117,18 @@ def test_unaligned_scales(w4a8, oracle, cuda, sms148, scale_dtype, shift_xs, shi
 
     call(None)
     w4a8.device_status()
-    assert tile_name(launched_kernels(call)) == "32/4e"
+    assert tile_name(launched_kernels(call)) == "16/4e"
     assert np.array_equal(Y.cpu().numpy().view(np.uint32), oracle.gemm_mmq_w4a8(*host).view(np.uint32))
 
 
 @pytest.mark.parametrize("scale_dtype", [0, 1])
 @pytest.mark.parametrize("policy", [0, 1])
-@pytest.mark.parametrize("M,N,K,kernel", [(16, 130, 256, "16/4"), (17, 130, 640, "32/4"), (48, 15001, 256, "48/4"), (64, 15001, 256, "64/4"),
-                                          (150, 17401, 128, "64/3"), (49, 131, 544, "32/4e"), (64, 9601, 224, "64/3e"), (193, 7700, 128, "tc"),
-                                          (2048, 2047, 128, "128/4")])
+@pytest.mark.parametrize("M,N,K,kernel", [(16, 130, 256, "16/4"), (17, 130, 640, "16/4"), (48, 15001, 256, "48/4"),
+                                          (64, 15001, 256, ("16/4", "32/4")), (150, 17401, 128, "80/4"),
+                                          (49, 131, 544, "16/4e"), (64, 9601, 224, "16/4e"),
+                                          (193, 7700, 128, "32/4"), (2048, 2047, 128, "48/4"),
+                                          (193, 12723, 128, ("32/4", "64/3")), (97, 15171, 128, "64/4"),
+                                          (262, 11397, 128, "96/4"), (149, 14307, 96, "80/4e")])
 def test_tiny_activation_scales(w4a8, oracle, cuda, sms148, M, N, K, kernel, policy, scale_dtype):
     """Activation scales down to a few multiples of the smallest subnormal: a factor folded into them would lose bits, and the
     tile that M and N select would show in the result."""
