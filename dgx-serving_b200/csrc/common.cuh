@@ -78,20 +78,6 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
     return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
-// While a kernel waits for the one before it, HBM is idle: about 3 us in a chain of decode steps.  One thread of a CTA asks, ahead of
-// its wait, for the first `budget` bytes of the CTA's contiguous rows of weights (and their scales) to be brought to L2.  Nothing
-// is read into the SM, so this is safe whatever the kernels before write: their stores meet the lines in L2.
-__device__ __forceinline__ void prefetch_rows_l2(const uint8_t *w, const void *s, int rows, uint32_t wrow, uint32_t srow, uint32_t budget) {
-    const int fit = (int)(budget / (wrow + srow)), n = rows < fit ? rows : fit;
-    if (n <= 0) return;
-    const auto range = [](const void *p, uint64_t bytes) {                // the 16-byte pieces inside [p, p + bytes)
-        const uint64_t a = (reinterpret_cast<uint64_t>(p) + 15) & ~15ull, e = (reinterpret_cast<uint64_t>(p) + bytes) & ~15ull;
-        if (e > a) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((uint32_t)(e - a)) : "memory");
-    };
-    range(w, (uint64_t)n * wrow);
-    range(s, (uint64_t)n * srow);
-}
-
 // ---- device-side error word (set when a bounded wait runs out) ---------------------------------
 __device__ unsigned int g_dev_error = 0u;  // one translation unit: w4a8_b200.cu includes every kernel file
 __device__ __forceinline__ void dev_set_error(unsigned int code) { atomicCAS(&g_dev_error, 0u, code); }
@@ -165,6 +151,23 @@ __device__ __forceinline__ uint32_t quantize4_pack(float4 v, float d, int &sum) 
     if (!sure) w = quantize4_div(v, d);
     sum = __dp4a((int)w, 0x01010101, 0);
     return w;
+}
+// Four elements of a 32-element block held by 8 consecutive lanes (d = amax / 127, q = rintf(x / d) clamped, zero block -> zeros):
+// the packed word, the block's scale and the sum of these four.  Every lane of the warp calls it.
+__device__ __forceinline__ uint32_t quantize_block_vec4(float4 v, float &d, int &sum) {
+    float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+    d = quant_scale(amax);
+    sum = 0;
+    return amax != 0.0f ? quantize4_pack(v, d, sum) : 0u;
+}
+// The block's sum from the 8 lanes' sums.
+__device__ __forceinline__ int block_sum(int sum) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    return sum + __shfl_xor_sync(0xffffffffu, sum, 4);
 }
 // Activation bytes x[0..7] (two words) split the same way: even = x0 x2 x4 x6, odd = x1 x3 x5 x7.
 __device__ __forceinline__ void split_even_odd(uint32_t x0, uint32_t x1, uint32_t &even, uint32_t &odd) {

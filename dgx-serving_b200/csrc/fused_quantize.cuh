@@ -10,21 +10,14 @@
 
 namespace w4a8 {
 
-// One float4 of a 32-element block held by 8 consecutive lanes: block maximum and sum by three xor-shuffles, outputs
-// as in quantize_x_q8_vec_kernel (d = amax / 127, q = rintf(x / d) clamped, zero block -> zeros).  Every lane of
-// the warp must call it; lanes with live == false carry zeros and store nothing.
+// One float4 of a 32-element block held by 8 consecutive lanes, outputs as in quantize_x_q8_vec_kernel.  Every lane of the
+// warp must call it; lanes with live == false carry zeros and store nothing.
 __device__ __forceinline__ void quantize_store_vec4(float4 v, long i, bool live, uint32_t *__restrict__ xq,
                                                     float *__restrict__ xs, int32_t *__restrict__ xsum) {
-    float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-    const float d = quant_scale(amax);
-    int sum = 0;
-    const uint32_t packed = amax != 0.0f ? quantize4_pack(v, d, sum) : 0u;
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+    float d;
+    int sum;
+    const uint32_t packed = quantize_block_vec4(v, d, sum);
+    sum = block_sum(sum);
     if (live) {
         xq[i] = packed;
         if ((i & 7) == 0) {
@@ -38,13 +31,9 @@ __device__ __forceinline__ void quantize_store_vec4(float4 v, long i, bool live,
 // of the row -> xrow[i], the scale of block i / 8 -> xs_row[i / 8]; g_xq / g_xs (null: skipped) receive the same values.
 __device__ __forceinline__ void quantize_row_vec4(float4 v, int i, bool live, uint32_t *xrow, float *xs_row,
                                                   uint32_t *__restrict__ g_xq, float *__restrict__ g_xs) {
-    float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-    const float d = quant_scale(amax);
-    int sum = 0;
-    const uint32_t packed = amax != 0.0f ? quantize4_pack(v, d, sum) : 0u;
+    float d;
+    int sum;
+    const uint32_t packed = quantize_block_vec4(v, d, sum);
     if (live) {
         xrow[i] = packed;
         if (g_xq) g_xq[i] = packed;
@@ -84,18 +73,12 @@ struct RowQuantizer {
                 const int i = i0 + u * NT;
                 if (i - lane < nvec) {                                              // the same for the whole warp
                     const bool live = i < nvec;
-                    float amax = fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w)));
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-                    const float d = quant_scale(amax);
-                    int sum = 0;
-                    const uint32_t packed = amax != 0.0f ? quantize4_pack(v[u], d, sum) : 0u;
+                    float d;
+                    int sum;
+                    const uint32_t packed = quantize_block_vec4(v[u], d, sum);
                     put(i, packed, d, live);
                     if (store) {
-                        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-                        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-                        sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                        sum = block_sum(sum);
                         if (live) {
                             src.xq[i] = packed;
                             if ((i & 7) == 0) {

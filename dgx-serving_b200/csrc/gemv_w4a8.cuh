@@ -17,6 +17,7 @@
 #pragma once
 #include "common.cuh"
 #include "fused_quantize.cuh"
+#include "ptx_sm100.cuh"
 #include "peer_allgather.cuh"
 
 namespace w4a8 {
@@ -160,7 +161,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_w4a8_dp4a_kernel(
     GemvBatch<U, ST> ba, bb;
     RowQuantizer<WARPS * 32, 6> rq;
     if constexpr (FUSE) {
-        if (tid == 0) prefetch_rows_l2(Wq + (size_t)r0 * wpitch, sw + (size_t)r0 * nb, r1 - r0, (uint32_t)wpitch, nb * sizeof(ST), FUSE_PREFETCH);
+        if (tid == 0) ptx::prefetch_rows_l2(Wq + (size_t)r0 * wpitch, sw + (size_t)r0 * nb, r1 - r0, (uint32_t)wpitch, nb * sizeof(ST), FUSE_PREFETCH);
         pdl_wait();
         rq.load(src, IN / 4, tid);
     }

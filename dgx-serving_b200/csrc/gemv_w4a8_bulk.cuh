@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(THREADS) gemv_w4a8_bulk_kernel(
     }
     __syncthreads();
     if (FUSE) {
-        if (tid == 0) prefetch_rows_l2(Wq + (size_t)r0 * wrow, sw + (size_t)r0 * nb, r1 - r0, wrow, srow, FUSE_PREFETCH);
+        if (tid == 0) ptx::prefetch_rows_l2(Wq + (size_t)r0 * wrow, sw + (size_t)r0 * nb, r1 - r0, wrow, srow, FUSE_PREFETCH);
         pdl_wait();
     }
     pdl_launch_dependents();

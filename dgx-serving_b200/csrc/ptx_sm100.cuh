@@ -88,6 +88,19 @@ __device__ __forceinline__ void tma_prefetch_desc(const void *tmap) {
 __device__ __forceinline__ void prefetch_l2_bulk(const void *gptr, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gptr), "r"(bytes) : "memory");
 }
+// While a kernel waits for the one before it, HBM is idle: about 3 us in a chain of decode steps.  One thread of a CTA asks, ahead of
+// its wait, for the first `budget` bytes of the CTA's contiguous rows of weights (and their scales) to be brought to L2.  Nothing
+// is read into the SM, so this is safe whatever the kernels before write: their stores meet the lines in L2.
+__device__ __forceinline__ void prefetch_rows_l2(const uint8_t *w, const void *s, int rows, uint32_t wrow, uint32_t srow, uint32_t budget) {
+    const int fit = (int)(budget / (wrow + srow)), n = rows < fit ? rows : fit;
+    if (n <= 0) return;
+    const auto range = [](const void *p, uint64_t bytes) {                // the 16-byte pieces inside [p, p + bytes)
+        const uint64_t a = (reinterpret_cast<uint64_t>(p) + 15) & ~15ull, e = (reinterpret_cast<uint64_t>(p) + bytes) & ~15ull;
+        if (e > a) prefetch_l2_bulk(reinterpret_cast<const void *>(a), (uint32_t)(e - a));
+    };
+    range(w, (uint64_t)n * wrow);
+    range(s, (uint64_t)n * srow);
+}
 
 // ---- tensor memory ------------------------------------------------------------------------------
 // Whole-warp calls (.sync.aligned).  ncols: power of two in [32, 512].

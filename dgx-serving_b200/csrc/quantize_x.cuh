@@ -37,16 +37,10 @@ __global__ void __launch_bounds__(256) quantize_x_q8_vec_kernel(const float4 *__
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) {
             long i = i0 + u * stride;
-            float amax = fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w)));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-            const float d = quant_scale(amax);
-            int sum = 0;
-            const uint32_t packed = amax != 0.0f ? quantize4_pack(v[u], d, sum) : 0u;
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+            float d;
+            int sum;
+            const uint32_t packed = quantize_block_vec4(v[u], d, sum);
+            sum = block_sum(sum);
             if (i < nvec) {
                 xq[i] = packed;
                 if ((i & 7) == 0) {
