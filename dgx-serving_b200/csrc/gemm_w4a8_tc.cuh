@@ -1,4 +1,5 @@
-// W4A8 prefill / verify GEMM for sm_100a on the 5th-generation tensor cores.
+// W4A8 prefill GEMM for sm_100a on the 5th-generation tensor cores: the N-sharded GEMM with peer stores and the group-dot dump.
+// (On one GPU gemm_w4a8_mma.cuh is faster for every shape.)
 //   Y[m,n] = sum_b ((float)D[m,n,b] * xs[m,b]) * sw[n,b],   D[m,n,b] = sum_{k in group b} X[m,k]*(Wq[n,k]-8)
 // Semantics and fp32 evaluation order of the reference's kernels/gemm_mmq.cuh:38-120 (t = (float)c*xs,
 // acc = fma(t, sw, acc), groups ascending, :104-105), shared by gemm_mma.cuh, gemm_mmq_tmpl.cuh,

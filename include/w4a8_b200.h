@@ -133,7 +133,7 @@ int w4a8_gemv_multi(const int8_t *xq, const float *xs, int count, const uint8_t 
  * (kernels/gemm_mmq.cuh:222-233, gemm_mmq_tmpl.cuh:100-119), launch_gemm_mmq_raster_w4a8
  * (kernels/gemm_mmq_raster.cuh:115-130), launch_gemm_mma_w4a8 / _bm<BM> (kernels/gemm_mma.cuh:119-132)
  * and launch_gemm_mmq_ms (kernels/gemm_mmq_ms.cuh).  Note the (M,N,K) argument order of this family.
- * Y[M,N] fp32 row-major.  Integer group dots come from int8 MMAs (mma.sync or tcgen05, see "gemm_kernel") and are exact; the fp32
+ * Y[M,N] fp32 row-major.  Integer group dots come from MMAs (see "gemm_kernel" for which) and are exact; the fp32
  * epilogue evaluates t = (float)D*xs[m,b]; acc = fma(t, sw[n,b], acc) for b ascending, the order of
  * kernels/gemm_mmq.cuh:104-105, so results match the reference MMQ kernels bit for bit.
  * Needs X and Wq 16-byte aligned (TMA); M, N arbitrary. */
@@ -187,7 +187,8 @@ int w4a8_group_dots(const int8_t *xq, const uint8_t *Wq, int32_t *D, int M, int 
  * Replaces the static mm()/MMs()/mmb() dispatchers of the model graphs (models/qwen35_decode.cu:51-62,
  * models/qwen35_batch.cu:120-139, models/gemma4_decode.cu:113-129): quantize X[S,K] into the caller's
  * scratch (xq, xs, xsum as for w4a8_quantize_x_q8) unless skip_quantize != 0 (the G4_QUANT_SHARE case,
- * models/gemma4_decode.cu:115), then S <= 16 -> w4a8_gemv, else -> w4a8_gemm. */
+ * models/gemma4_decode.cu:115), then S <= 16 -> w4a8_gemv, else -> w4a8_gemm.  One row of device memory goes in a
+ * single launch where that is faster; xq, xs, xsum and Y get the same bits either way. */
 int w4a8_linear(const float *X, int8_t *xq, float *xs, int32_t *xsum, const uint8_t *Wq, const void *sw,
                 float *Y, int S, int N, int K, int scale_dtype, int skip_quantize, void *stream);
 
