@@ -41,7 +41,10 @@ namespace w4a8 {
 namespace gemm_mma {
 
 constexpr int GPK = 4;                    // groups per K-tile
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+// bytes = 0 writes zeros and reads nothing
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -124,7 +127,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     }
     const int nkt = (g1 - g0 + GPK - 1) / GPK;
 
-    // ---- copies.  Rows past the end come from the next expert or are zeros (their scales are the last row's) and never stored.
+    // ---- copies.  Rows and columns past the end come from the next expert or are zeros, and are never stored.
     // The thread that starts the bulk copies.  Where one warp copies all of the activations' scales besides, it is one of the last
     // warp: 16 x 18944 x 5120 24.8 us by the first thread, 23.1 so; 192 x 9472 x 5120 56.6 and 59.1.
     constexpr int ISSUER = !GROUPED && BM <= 32 ? NT - 32 : 0;
@@ -139,6 +142,14 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     __syncthreads();
     static_assert(!GROUPED || C::WM == 1, "an item's live tiles are every warp's");
     const int live = GROUPED ? min(TM, (mend - m0 + 15) / 16) : TM;            // live m16 tiles
+    // Scales past the end: the address is the last row's, the 16-byte copies (which pass L1 by) read nothing from it.  When they did,
+    // all lanes past the end of all CTAs of a column, or of all CTAs with few rows, asked L2 for the same 16 bytes:
+    // 2034 x 162 x 5376 67.6 us, 30.7 so; one row x 18944 x 5120 29.4, 22.7 so.
+    int bytes_a[C::RA], bytes_b[C::RB];
+#pragma unroll
+    for (int r = 0; r < C::RA; r++) bytes_a[r] = m0 + tid + r * NT < mend ? 16 : 0;
+#pragma unroll
+    for (int r = 0; r < C::RB; r++) bytes_b[r] = n0 + tid + r * NT < N ? 16 : 0;
     auto copy = [&](int kt, bool ok) {
         if (kt < nkt) {
             const int b0 = g0 + kt * GPK, ng = FULL ? GPK : g1 - b0;          // groups left
@@ -160,14 +171,14 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
 #pragma unroll
                 for (int r = 0; r < C::RA; r++) {
                     const int m = tid + r * NT;
-                    if (BM % NT == 0 || m < BM) cp_async16(smem_u + so + C::OFF_SX + m * (GPK * 4), xs + (size_t)min(m0 + m, mend - 1) * nb + b0);
+                    if (BM % NT == 0 || m < BM) cp_async16(smem_u + so + C::OFF_SX + m * (GPK * 4), xs + (size_t)min(m0 + m, mend - 1) * nb + b0, bytes_a[r]);
                 }
 #pragma unroll
                 for (int r = 0; r < C::RB; r++) {
                     const int n = tid + r * NT;
                     if (BN % NT == 0 || n < BN) {
                         const ST *p = sw + (wrow0 + min(n0 + n, N - 1)) * (size_t)nb + b0;
-                        if (sizeof(ST) == 4) cp_async16(smem_u + so + C::OFF_SW + n * (GPK * 4), p);
+                        if (sizeof(ST) == 4) cp_async16(smem_u + so + C::OFF_SW + n * (GPK * 4), p, bytes_b[r]);
                         else cp_async8(smem_u + so + C::OFF_SW + n * (GPK * 4), p);
                     }
                 }
