@@ -96,7 +96,21 @@ __device__ __forceinline__ float sval(__half x) { return __half2float(x); }
 // fp32 scale, where it is exact.  Cost: 3 logic ops per 8 weights, no per-byte subtraction.
 //   even: bytes = 16*w[0], 16*w[2], 16*w[4], 16*w[6]   (the word's low nibbles)
 //   odd : bytes = 16*w[1], 16*w[3], 16*w[5], 16*w[7]   (the word's high nibbles)
+// The three-input logic instruction by hand: from the C expression the compiler makes two instructions of one constant each, ten for
+// the two words of a tensor instruction's operand instead of six (counted under ncu).  Half-rate ones: they are what the decode
+// kernels for 8 and 16 rows and the experts' run out of.  us, expression / this: 16 x 17408 x 5120 fp16 scales three times 65.8 / 58.9,
+// expert block of 8 rows 40.6 / 38.6, 333 x 15360 x 3840 122.9 / 118.9, one row x 151936 x 5120 71.1 / 69.6.
+__device__ __forceinline__ uint32_t and_xor(uint32_t a, uint32_t mask, uint32_t x) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(r) : "r"(a), "r"(mask), "r"(x));
+    return r;
+}
 __device__ __forceinline__ void unpack8_x16(uint32_t w, uint32_t &even, uint32_t &odd) {
+    odd = and_xor(w, 0xF0F0F0F0u, 0x80808080u);
+    even = and_xor(w << 4, 0xF0F0F0F0u, 0x80808080u);
+}
+// The same, left to the compiler.
+__device__ __forceinline__ void unpack8_x16_expr(uint32_t w, uint32_t &even, uint32_t &odd) {
     odd = (w & 0xF0F0F0F0u) ^ 0x80808080u;
     even = ((w << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
 }

@@ -41,6 +41,7 @@ namespace w4a8 {
 namespace gemm_mma {
 
 constexpr int GPK = 4;                    // groups per K-tile
+constexpr unsigned SMS = 148;             // of a B200: the first 148 CTAs of a launch are on an SM each, the next 148 beside them
 // bytes = 0 writes zeros and reads nothing
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, int bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
@@ -102,7 +103,7 @@ struct GroupList {
 template <class C, typename ST, bool GROUPED, bool VEC>
 __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const float *__restrict__ xs, const ST *__restrict__ sw,
-    float *__restrict__ Y, int M, int N, int K, int m_tiles, int n_tiles, int gsplit, bool pairs, const GroupList gl) {
+    float *__restrict__ Y, int M, int N, int K, int m_tiles, int n_tiles, int gsplit, bool pairs, int stagger, const GroupList gl) {
     extern __shared__ __align__(1024) unsigned char smem[];
     constexpr int TM = C::TM, TN = C::TN, BM = C::BM, BN = C::BN, NT = C::THREADS, STAGES = C::STAGES;
     constexpr bool FULL = VEC;                             // scales that line up make every K-tile complete: 1 to 10 % faster when known here
@@ -133,6 +134,11 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     constexpr int ISSUER = !GROUPED && BM <= 32 ? NT - 32 : 0;
     const uint32_t smem_u = (uint32_t)__cvta_generic_to_shared(smem);
     auto FULL_BAR = [&](int i) { return smem_u + C::OFF_BAR + 8u * i; };
+    // The second CTA of an SM starts `stagger` cycles after the first (host side: stagger_cycles).
+    if (C::CTAS == 2 && !GROUPED && stagger > 0 && blockIdx.x < 2 * SMS && blockIdx.x >= SMS) {
+        const long long t1 = clock64() + stagger;
+        while (clock64() < t1) __nanosleep(200);
+    }
     if (tid == 0) {
         for (int i = 0; i < STAGES; i++) ptx::mbar_init(FULL_BAR(i), 1);
         ptx::mbar_fence_init();
@@ -245,7 +251,12 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
                 }
             }
             uint32_t b0, b1;
-            unpack8_x16(*reinterpret_cast<const uint32_t *>(Bs + (boff ^ ((bfirst + bg) << 4)) + j * 512), b0, b1);
+            // two tiles that ptxas orders worse with the shorter form (64 rows, fp32 scales: 768 x 9000 x 3840 156 us, 164 with it, 1024 x 17408 x
+            // 5120 504 and 560; 80 rows, fp16: 2048 x 17408 x 5120 952 and 966); every other one gains, up to 11 %
+            constexpr bool EXPR = !GROUPED && ((TM == 4 && sizeof(ST) == 4) || (TM == 5 && sizeof(ST) == 2));
+            const uint32_t word = *reinterpret_cast<const uint32_t *>(Bs + (boff ^ ((bfirst + bg) << 4)) + j * 512);
+            if constexpr (EXPR) unpack8_x16_expr(word, b0, b1);
+            else unpack8_x16(word, b0, b1);
             sv[q & 1][0] = sval(*reinterpret_cast<const ST *>(ss + bg * sizeof(ST) + 8 * j * (GPK * 4)));
             sv[q & 1][1] = sval(*reinterpret_cast<const ST *>(ss + bg * sizeof(ST) + (8 * j + 1) * (GPK * 4)));
 #pragma unroll
@@ -336,6 +347,18 @@ template <typename ST>
 inline bool scales_pair_up(const ST *sw, int K, int nsplit, int gsplit) {
     return (K / QBLK) % 2 == 0 && (nsplit == 1 || gsplit % 2 == 0) && aligned(sw, 4);
 }
+// Two CTAs of an SM that start together end together, and those of the last wave then pair up on the SMs that come free first; they
+// also want the same pipes at the same time.  So where there is more than one wave the second CTA of an SM starts 5 % of a tile's time
+// later, which is more than SMs differ by.  us, without / with: 768 x 9000 x 3840 in 80-row tiles 173 / 152, fp16 scales 182 / 167;
+// 500 x 9000 x 2048 in 96-row tiles 79 / 69; 1500 x 5000 x 4096 in 96-row tiles, fp16, 216 / 191; 2048 x 17408 x 5120 911 / 905.  Where
+// nothing pairs up it costs up to 1.5 %: 768 x 9000 x 3840 in 96-row tiles 144.6 / 145.9.  2 % of a tile's time is too little (172.8 in
+// the first case), 10 % dearer.  Three and four CTAs per SM drift apart by themselves (48 rows: 154.8 / 155.1; 333 x 15360 x 3840
+// 116 / 118).  Not on a chip whose number of SMs is another one.
+inline int stagger_cycles(long ctas, int per_sm, int rows, int groups) {
+    if (per_sm != 2 || sm_count() != (int)SMS || ctas <= 2 * (long)SMS) return 0;
+    const long cycles = (long)groups * rows * 12 / 20;         // a group of a tile's row takes about 12 cycles with two CTAs on the SM
+    return (int)(cycles < 100000 ? cycles : 100000);
+}
 template <class C, typename ST, bool GROUPED, bool VEC>
 inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int M, int N, int K, int nsplit,
                     int gsplit, cudaStream_t st, const GroupList &gl = GroupList(), int max_items = 0, long w_rows = 0) {
@@ -355,7 +378,8 @@ inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const S
     const bool pairs = scales_pair_up(sw, K, nsplit, gsplit);
     const long units = GROUPED ? (long)max_items * n_tiles : (long)m_tiles * n_tiles * nsplit;
     if (units > 0x7FFFFFFFL) return fail(W4A8_ERR_UNSUPPORTED, "gemm: %ld work units", units);
-    kern<<<(unsigned)units, C::THREADS, C::SMEM, st>>>(tmX, tmW, xs, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs, gl);
+    kern<<<(unsigned)units, C::THREADS, C::SMEM, st>>>(tmX, tmW, xs, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs,
+                                                       GROUPED ? 0 : stagger_cycles(units, C::CTAS, C::BM, nsplit > 1 ? gsplit : K / QBLK), gl);
     return launch_status("gemm_w4a8_mma");
 }
 
