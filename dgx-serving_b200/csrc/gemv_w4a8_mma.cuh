@@ -32,6 +32,7 @@ constexpr int WARPS = W4A8_MMA_WARPS;
 #define W4A8_GEMV_RELAY 1
 #endif
 constexpr bool RELAY = W4A8_GEMV_RELAY != 0;
+constexpr int RELAY16_TILES = 2;                 // 9 to 16 rows: most 16-row tiles of a CTA that are relayed
 // A step = 16 weight rows x GS groups (GS * 16 B contiguous per row) plus the 16 x GS scales (slot sized for fp32).
 __host__ __device__ constexpr int step_w(int GS) { return 16 * GS * 16; }
 __host__ __device__ constexpr int step_bytes(int GS) { return 16 * GS * 16 + 16 * GS * 4; }
@@ -51,7 +52,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr) : "memory");
+                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
 }
 // D(16x8, s32) = A(16x32, s8, row) * B(32x8, s8, col); accumulators start at zero.
 __device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -97,13 +98,14 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
     // When the CTA has fewer tiles than warps (narrow matrices), the idle warps' ring slots are lent to the working
     // ones: a warp that is alone with a long row range needs more bytes in flight to stream at full speed.
     int mult = 1;
-    // Narrow matrices, MH == 1: K relay.  A CTA with at most WARPS/2 tiles gives each tile KS warps; warp (tile, ks)
-    // streams steps ks, ks + KS, ... of the tile and computes their products t = (float)D * xs, and the fp32
-    // accumulators travel from the warp of step q to the warp of step q + 1 through a mailbox in shared memory, so
-    // that every accumulator still sees its groups in ascending order (the bits do not change) while KS rings of
-    // copies are in flight per tile instead of one.
+    // Narrow matrices: K relay (for more than eight rows where a step is eight groups, whose products fit the registers).  A CTA
+    // with at most WARPS/2 tiles gives each tile KS warps; warp (tile, ks) streams steps ks, ks + KS, ... of the tile and computes
+    // their products t = (float)D * xs, and the fp32 accumulators travel from the warp of step q to the warp of step q + 1 through a
+    // mailbox in shared memory, so that every accumulator still sees its groups in ascending order (the bits do not change) while KS
+    // rings of copies are in flight per tile instead of one.
+    constexpr bool CAN_RELAY = RELAY && (MH == 1 || GS == 8);
     int KS = 1;
-    if (MH == 1 && RELAY) while (KS < WARPS && ntiles_cta * KS * 2 <= WARPS) KS *= 2;
+    if (CAN_RELAY && (MH == 1 || ntiles_cta <= RELAY16_TILES)) while (KS < WARPS && ntiles_cta * KS * 2 <= WARPS) KS *= 2;
     if (KS == 1) while (mult < 4 && ntiles_cta * mult * 2 <= WARPS) mult *= 2;
     const int rtile = warp / KS, rks = warp % KS;            // relay: tile of this warp inside the CTA, first step
     const int depth = STAGES * mult;
@@ -114,36 +116,51 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
 
     // Producer side of the warp's ring: copies of the next step (tile it, step iq) into slot isl.  One weight-copy
     // instruction covers 32/GS rows x GS*16 contiguous bytes each.
+    // The addresses of a lane's pieces advance by whole steps: computed per copy they were a sixth of the kernel's instructions (34.0 of a
+    // tile's group, 30.9 so; 8 x 15360 x 3840 9.3 us, 9.0 so; 9 x 151936 x 2048 fp16 46.2 and 41.7).  Rows past the end repeat the last
+    // one (and are never stored).
     int it = 0, iq = KS > 1 ? rks : 0, isl = 0;
+    constexpr int RPI = 32 / GS, NW = 16 / RPI;                  // rows per copy instruction, copy instructions of a step
+    constexpr int SP = sizeof(ST) == 4 ? GS / 4 : GS / 8, NS = (16 * SP + 31) / 32;   // 16-byte scale pieces per row
+    const int lr = lane / GS, lj = lane % GS;
+    const uint8_t *wbase = Wq + (size_t)u0 * 8 * wpitch;        // 32-bit offsets from the CTA's first row (launch_p: its rows are under 2 GB)
+    const unsigned char *sbase = reinterpret_cast<const unsigned char *>(sw + (size_t)u0 * 8 * nb);
+    const int last = OUT - 1 - u0 * 8;
+    uint32_t woff[NW], soff[NS];
+    auto tile_rows = [&]() {
+        const int base = 16 * (KS > 1 ? rtile : warp + it * WARPS);
+#pragma unroll
+        for (int i = 0; i < NW; i++) woff[i] = (uint32_t)min(base + i * RPI + lr, last) * (uint32_t)(IN / 2) + (uint32_t)(iq * GS + lj) * 16;
+#pragma unroll
+        for (int i = 0; i < NS; i++) {
+            const int pc = i * 32 + lane;
+            soff[i] = (uint32_t)min(base + pc / SP, last) * (uint32_t)(nb * sizeof(ST)) + (uint32_t)(iq * GS * sizeof(ST) + pc % SP * 16);
+        }
+    };
+    if (my_tiles > 0) tile_rows();
     auto issue = [&]() {
         if (it < my_tiles) {
-            const int base = (u0 + 2 * (KS > 1 ? rtile : warp + it * WARPS)) * 8;
             const uint32_t slot = ring_u32 + (uint32_t)isl * STEP_BYTES;
-            constexpr int RPI = 32 / GS;                         // rows per copy instruction
-            const int lr = lane / GS, lj = lane % GS;
 #pragma unroll
-            for (int i = 0; i < 16 / RPI; i++) {
+            for (int i = 0; i < NW; i++) {
                 const int r = i * RPI + lr;
-                int row = base + r;
-                row = row < OUT ? row : OUT - 1;                 // rows past the end re-read the last row; never stored
-                cp_async16_cg(slot + r * (GS * 16) + ((lj ^ swz(r, GS)) << 4), Wq + (size_t)row * wpitch + (size_t)(iq * GS + lj) * 16);
+                cp_async16_cg(slot + r * (GS * 16) + ((lj ^ swz(r, GS)) << 4), wbase + woff[i]);
+                woff[i] += KS * GS * 16;
             }
-            constexpr int SP = sizeof(ST) == 4 ? GS / 4 : GS / 8;   // 16-byte scale pieces per row
 #pragma unroll
-            for (int i = 0; i < (16 * SP + 31) / 32; i++) {
+            for (int i = 0; i < NS; i++) {
                 const int pc = i * 32 + lane;
-                if (pc < 16 * SP) {
-                    const int r = pc / SP, k = pc % SP;
-                    int row = base + r;
-                    row = row < OUT ? row : OUT - 1;
-                    cp_async16_ca(slot + STEP_W + r * (GS * (int)sizeof(ST)) + k * 16,
-                                  reinterpret_cast<const unsigned char *>(sw + (size_t)row * nb + iq * GS) + k * 16);
-                }
+                if (16 * SP % 32 == 0 || pc < 16 * SP) cp_async16_ca(slot + STEP_W + (pc / SP) * (GS * (int)sizeof(ST)) + pc % SP * 16, sbase + soff[i]);
+                soff[i] += KS * GS * (int)sizeof(ST);
             }
         }
         cp_async_commit();                                        // one group per step, also when empty
         iq += KS;
-        if (iq >= nsteps) { iq = KS > 1 ? rks : 0; it++; }
+        if (iq >= nsteps) {
+            iq = KS > 1 ? rks : 0;
+            it++;
+            if (it < my_tiles) tile_rows();
+        }
         if (++isl == depth) isl = 0;
     };
 
@@ -202,7 +219,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
             }
         }
     }
-    __shared__ float4 relay_box[WARPS / 2][32];
+    __shared__ float4 relay_box[WARPS / 2][MH][32];
     __shared__ unsigned int relay_flag[WARPS / 2];
     if (tid < WARPS / 2) relay_flag[tid] = 0u;
     for (int i0 = tid; i0 < nb * 8 * MH; i0 += NT * 4) {
@@ -223,8 +240,11 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
     float acc[MH][4];
     // ldmatrix row address of this lane inside a slot: matrix i = lane/8 -> rows (i&1)*8.., group 2*jj + (i>>1)
     const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lgrp = lane >> 4;
+    const uint2 *xrow[MH];                                        // this lane's row of each half; rows from S on repeat the last one and are never stored
+#pragma unroll
+    for (int h = 0; h < MH; h++) xrow[h] = xqp + (size_t)min(8 * h + g, S - 1) * pitch2 + t;
     int csl = 0;
-    if (MH == 1 && RELAY && KS > 1) {
+    if (CAN_RELAY && KS > 1) {
         if (my_tiles > 0) {
             volatile unsigned int *flag = &relay_flag[rtile];
             bool alive = true;
@@ -235,7 +255,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
                 const uint32_t slot = ring_u32 + (uint32_t)csl * STEP_BYTES;
                 const unsigned char *slot_p = ring + (size_t)csl * STEP_BYTES;
                 // ---- all products of this step first: tb[j][i] = (float)D * xs for group j of the step
-                float tb[GS][4];
+                float tb[GS][MH][4];
 #pragma unroll
                 for (int j2 = 0; j2 < GS / 2; j2++) {
                     uint32_t w[4];
@@ -246,16 +266,19 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
                         uint32_t a0, a1, a2, a3;
                         unpack8_x16(w[2 * k], a0, a2);
                         unpack8_x16(w[2 * k + 1], a1, a3);
-                        const uint2 bx = (g < S) ? xqp[(size_t)g * pitch2 + 4 * b + t] : make_uint2(0u, 0u);
-                        int c[4];
-                        mma_s8(c, a0, a1, a2, a3, bx.x, bx.y);
-                        const float2 xv = *reinterpret_cast<const float2 *>(sxs + (size_t)b * 8 + 2 * t);
-                        tb[j][0] = (float)c[0] * xv.x; tb[j][1] = (float)c[1] * xv.y;
-                        tb[j][2] = (float)c[2] * xv.x; tb[j][3] = (float)c[3] * xv.y;
+#pragma unroll
+                        for (int h = 0; h < MH; h++) {
+                            const uint2 bx = xrow[h][4 * b];
+                            int c[4];
+                            mma_s8(c, a0, a1, a2, a3, bx.x, bx.y);
+                            const float2 xv = *reinterpret_cast<const float2 *>(sxs + (size_t)b * 8 * MH + 8 * h + 2 * t);
+                            tb[j][h][0] = (float)c[0] * xv.x; tb[j][h][1] = (float)c[1] * xv.y;
+                            tb[j][h][2] = (float)c[2] * xv.x; tb[j][h][3] = (float)c[3] * xv.y;
+                        }
                     }
                 }
                 // ---- take the accumulators over from the warp of step q - 1 (bounded wait)
-                float a[4] = {0.f, 0.f, 0.f, 0.f};
+                float a[MH][4] = {};
                 if (q > 0) {
                     unsigned int n = 0;
                     while (*flag < (unsigned)q) {
@@ -264,8 +287,11 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
                     alive = __all_sync(0xffffffffu, alive);
                     if (!alive) break;
                     __threadfence_block();
-                    const float4 v = relay_box[rtile][lane];
-                    a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
+#pragma unroll
+                    for (int h = 0; h < MH; h++) {
+                        const float4 v = relay_box[rtile][h][lane];
+                        a[h][0] = v.x; a[h][1] = v.y; a[h][2] = v.z; a[h][3] = v.w;
+                    }
                 }
                 // ---- this step's groups, ascending
 #pragma unroll
@@ -285,28 +311,36 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
 #pragma unroll
                     for (int js = 0; js < 4; js++) {
                         const int j = 4 * j4 + js;
-                        a[0] = fmaf(tb[j][0], swA[js], a[0]);
-                        a[1] = fmaf(tb[j][1], swA[js], a[1]);
-                        a[2] = fmaf(tb[j][2], swB[js], a[2]);
-                        a[3] = fmaf(tb[j][3], swB[js], a[3]);
+#pragma unroll
+                        for (int h = 0; h < MH; h++) {
+                            a[h][0] = fmaf(tb[j][h][0], swA[js], a[h][0]);
+                            a[h][1] = fmaf(tb[j][h][1], swA[js], a[h][1]);
+                            a[h][2] = fmaf(tb[j][h][2], swB[js], a[h][2]);
+                            a[h][3] = fmaf(tb[j][h][3], swB[js], a[h][3]);
+                        }
                     }
                 }
                 if (q + 1 < nsteps) {                          // hand over to the warp of step q + 1
-                    relay_box[rtile][lane] = make_float4(a[0], a[1], a[2], a[3]);
+#pragma unroll
+                    for (int h = 0; h < MH; h++) relay_box[rtile][h][lane] = make_float4(a[h][0], a[h][1], a[h][2], a[h][3]);
                     __threadfence_block();
                     __syncwarp();
                     if (lane == 0) *flag = (unsigned)(q + 1);
                 } else {                                       // last step: these are the outputs
                     const int base = (u0 + 2 * rtile) * 8;
                     const int lim = min(OUT, u1 * 8);
-                    const int m0 = 2 * t, rA = base + g, rB = base + 8 + g;
-                    if (rA < lim) {
-                        if (m0 < S) store_out<PEER>(Y, oa, OUT, m0, rA, a[0]);
-                        if (m0 + 1 < S) store_out<PEER>(Y, oa, OUT, m0 + 1, rA, a[1]);
-                    }
-                    if (rB < lim) {
-                        if (m0 < S) store_out<PEER>(Y, oa, OUT, m0, rB, a[2]);
-                        if (m0 + 1 < S) store_out<PEER>(Y, oa, OUT, m0 + 1, rB, a[3]);
+                    const int rA = base + g, rB = base + 8 + g;
+#pragma unroll
+                    for (int h = 0; h < MH; h++) {
+                        const int m0 = 8 * h + 2 * t;
+                        if (rA < lim) {
+                            if (m0 < S) store_out<PEER>(Y, oa, OUT, m0, rA, a[h][0]);
+                            if (m0 + 1 < S) store_out<PEER>(Y, oa, OUT, m0 + 1, rA, a[h][1]);
+                        }
+                        if (rB < lim) {
+                            if (m0 < S) store_out<PEER>(Y, oa, OUT, m0, rB, a[h][2]);
+                            if (m0 + 1 < S) store_out<PEER>(Y, oa, OUT, m0 + 1, rB, a[h][3]);
+                        }
                     }
                 }
                 __syncwarp();                                  // the slot is refilled by the next iteration's copies
@@ -354,7 +388,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
 #pragma unroll
                         for (int h = 0; h < MH; h++) {
                             // activation row m = 8h + g of this lane; rows beyond S contribute zeros and are not staged
-                            const uint2 bx = (8 * h + g < S) ? xqp[(size_t)(8 * h + g) * pitch2 + 4 * b + t] : make_uint2(0u, 0u);
+                            const uint2 bx = xrow[h][4 * b];
                             int c[4];
                             mma_s8(c, a0, a1, a2, a3, bx.x, bx.y);
                             const float2 xv = *reinterpret_cast<const float2 *>(sxs + (size_t)b * 8 * MH + 8 * h + 2 * t);
@@ -395,17 +429,22 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
 struct Plan { int MH, GS, STAGES; };
 constexpr size_t SMEM_LIMIT = 224 * 1024;
 inline int env_int(const char *name, int dflt) { const char *e = getenv(name); return e ? atoi(e) : dflt; }
-inline bool plan_for(const void *Wq, const void *sw, int IN, int S, Plan *p) {
+inline bool plan_for(const void *Wq, const void *sw, int IN, int OUT, int S, Plan *p) {
     const int nb = IN / QBLK;
     if (IN <= 0 || nb % 8 != 0) return false;
     if (!aligned(Wq, 16) || !aligned(sw, 16)) return false;
     static const int want_gs = env_int("W4A8_GEMV_GS", 16);
     static const int want_st = env_int("W4A8_GEMV_STAGES", 0);
     const int MH = S > 8 ? 2 : 1;
+    // 9 to 16 rows of a matrix with at most two tiles per CTA: steps of eight groups, which the relay takes.  us, one warp a tile /
+    // relay: 16 x 2048 x 8192 16.7 / 11.3, 16 x 4096 x 3840 8.9 / 7.3 (fp16 9.5 / 7.3), 10 x 2500 x 2304 fp16 6.5 / 5.2, 9 x 2048 x 2048
+    // 4.7 / 4.2.  With three or four tiles two warps each gain nothing (12 x 5120 x 5120 10.6 / 11.0, 16 x 9472 x 4096 9.4 / 10.1),
+    // nor do rows of a few steps (12 x 4000 x 512 2.8 / 3.2).
+    const bool relay16 = RELAY && MH == 2 && nb >= 48 && ((long)OUT + 7) / 8 <= (long)sm_count() * 2 * RELAY16_TILES;
     const int gs_opts[2] = {16, 8};
     for (int gi = 0; gi < 2; gi++) {
         const int GS = gs_opts[gi];
-        if (GS > want_gs || nb % GS != 0) continue;
+        if (GS > want_gs || nb % GS != 0 || (GS == 16 && relay16)) continue;
         const int st_opts[3] = {GS == 16 ? 4 : 8, GS == 16 ? 3 : 6, GS == 16 ? 2 : 3};
         for (int si = 0; si < 3; si++)
             if (st_opts[si] <= (want_st > 0 ? want_st : (GS == 16 ? 2 : 3)))
@@ -430,6 +469,7 @@ inline int launch_p(const int8_t *xq, const float *xs, const uint8_t *Wq, const 
     const int units = (OUT + 7) / 8;
     long want = (units + 1) / 2;                         // at least one 16-row tile per CTA
     long cap = sm_count();                               // one persistent CTA per SM
+    while ((units / cap + 2) * 8l * (IN / 2) >= (1l << 31)) cap *= 2;   // the copies' offsets are 32-bit
     const dim3 grid((unsigned)(want < cap ? want : cap));
     cudaError_t le = launch_pdl(kern, grid, dim3(WARPS * 32), smem, st, xq, xs, Wq, sw, Y, IN, OUT, S, oa);
     if (le != cudaSuccess) return cuda_fail(le, "gemv_w4a8_mma launch");

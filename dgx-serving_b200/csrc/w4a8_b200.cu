@@ -218,14 +218,14 @@ static int gemv_dispatch(const int8_t *xq, const float *xs, const uint8_t *Wq, c
         // rows go in passes of up to 16 (8 when 16 rows of activations do not fit in shared memory next to the ring)
         gemv_mma::Plan plan;
         int per = S < 16 ? S : 16;
-        bool ok = gemv_mma::plan_for(Wq, sw, IN, per, &plan);
-        if (!ok && per > 8) { per = 8; ok = gemv_mma::plan_for(Wq, sw, IN, per, &plan); }
+        bool ok = gemv_mma::plan_for(Wq, sw, IN, OUT, per, &plan);
+        if (!ok && per > 8) { per = 8; ok = gemv_mma::plan_for(Wq, sw, IN, OUT, per, &plan); }
         if (ok) {
             if (count_only) { *count_only = (S + per - 1) / per; return W4A8_OK; }
             for (int s0 = 0; s0 < S; s0 += per) {
                 const int s = S - s0 < per ? S - s0 : per;
                 gemv_mma::Plan pl = plan;
-                if (s <= 8 && pl.MH == 2) gemv_mma::plan_for(Wq, sw, IN, s, &pl);
+                if (s <= 8 && pl.MH == 2) gemv_mma::plan_for(Wq, sw, IN, OUT, s, &pl);
                 OutArgs oa = oa_in;
                 if (oa.peers) oa.y_off += (size_t)s0 * oa.ld * sizeof(float);
                 int rc = gemv_mma::launch(xq + (size_t)s0 * IN, xs + (size_t)s0 * (IN / QBLK), Wq, sw, Y + (size_t)s0 * OUT, IN, OUT, s,
@@ -497,7 +497,7 @@ static int linear_row(const float *X, int8_t *xq, float *xs, int32_t *xsum, cons
     gemv_bulk::Plan bp;
     const bool bulk_plan = pol != 1 && gemv_bulk::plan_for(xq, Wq, sw, K, scale_dtype, &bp);
     // fp16 scales: where the general way takes the tensor path for one row, its fp32 order is another one
-    if (pol == 0 && scale_dtype == 1 && !(K >= 2048 && bulk_plan) && gemv_mma::plan_for(Wq, sw, K, 1, &mp)) return W4A8_OK;
+    if (pol == 0 && scale_dtype == 1 && !(K >= 2048 && bulk_plan) && gemv_mma::plan_for(Wq, sw, K, N, 1, &mp)) return W4A8_OK;
     const bool bulk_fits = bulk_plan && bp.smem + gemv_bulk::row_bytes(K) <= 227 * 1024;
     const size_t wbytes = (size_t)N * ((size_t)K / 2 + (size_t)(K / QBLK) * (scale_dtype == 1 ? 2 : 4));
     // Which of the two streams, us per linear of one row, dp4a / bulk.  fp32 scales: the bulk copies win where a lane has five or six
