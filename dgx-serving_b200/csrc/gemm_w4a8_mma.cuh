@@ -116,6 +116,8 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
     int m0, mend, n0, g0 = 0, g1 = nb, split = 0;
     size_t wrow0 = 0;
     if (GROUPED) {
+        pdl_wait();                                        // the items and the rows come from the kernel before this one
+        pdl_launch_dependents();
         const int item = blockIdx.x / n_tiles;
         if (item >= *gl.num_items) return;
         const int4 it = __ldg(gl.items + item);
@@ -378,7 +380,10 @@ inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const S
     const bool pairs = scales_pair_up(sw, K, nsplit, gsplit);
     const long units = GROUPED ? (long)max_items * n_tiles : (long)m_tiles * n_tiles * nsplit;
     if (units > 0x7FFFFFFFL) return fail(W4A8_ERR_UNSUPPORTED, "gemm: %ld work units", units);
-    kern<<<(unsigned)units, C::THREADS, C::SMEM, st>>>(tmX, tmW, xs, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs,
+    if (GROUPED) {
+        const cudaError_t e = launch_pdl(kern, dim3((unsigned)units), dim3(C::THREADS), C::SMEM, st, tmX, tmW, xs, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs, 0, gl);
+        if (e != cudaSuccess) return cuda_fail(e, "gemm_w4a8_mma launch");
+    } else kern<<<(unsigned)units, C::THREADS, C::SMEM, st>>>(tmX, tmW, xs, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs,
                                                        GROUPED ? 0 : stagger_cycles(units, C::CTAS, C::BM, nsplit > 1 ? gsplit : K / QBLK), gl);
     return launch_status("gemm_w4a8_mma");
 }

@@ -70,9 +70,8 @@ inline Layout layout_for(int S, int topk, int H, int MI, int experts) {
 //   4. every warp walks its segment 32 slots at a time: a slot's position = its warp's running position for the
 //      expert + its rank among the equal ids of the 32 (match_any), so an expert's rows keep the slots' order.
 // More than FAST_EXPERTS experts: step 4 is done expert by expert (a warp takes an expert and walks all slots).
-__global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t *__restrict__ idx, int nslots, int expert_base, int experts,
-                                                        int *__restrict__ perm, int *__restrict__ pos, int *__restrict__ offsets,
-                                                        int4 *__restrict__ items, int *__restrict__ num_items) {
+__device__ void sort_slots(const int32_t *__restrict__ idx, int nslots, int expert_base, int experts, int *__restrict__ perm, int *__restrict__ pos,
+                           int *__restrict__ offsets, int4 *__restrict__ items, int *__restrict__ num_items) {
     constexpr int FAST_EXPERTS = 256, NW = 32;
     __shared__ int cnt[MAX_EXPERTS];
     __shared__ int off[MAX_EXPERTS + 1];
@@ -163,10 +162,24 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t *__restric
     }
 }
 
+// The first CTA sorts the slots; the others, if any, quantize the tokens meanwhile (nvec vectors of eight elements, quantize_x_q8_wide_kernel).
+// The sort is one CTA's chain of 10 us, the quantizer 5 us of all the others: one launch instead of two saves the latter.
+__global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t *__restrict__ idx, int nslots, int expert_base, int experts,
+                                                        int *__restrict__ perm, int *__restrict__ pos, int *__restrict__ offsets,
+                                                        int4 *__restrict__ items, int *__restrict__ num_items, const float *__restrict__ X,
+                                                        uint2 *__restrict__ xq, float *__restrict__ xs, long nvec) {
+    pdl_wait();
+    pdl_launch_dependents();
+    if (blockIdx.x == 0) sort_slots(idx, nslots, expert_base, experts, perm, pos, offsets, items, num_items);
+    else quantize_wide(X, xq, xs, nullptr, nvec, (long)(blockIdx.x - 1) * blockDim.x + threadIdx.x, (long)(gridDim.x - 1) * blockDim.x);
+}
+
 // Sorted row p < offsets[experts] gets the quantized activations of its token perm[p] / topk.
 __global__ void __launch_bounds__(128) moe_gather_rows_kernel(const int8_t *__restrict__ xq, const float *__restrict__ xs,
                                                               const int *__restrict__ perm, const int *__restrict__ count, int topk, int K,
                                                               int8_t *__restrict__ xq_g, float *__restrict__ xs_g) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int n = *count, nb = K / QBLK;
     for (int p = blockIdx.x; p < n; p += gridDim.x) {
         const int tok = perm[p] / topk;
@@ -187,19 +200,30 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float4 *__restri
     pdl_launch_dependents();
     pdl_wait();   // the down outputs come from the kernel before this one
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        const long b = i / H4;
+        const long b = total < (1L << 31) ? (long)((uint32_t)i / (uint32_t)H4) : i / H4;
         const int o = (int)(i - b * H4);
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int k = 0; k < topk; k++) {
-            const long slot = b * topk + k;
-            const long row = pos ? pos[slot] : slot;
-            if (row < 0) continue;
-            const float w = dw[slot];
-            const float4 v = Sout[row * H4 + o];
-            acc.x = __fadd_rn(acc.x, __fmul_rn(w, v.x));
-            acc.y = __fadd_rn(acc.y, __fmul_rn(w, v.y));
-            acc.z = __fadd_rn(acc.z, __fmul_rn(w, v.z));
-            acc.w = __fadd_rn(acc.w, __fmul_rn(w, v.w));
+        // eight slots' rows are asked for at once; one after the other each waited for its position and its row
+        for (int k0 = 0; k0 < topk; k0 += 8) {
+            long row[8];
+            float w[8];
+            float4 v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const long slot = b * topk + k0 + k;
+                row[k] = k0 + k < topk ? (pos ? (long)pos[slot] : slot) : -1;
+                w[k] = k0 + k < topk ? dw[slot] : 0.f;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = row[k] >= 0 ? Sout[row[k] * H4 + o] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                if (row[k] < 0) continue;
+                acc.x = __fadd_rn(acc.x, __fmul_rn(w[k], v[k].x));
+                acc.y = __fadd_rn(acc.y, __fmul_rn(w[k], v[k].y));
+                acc.z = __fadd_rn(acc.z, __fmul_rn(w[k], v[k].z));
+                acc.w = __fadd_rn(acc.w, __fmul_rn(w[k], v[k].w));
+            }
         }
         out[i] = acc;
     }
@@ -355,17 +379,23 @@ inline int launch_experts(const BlockArgs &a, const Buffers &b, bool use_gemm, l
     // in the prologue of down — so the block is three launches instead of five; same values in the same stage buffers.
     const bool fuse_rows = !use_gemm && a.H <= 64 * QBLK && a.H != 24 * QBLK && a.MI == 24 * QBLK && aligned(a.n2, 16) && aligned(a.dn_wq, 16) &&
                            aligned(b.xq_h, 16) && aligned(b.gu, 16) && (long)a.H * 24 < (1L << 30);
+    const bool sort_quantizes = use_gemm && aligned(a.n2, 32);      // the workspace's rows are aligned
     int rc = W4A8_OK;
-    if (!fuse_rows) rc = launch_quantize_x(a.n2, b.xq, b.xs, nullptr, a.H, a.S, st);
+    if (!fuse_rows && !sort_quantizes) rc = launch_quantize_x(a.n2, b.xq, b.xs, nullptr, a.H, a.S, st);
     if (rc != W4A8_OK) return rc;
     if (use_gemm) {
-        moe_sort_kernel<<<1, 1024, 0, st>>>(a.idx, nslots, a.expert_base, a.experts, b.perm, b.pos, b.offsets, b.items, b.num_items);
+        const long nvec = sort_quantizes ? (long)a.S * (a.H / 8) : 0, want = (nvec + 1023) / 1024;
+        const cudaError_t e = launch_pdl(moe_sort_kernel, dim3(1 + (unsigned)(want < 2L * sms - 1 ? want : 2L * sms - 1)), dim3(1024), 0, st, a.idx, nslots,
+                                         a.expert_base, a.experts, b.perm, b.pos, b.offsets, b.items, b.num_items, a.n2, reinterpret_cast<uint2 *>(b.xq), b.xs, nvec);
+        if (e != cudaSuccess) return cuda_fail(e, "moe_sort launch");
         rc = launch_status("moe_sort");
         if (rc != W4A8_OK) return rc;
     }
     if (use_gemm) {
         const unsigned gg = (unsigned)(nslots < sms * 8 ? nslots : sms * 8);
-        moe_gather_rows_kernel<<<gg, 128, 0, st>>>(b.xq, b.xs, b.perm, b.offsets + a.experts, a.topk, a.H, b.xq_g, b.xs_g);
+        const cudaError_t e = launch_pdl(moe_gather_rows_kernel, dim3(gg), dim3(128), 0, st, (const int8_t *)b.xq, (const float *)b.xs, (const int *)b.perm,
+                                         (const int *)(b.offsets + a.experts), a.topk, a.H, b.xq_g, b.xs_g);
+        if (e != cudaSuccess) return cuda_fail(e, "moe_gather_rows launch");
         rc = launch_status("moe_gather_rows");
         if (rc != W4A8_OK) return rc;
         gemm_mma::GroupList gl;
