@@ -18,6 +18,7 @@
 //   the activations, staged once per CTA and pre-split into the matching even / odd byte order, are the B fragment;
 //   D[16 x 8] int32 = 16 * group dots; the factor 1/16 is folded (exactly) into the staged activation scales.
 #pragma once
+#include <type_traits>
 #include "common.cuh"
 #include "gemv_w4a8.cuh"
 
@@ -77,10 +78,20 @@ __host__ __device__ inline size_t smem_bytes(int MH, int S, int nb, int GS, int 
 // matrix hit eight different 16-byte bank groups (row pitch GS*16 B is a multiple of 128 B for GS >= 8).
 __device__ __forceinline__ int swz(int r, int GS) { return GS >= 8 ? (r & 7) : ((r >> 1) & 3); }
 
-template <int MH, int GS, int STAGES, typename ST, bool PEER>
+// Up to four matrices that share the activations, one behind the other: matrix i has the 16-row tiles tile0[i] .. tile0[i + 1] - 1.
+constexpr int MAX_MATS = 4;
+struct Mats {
+    const uint8_t *Wq[MAX_MATS];
+    const void *sw[MAX_MATS];
+    float *Y[MAX_MATS];
+    int OUT[MAX_MATS], tile0[MAX_MATS + 1];
+};
+struct NoMats { };
+
+template <int MH, int GS, int STAGES, typename ST, bool PEER, bool MULTI = false>
 __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
     const int8_t *__restrict__ xq, const float *__restrict__ xs, const uint8_t *__restrict__ Wq,
-    const ST *__restrict__ sw, float *__restrict__ Y, int IN, int OUT, int S, OutArgs oa) {
+    const ST *__restrict__ sw, float *__restrict__ Y, int IN, int OUT, int S, OutArgs oa, const std::conditional_t<MULTI, Mats, NoMats> mats) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int STEP_W = step_w(GS), STEP_BYTES = step_bytes(GS);
     const int nb = IN / QBLK, nsteps = nb / GS;       // nb % GS == 0 is a launch precondition
@@ -91,8 +102,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     // 8-row units [u0, u1) of this CTA; a warp walks them two at a time (one 16-row MMA tile)
-    const int units = (OUT + 7) / 8;
-    const int u0 = (int)(((long)units * blockIdx.x) / gridDim.x), u1 = (int)(((long)units * (blockIdx.x + 1)) / gridDim.x);
+    const int units = (OUT + 7) / 8;                        // several matrices: OUT is 16 times the number of tiles, and tiles are whole
+    const int u0 = MULTI ? 2 * (int)(((long)(units / 2) * blockIdx.x) / gridDim.x) : (int)(((long)units * blockIdx.x) / gridDim.x);
+    const int u1 = MULTI ? 2 * (int)(((long)(units / 2) * (blockIdx.x + 1)) / gridDim.x) : (int)(((long)units * (blockIdx.x + 1)) / gridDim.x);
     const int ntiles_cta = (u1 - u0 + 1) / 2;
     int my_tiles = ntiles_cta > warp ? (ntiles_cta - warp + WARPS - 1) / WARPS : 0;
     // When the CTA has fewer tiles than warps (narrow matrices), the idle warps' ring slots are lent to the working
@@ -123,12 +135,30 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
     constexpr int RPI = 32 / GS, NW = 16 / RPI;                  // rows per copy instruction, copy instructions of a step
     constexpr int SP = sizeof(ST) == 4 ? GS / 4 : GS / 8, NS = (16 * SP + 31) / 32;   // 16-byte scale pieces per row
     const int lr = lane / GS, lj = lane % GS;
+    // the matrix of a tile of this CTA, and the tile's first row in it
+    struct Place { int mat, row0; };
+    auto place = [&](int tile) {
+        Place p = {0, 0};
+        if constexpr (MULTI) {
+            const int gt = u0 / 2 + tile;
+            while (p.mat + 1 < MAX_MATS && gt >= mats.tile0[p.mat + 1]) p.mat++;
+            p.row0 = (gt - mats.tile0[p.mat]) * 16;
+        }
+        return p;
+    };
     const uint8_t *wbase = Wq + (size_t)u0 * 8 * wpitch;        // 32-bit offsets from the CTA's first row (launch_p: its rows are under 2 GB)
     const unsigned char *sbase = reinterpret_cast<const unsigned char *>(sw + (size_t)u0 * 8 * nb);
-    const int last = OUT - 1 - u0 * 8;
+    int last = OUT - 1 - u0 * 8;
     uint32_t woff[NW], soff[NS];
     auto tile_rows = [&]() {
-        const int base = 16 * (KS > 1 ? rtile : warp + it * WARPS);
+        int base = 16 * (KS > 1 ? rtile : warp + it * WARPS);
+        if constexpr (MULTI) {
+            const Place p = place(base / 16);
+            wbase = mats.Wq[p.mat] + (size_t)p.row0 * wpitch;
+            sbase = static_cast<const unsigned char *>(mats.sw[p.mat]) + (size_t)p.row0 * nb * sizeof(ST);
+            last = mats.OUT[p.mat] - 1 - p.row0;
+            base = 0;
+        }
 #pragma unroll
         for (int i = 0; i < NW; i++) woff[i] = (uint32_t)min(base + i * RPI + lr, last) * (uint32_t)(IN / 2) + (uint32_t)(iq * GS + lj) * 16;
 #pragma unroll
@@ -327,19 +357,23 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
                     __syncwarp();
                     if (lane == 0) *flag = (unsigned)(q + 1);
                 } else {                                       // last step: these are the outputs
-                    const int base = (u0 + 2 * rtile) * 8;
-                    const int lim = min(OUT, u1 * 8);
+                    int base = (u0 + 2 * rtile) * 8, lim = min(OUT, u1 * 8), ld = OUT;
+                    float *Yt = Y;
+                    if constexpr (MULTI) {
+                        const Place p = place(rtile);
+                        base = p.row0; lim = ld = mats.OUT[p.mat]; Yt = mats.Y[p.mat];
+                    }
                     const int rA = base + g, rB = base + 8 + g;
 #pragma unroll
                     for (int h = 0; h < MH; h++) {
                         const int m0 = 8 * h + 2 * t;
                         if (rA < lim) {
-                            if (m0 < S) store_out<PEER>(Y, oa, OUT, m0, rA, a[h][0]);
-                            if (m0 + 1 < S) store_out<PEER>(Y, oa, OUT, m0 + 1, rA, a[h][1]);
+                            if (m0 < S) store_out<PEER>(Yt, oa, ld, m0, rA, a[h][0]);
+                            if (m0 + 1 < S) store_out<PEER>(Yt, oa, ld, m0 + 1, rA, a[h][1]);
                         }
                         if (rB < lim) {
-                            if (m0 < S) store_out<PEER>(Y, oa, OUT, m0, rB, a[h][2]);
-                            if (m0 + 1 < S) store_out<PEER>(Y, oa, OUT, m0 + 1, rB, a[h][3]);
+                            if (m0 < S) store_out<PEER>(Yt, oa, ld, m0, rB, a[h][2]);
+                            if (m0 + 1 < S) store_out<PEER>(Yt, oa, ld, m0 + 1, rB, a[h][3]);
                         }
                     }
                 }
@@ -404,18 +438,22 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
             __syncwarp();                                  // the slot is refilled by the next iteration's copies
             if (++csl == depth) csl = 0;
         }
-        const int base = (u0 + 2 * (warp + ti * WARPS)) * 8;
-        const int lim = min(OUT, u1 * 8);
+        int base = (u0 + 2 * (warp + ti * WARPS)) * 8, lim = min(OUT, u1 * 8), ld = OUT;
+        float *Yt = Y;
+        if constexpr (MULTI) {
+            const Place p = place(warp + ti * WARPS);
+            base = p.row0; lim = ld = mats.OUT[p.mat]; Yt = mats.Y[p.mat];
+        }
 #pragma unroll
         for (int h = 0; h < MH; h++) {
             const int m0 = 8 * h + 2 * t, rA = base + g, rB = base + 8 + g;
             if (rA < lim) {
-                if (m0 < S) store_out<PEER>(Y, oa, OUT, m0, rA, acc[h][0]);
-                if (m0 + 1 < S) store_out<PEER>(Y, oa, OUT, m0 + 1, rA, acc[h][1]);
+                if (m0 < S) store_out<PEER>(Yt, oa, ld, m0, rA, acc[h][0]);
+                if (m0 + 1 < S) store_out<PEER>(Yt, oa, ld, m0 + 1, rA, acc[h][1]);
             }
             if (rB < lim) {
-                if (m0 < S) store_out<PEER>(Y, oa, OUT, m0, rB, acc[h][2]);
-                if (m0 + 1 < S) store_out<PEER>(Y, oa, OUT, m0 + 1, rB, acc[h][3]);
+                if (m0 < S) store_out<PEER>(Yt, oa, ld, m0, rB, acc[h][2]);
+                if (m0 + 1 < S) store_out<PEER>(Yt, oa, ld, m0 + 1, rB, acc[h][3]);
             }
         }
     }
@@ -453,12 +491,12 @@ inline bool plan_for(const void *Wq, const void *sw, int IN, int OUT, int S, Pla
     return false;
 }
 
-template <int MH, int GS, int STAGES, typename ST, bool PEER>
+template <int MH, int GS, int STAGES, typename ST, bool PEER, bool MULTI = false>
 inline int launch_p(const int8_t *xq, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int IN, int OUT, int S,
-                    cudaStream_t st, const OutArgs &oa) {
+                    cudaStream_t st, const OutArgs &oa, const std::conditional_t<MULTI, Mats, NoMats> &mats = {}) {
     const int nb = IN / QBLK;
     const size_t smem = smem_bytes(MH, S, nb, GS, STAGES);
-    auto kern = gemv_w4a8_mma_kernel<MH, GS, STAGES, ST, PEER>;
+    auto kern = gemv_w4a8_mma_kernel<MH, GS, STAGES, ST, PEER, MULTI>;
     static PerDevice<size_t> configured_dev;            // grow-only; the opt-in is a per-device function attribute
     size_t &configured = configured_dev.get();
     if (smem > configured) {
@@ -471,7 +509,7 @@ inline int launch_p(const int8_t *xq, const float *xs, const uint8_t *Wq, const 
     long cap = sm_count();                               // one persistent CTA per SM
     while ((units / cap + 2) * 8l * (IN / 2) >= (1l << 31)) cap *= 2;   // the copies' offsets are 32-bit
     const dim3 grid((unsigned)(want < cap ? want : cap));
-    cudaError_t le = launch_pdl(kern, grid, dim3(WARPS * 32), smem, st, xq, xs, Wq, sw, Y, IN, OUT, S, oa);
+    cudaError_t le = launch_pdl(kern, grid, dim3(WARPS * 32), smem, st, xq, xs, Wq, sw, Y, IN, OUT, S, oa, mats);
     if (le != cudaSuccess) return cuda_fail(le, "gemv_w4a8_mma launch");
     return launch_status("gemv_w4a8_mma");
 }
@@ -499,6 +537,25 @@ inline int launch(const int8_t *xq, const float *xs, const uint8_t *Wq, const vo
     if (scale_dtype == 1) return launch_st<__half>(xq, xs, Wq, (const __half *)sw, Y, IN, OUT, S, p, st, oa);
     return launch_st<float>(xq, xs, Wq, (const float *)sw, Y, IN, OUT, S, p, st, oa);
 }
+
+// Several matrices in one launch, the SMs divided over all their tiles; the bits of one launch each.  What it saves is a launch's
+// release and the staging of the rows.
+inline int launch_multi(const int8_t *xq, const float *xs, const Mats &m, int IN, int S, int scale_dtype, const Plan &p, cudaStream_t st) {
+    const int OUT = 16 * m.tile0[MAX_MATS];
+    const auto run = [&](auto mh, auto gs, auto stages, auto *w) {
+        using ST = std::remove_const_t<std::remove_pointer_t<decltype(w)>>;
+        return launch_p<decltype(mh)::value, decltype(gs)::value, decltype(stages)::value, ST, false, true>(xq, xs, m.Wq[0], w, m.Y[0], IN, OUT, S, st, OutArgs(), m);
+    };
+    const auto typed = [&](auto mh, auto gs, auto stages) {
+        return scale_dtype == 1 ? run(mh, gs, stages, (const __half *)m.sw[0]) : run(mh, gs, stages, (const float *)m.sw[0]);
+    };
+    using std::integral_constant;
+    if (p.MH == 1 && p.GS == 16) return typed(integral_constant<int, 1>(), integral_constant<int, 16>(), integral_constant<int, 2>());
+    if (p.MH == 1) return typed(integral_constant<int, 1>(), integral_constant<int, 8>(), integral_constant<int, 3>());
+    if (p.GS == 16) return typed(integral_constant<int, 2>(), integral_constant<int, 16>(), integral_constant<int, 2>());
+    return typed(integral_constant<int, 2>(), integral_constant<int, 8>(), integral_constant<int, 3>());
+}
+inline bool multi_serves(const Plan &p) { return p.STAGES == (p.GS == 16 ? 2 : 3); }
 
 }  // namespace gemv_mma
 }  // namespace w4a8

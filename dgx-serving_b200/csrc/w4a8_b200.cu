@@ -300,7 +300,8 @@ W4A8_API int w4a8_gemv_multi(const int8_t *xq, const float *xs, int count, const
     if (count == 0 || S == 0) return W4A8_OK;
     if (!Wq || !sw || !Y || !OUT) return fail(W4A8_ERR_ARG, "gemv_multi: null array argument");
     // One launch when every matrix can take the bulk-copy stream (one row, the auto policy's conditions); else the
-    // matrices go one after the other through w4a8_gemv.  Either way each output equals w4a8_gemv's, bit for bit.
+    // matrices go one after the other through w4a8_gemv, or two to sixteen rows in one launch of the tensor-path kernel.  Either way each
+    // output equals w4a8_gemv's, bit for bit.
     bool one = S == 1 && (gemv_policy() == 3 || (gemv_policy() == 0 && IN >= 2048));
     gemv_bulk::Plan bp;
     gemv_bulk::Mats m = {};
@@ -317,6 +318,22 @@ W4A8_API int w4a8_gemv_multi(const int8_t *xq, const float *xs, int count, const
         if (rc != W4A8_OK) return rc;
         m.count = count;
         return gemv_bulk::launch_multi(xq, xs, m, IN, scale_dtype, bp, (cudaStream_t)stream);
+    }
+    // Two to sixteen rows: one launch of the tensor-path kernel where each matrix alone would take it in one pass.
+    one = count > 1 && S >= 2 && S <= 16 && IN > 0 && IN % QBLK == 0 && (scale_dtype == 0 || scale_dtype == 1) && xq && xs && aligned(xq, 4) && gemv_use_mma(S, scale_dtype);
+    gemv_mma::Plan mp;
+    gemv_mma::Mats mm = {};
+    long tiles = 0;
+    for (int i = 0; i < count && one; i++) {
+        if (OUT[i] <= 0 || !Wq[i] || !sw[i] || !Y[i] || !gemv_mma::plan_for(Wq[i], sw[i], IN, OUT[i], S, &mp)) { one = false; break; }
+        mm.Wq[i] = Wq[i]; mm.sw[i] = sw[i]; mm.Y[i] = Y[i]; mm.OUT[i] = OUT[i]; mm.tile0[i] = (int)tiles;
+        tiles += ((long)OUT[i] + 15) / 16;
+    }
+    if (one && tiles < (1L << 27) && gemv_mma::plan_for(Wq[0], sw[0], IN, (int)(tiles * 16), S, &mp) && gemv_mma::multi_serves(mp)) {
+        int rc = require_sm100();
+        if (rc != W4A8_OK) return rc;
+        for (int i = count; i <= gemv_mma::MAX_MATS; i++) mm.tile0[i] = (int)tiles;
+        return gemv_mma::launch_multi(xq, xs, mm, IN, S, scale_dtype, mp, (cudaStream_t)stream);
     }
     for (int i = 0; i < count; i++) {
         int rc = w4a8_gemv(xq, xs, Wq[i], sw[i], Y[i], IN, OUT[i], S, scale_dtype, stream);
