@@ -501,13 +501,37 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_w4a8_tc_kernel(
 
 // Adds the split-K partial sums in ascending split order (the order of the reference's
 // reduce_splitk_kernel, kernels/gemm_mmq.cuh:201-204): Y[i] = ((0 + P0[i]) + P1[i]) + ...
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restrict__ P, float *__restrict__ Y, long MN, int nsplit) {
+// VEC: float or float4 (MN a multiple of four, both pointers aligned).  Launched dependent: it waits at once, but its launch latency
+// hides behind the end of the product.
+template <typename VEC>
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const VEC *__restrict__ P, VEC *__restrict__ Y, long n, int nsplit) {
     const long stride = (long)gridDim.x * blockDim.x;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < MN; i += stride) {
-        float s = 0.f;
-        for (int sp = 0; sp < nsplit; sp++) s += P[(size_t)sp * MN + i];
-        Y[i] = s;
+    pdl_wait();
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        if constexpr (sizeof(VEC) == 16) {
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+            for (int sp = 0; sp < nsplit; sp++) {
+                const float4 v = P[(size_t)sp * n + i];
+                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+            }
+            Y[i] = s;
+        } else {
+            float s = 0.f;
+#pragma unroll 4
+            for (int sp = 0; sp < nsplit; sp++) s += P[(size_t)sp * n + i];
+            Y[i] = s;
+        }
     }
+}
+inline int launch_splitk_reduce(const float *P, float *Y, long MN, int nsplit, cudaStream_t st) {
+    const bool vec = MN % 4 == 0 && aligned(P, 16) && aligned(Y, 16);
+    const long n = vec ? MN / 4 : MN, want = (n + 255) / 256, cap = (long)sm_count() * 8;
+    const dim3 grid((unsigned)(want < cap ? want : cap));
+    const cudaError_t e = vec ? launch_pdl(splitk_reduce_kernel<float4>, grid, dim3(256), 0, st, reinterpret_cast<const float4 *>(P), reinterpret_cast<float4 *>(Y), n, nsplit)
+                              : launch_pdl(splitk_reduce_kernel<float>, grid, dim3(256), 0, st, P, Y, n, nsplit);
+    if (e != cudaSuccess) return cuda_fail(e, "splitk_reduce launch");
+    return launch_status("splitk_reduce");
 }
 
 // ---- host side ------------------------------------------------------------------------------------

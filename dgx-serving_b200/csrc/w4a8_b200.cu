@@ -404,10 +404,7 @@ W4A8_API int w4a8_gemm_splitk(const int8_t *X, const float *xs, const uint8_t *W
     if (!aligned(workspace, 16)) return fail(W4A8_ERR_ALIGN, "gemm_splitk: workspace must be 16-byte aligned");
     rc = gemm_launch(X, xs, Wq, sw, (float *)workspace, M, N, K, scale_dtype, ns, gs, st);
     if (rc != W4A8_OK) return rc;
-    const long MN = (long)M * N;
-    long want = (MN + 255) / 256, cap = (long)sm_count() * 8;
-    gemm::splitk_reduce_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>((const float *)workspace, Y, MN, ns);
-    return launch_status("splitk_reduce");
+    return gemm::launch_splitk_reduce((const float *)workspace, Y, (long)M * N, ns, st);
 }
 
 // ---- split-K without an allocator ---------------------------------------------------------------------
@@ -469,10 +466,7 @@ W4A8_API int w4a8_gemm_splitk_static(const int8_t *X, const float *xs, const uin
     // exactly those: nothing left over from an earlier call is ever read, so nothing needs clearing.
     rc = gemm_launch(X, xs, Wq, sw, scratch, M, N, K, scale_dtype, ns, gs, st);
     if (rc != W4A8_OK) return rc;
-    const long MN = (long)M * N;
-    long want = (MN + 255) / 256, cap = (long)sm_count() * 8;
-    gemm::splitk_reduce_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>(scratch, Y, MN, ns);
-    return launch_status("splitk_reduce (static)");
+    return gemm::launch_splitk_reduce(scratch, Y, (long)M * N, ns, st);
 }
 
 W4A8_API int w4a8_group_dots(const int8_t *xq, const uint8_t *Wq, int32_t *D, int M, int N, int K, int path, void *stream) {
