@@ -52,11 +52,13 @@ __global__ void __launch_bounds__(256) quantize_x_q8_vec_kernel(const float4 *__
     }
 }
 
-// The same with eight elements a thread, for X aligned to 32 bytes: a third fewer instructions an element, because four lanes share a
-// block's maximum, scale and sum and not eight, maxima take three operands, multiply and fma two elements, and a 256-bit load is a
-// whole sector per lane.  What bounds it is then HBM: 8192 x 5120 44.5 -> 34.9 us in a chain, 5.25 bytes an element = 6.3 TB/s of the measured
-// 6.56; 2048 x 5120 14.2 -> 9.3, 512 x 2048 3.6 -> 3.4, one row of 5120 2.7 -> 2.0 (333 x 3840 3.6 -> 3.8).  One vector a thread: two,
-// three and four in flight 35.3 to 40.2, and fewer threads hide less in the small cases (16 x 5120 2.9, 3.2, 3.7).
+// The same with eight elements a thread, for X aligned to 32 bytes: 56 instead of 96 warp instructions per 128 elements, because four
+// lanes share a block's maximum, scale and sum and not eight, maxima take three operands, multiply and fma two elements, and a 256-bit
+// load is a whole sector per lane.  What bounds it now is HBM and its latency: 8192 x 5120 44.4 -> 36.3 us in a chain, 5.25 bytes an
+// element = 6.1 TB/s of the measured 6.56; 4000 x 3840 18.8 -> 14.2, 2048 x 5120 14.2 -> 9.7, one row of 5120 2.7 -> 2.2.  One vector a
+// thread: two, three and four in flight 1 to 5 us more at 8192 rows, and fewer threads hide less in the small cases (16 x 5120 2.9,
+// 3.2, 3.7).
+constexpr int WIDE_CTAS = 6;                     // of 256 threads on an SM with 42 registers; a grid of eight per SM is 1.3 waves: 44.0 us
 __device__ __forceinline__ void load8(const float *p, float (&v)[8]) {
     asm volatile("ld.global.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
@@ -132,7 +134,7 @@ __device__ __forceinline__ void quantize_wide(const float *__restrict__ X, uint2
         quantize_store_vec8(v, i, i < nvec, xq, xs, xsum);
     }
 }
-__global__ void __launch_bounds__(256) quantize_x_q8_wide_kernel(const float *__restrict__ X, uint2 *__restrict__ xq, float *__restrict__ xs,
+__global__ void __launch_bounds__(256, WIDE_CTAS) quantize_x_q8_wide_kernel(const float *__restrict__ X, uint2 *__restrict__ xq, float *__restrict__ xs,
                                                                  int32_t *__restrict__ xsum, long nvec /* = S*IN/8 */) {
     pdl_wait();                  // and what stands at the same place of the kernel above
     pdl_launch_dependents();
@@ -171,7 +173,7 @@ inline int launch_quantize_x(const float *X, int8_t *xq, float *xs, int32_t *xsu
     const long nblk = (long)S * (IN / QBLK);
     const int sms = sm_count();
     if (aligned(X, 32) && aligned(xq, 8)) {
-        const long nvec = nblk * 4, want = (nvec + 255) / 256, cap = (long)sms * 8;
+        const long nvec = nblk * 4, want = (nvec + 255) / 256, cap = (long)sms * WIDE_CTAS;
         cudaError_t e = launch_pdl(quantize_x_q8_wide_kernel, dim3((unsigned)(want < cap ? want : cap)), dim3(256), 0, st, X, reinterpret_cast<uint2 *>(xq), xs, xsum, nvec);
         if (e != cudaSuccess) return cuda_fail(e, "quantize_x_q8 launch");
     } else if (aligned(X, 16) && aligned(xq, 4)) {
