@@ -162,7 +162,7 @@ def launch_glu_quantize_x_q8(G, U, act, Y, xq, xs, xsum, IN, S, stream=None):
 
 def gemv_multi(xq, xs, Wqs, sws, Ys, OUTs, IN, S, scale_dtype=0, stream=None):
     """Several matrices (at most 4) against the same activation rows in one call; one launch for a single row on the
-    bulk-copy kernel.  Each Ys[i] equals launch_gemv_w4a8 of matrix i."""
+    bulk-copy kernel and for 2 to 16 rows on the tensor-path kernel.  Each Ys[i] equals launch_gemv_w4a8 of matrix i."""
     n = len(Wqs)
     arr = lambda xs_: (ctypes.c_void_p * n)(*[_ptr(t) for t in xs_])
     outs = (ctypes.c_int * n)(*[int(o) for o in OUTs])
