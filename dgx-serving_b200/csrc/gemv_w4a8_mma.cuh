@@ -20,23 +20,11 @@
 #pragma once
 #include <type_traits>
 #include "common.cuh"
+#include "gemv_mma_plan.cuh"
 #include "gemv_w4a8.cuh"
 
 namespace w4a8 {
 namespace gemv_mma {
-
-#ifndef W4A8_MMA_WARPS
-#define W4A8_MMA_WARPS 8
-#endif
-constexpr int WARPS = W4A8_MMA_WARPS;
-#ifndef W4A8_GEMV_RELAY
-#define W4A8_GEMV_RELAY 1
-#endif
-constexpr bool RELAY = W4A8_GEMV_RELAY != 0;
-constexpr int RELAY16_TILES = 2;                 // 9 to 16 rows: most 16-row tiles of a CTA that are relayed
-// A step = 16 weight rows x GS groups (GS * 16 B contiguous per row) plus the 16 x GS scales (slot sized for fp32).
-__host__ __device__ constexpr int step_w(int GS) { return 16 * GS * 16; }
-__host__ __device__ constexpr int step_bytes(int GS) { return 16 * GS * 16 + 16 * GS * 4; }
 
 __device__ __forceinline__ void cp_async16_cg(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -62,18 +50,6 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, ui
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
 
-// Shared-memory plan (bytes), all offsets multiples of 16:
-//   xq'  : S rows x pitch2 uint2      (pitch2 = 4*nb + 4: rows 4 uint2 apart modulo 16 -> conflict-free LDS.64)
-//   xs'  : nb x (8*MH) floats          ([group][m], already multiplied by 1/16)
-//   ring : WARPS x STAGES x step_bytes(GS)
-__host__ __device__ inline int pitch2_of(int nb) { return 4 * nb + 4; }
-// Only the S rows that exist are staged (rows S..8*MH-1 of the MMA's B operand are zeros made in registers), so a
-// single-row decode call keeps its footprint small enough for the next kernel's CTA to become resident beside it.
-__host__ __device__ inline size_t xq_bytes(int S, int nb) { return (size_t)S * pitch2_of(nb) * 8; }
-__host__ __device__ inline size_t act_bytes(int MH, int S, int nb) { return xq_bytes(S, nb) + (size_t)nb * 8 * MH * 4; }
-__host__ __device__ inline size_t smem_bytes(int MH, int S, int nb, int GS, int STAGES) {
-    return act_bytes(MH, S, nb) + (size_t)WARPS * STAGES * step_bytes(GS);
-}
 // 16-byte piece j of row r of a slot sits at piece position j ^ swz(r): with it the eight rows of an ldmatrix
 // matrix hit eight different 16-byte bank groups (row pitch GS*16 B is a multiple of 128 B for GS >= 8).
 __device__ __forceinline__ int swz(int r, int GS) { return GS >= 8 ? (r & 7) : ((r >> 1) & 3); }
@@ -88,7 +64,9 @@ struct Mats {
 };
 struct NoMats { };
 
-template <int MH, int GS, int STAGES, typename ST, bool PEER, bool MULTI = false>
+// RLY: tiles may be relayed.  With more than eight rows it is an argument of its own: the relay's products take 60 registers and its
+// mailboxes 5 KB, which launches without it have no use for.
+template <int MH, int GS, int STAGES, typename ST, bool PEER, bool MULTI, bool RLY>
 __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
     const int8_t *__restrict__ xq, const float *__restrict__ xs, const uint8_t *__restrict__ Wq,
     const ST *__restrict__ sw, float *__restrict__ Y, int IN, int OUT, int S, OutArgs oa, const std::conditional_t<MULTI, Mats, NoMats> mats) {
@@ -110,14 +88,14 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
     // When the CTA has fewer tiles than warps (narrow matrices), the idle warps' ring slots are lent to the working
     // ones: a warp that is alone with a long row range needs more bytes in flight to stream at full speed.
     int mult = 1;
-    // Narrow matrices: K relay (for more than eight rows where a step is eight groups, whose products fit the registers).  A CTA
+    // Narrow matrices: K relay (for more than eight rows only in steps of eight groups, whose products fit the registers).  A CTA
     // with at most WARPS/2 tiles gives each tile KS warps; warp (tile, ks) streams steps ks, ks + KS, ... of the tile and computes
     // their products t = (float)D * xs, and the fp32 accumulators travel from the warp of step q to the warp of step q + 1 through a
     // mailbox in shared memory, so that every accumulator still sees its groups in ascending order (the bits do not change) while KS
     // rings of copies are in flight per tile instead of one.
-    constexpr bool CAN_RELAY = RELAY && (MH == 1 || GS == 8);
+    static_assert(!RLY || MH == 1 || GS == 8);
     int KS = 1;
-    if (CAN_RELAY && (MH == 1 || ntiles_cta <= RELAY16_TILES)) while (KS < WARPS && ntiles_cta * KS * 2 <= WARPS) KS *= 2;
+    if (RLY) while (KS < WARPS && ntiles_cta * KS * 2 <= WARPS) KS *= 2;
     if (KS == 1) while (mult < 4 && ntiles_cta * mult * 2 <= WARPS) mult *= 2;
     const int rtile = warp / KS, rks = warp % KS;            // relay: tile of this warp inside the CTA, first step
     const int depth = STAGES * mult;
@@ -249,9 +227,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
             }
         }
     }
-    __shared__ float4 relay_box[WARPS / 2][MH][32];
-    __shared__ unsigned int relay_flag[WARPS / 2];
-    if (tid < WARPS / 2) relay_flag[tid] = 0u;
+    __shared__ float4 relay_box[RLY ? WARPS / 2 : 1][MH][32];
+    __shared__ unsigned int relay_flag[RLY ? WARPS / 2 : 1];
+    static_assert(!RLY || sizeof(relay_box) + sizeof(relay_flag) + 64 <= static_bytes(MH, true));
+    if (RLY && tid < WARPS / 2) relay_flag[tid] = 0u;
     for (int i0 = tid; i0 < nb * 8 * MH; i0 += NT * 4) {
         float v[4];
 #pragma unroll
@@ -274,7 +253,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
 #pragma unroll
     for (int h = 0; h < MH; h++) xrow[h] = xqp + (size_t)min(8 * h + g, S - 1) * pitch2 + t;
     int csl = 0;
-    if (CAN_RELAY && KS > 1) {
+    if (RLY && KS > 1) {
         if (my_tiles > 0) {
             volatile unsigned int *flag = &relay_flag[rtile];
             bool alive = true;
@@ -421,7 +400,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
                         unpack8_x16(w[2 * k + 1], a1, a3);    // rows g+8
 #pragma unroll
                         for (int h = 0; h < MH; h++) {
-                            // activation row m = 8h + g of this lane; rows beyond S contribute zeros and are not staged
+                            // activation row m = 8h + g of this lane; for m >= S the last row again, whose columns are never stored
                             const uint2 bx = xrow[h][4 * b];
                             int c[4];
                             mma_s8(c, a0, a1, a2, a3, bx.x, bx.y);
@@ -461,42 +440,22 @@ __global__ void __launch_bounds__(WARPS * 32, 1) gemv_w4a8_mma_kernel(
     publish_out<PEER>(oa, 2 * t < S || MH == 2);          // lanes whose columns m = 8h + 2t (+1) exist
 }
 
-// Launch plan: groups per step (the largest of 16, 8 that divides the group count), ring depth and rows per pass
-// such that the shared-memory plan fits.  Preconditions: K % 256 == 0 (whole steps; 16-byte aligned scale pieces for
-// fp32 and fp16), Wq and sw 16-byte aligned, xq 4-byte aligned.
-struct Plan { int MH, GS, STAGES; };
-constexpr size_t SMEM_LIMIT = 224 * 1024;
+// Launch plan.  Preconditions: K % 256 == 0 (whole steps; 16-byte aligned scale pieces for fp32 and fp16), Wq and sw 16-byte aligned,
+// xq 4-byte aligned.
 inline int env_int(const char *name, int dflt) { const char *e = getenv(name); return e ? atoi(e) : dflt; }
 inline bool plan_for(const void *Wq, const void *sw, int IN, int OUT, int S, Plan *p) {
-    const int nb = IN / QBLK;
-    if (IN <= 0 || nb % 8 != 0) return false;
     if (!aligned(Wq, 16) || !aligned(sw, 16)) return false;
     static const int want_gs = env_int("W4A8_GEMV_GS", 16);
     static const int want_st = env_int("W4A8_GEMV_STAGES", 0);
-    const int MH = S > 8 ? 2 : 1;
-    // 9 to 16 rows of a matrix with at most two tiles per CTA: steps of eight groups, which the relay takes.  us, one warp a tile /
-    // relay: 16 x 2048 x 8192 16.7 / 11.3, 16 x 4096 x 3840 8.9 / 7.3 (fp16 9.5 / 7.3), 10 x 2500 x 2304 fp16 6.5 / 5.2, 9 x 2048 x 2048
-    // 4.7 / 4.2.  With three or four tiles two warps each gain nothing (12 x 5120 x 5120 10.6 / 11.0, 16 x 9472 x 4096 9.4 / 10.1),
-    // nor do rows of a few steps (12 x 4000 x 512 2.8 / 3.2).
-    const bool relay16 = RELAY && MH == 2 && nb >= 48 && ((long)OUT + 7) / 8 <= (long)sm_count() * 2 * RELAY16_TILES;
-    const int gs_opts[2] = {16, 8};
-    for (int gi = 0; gi < 2; gi++) {
-        const int GS = gs_opts[gi];
-        if (GS > want_gs || nb % GS != 0 || (GS == 16 && relay16)) continue;
-        const int st_opts[3] = {GS == 16 ? 4 : 8, GS == 16 ? 3 : 6, GS == 16 ? 2 : 3};
-        for (int si = 0; si < 3; si++)
-            if (st_opts[si] <= (want_st > 0 ? want_st : (GS == 16 ? 2 : 3)))
-            if (smem_bytes(MH, S, nb, GS, st_opts[si]) <= SMEM_LIMIT) { p->MH = MH; p->GS = GS; p->STAGES = st_opts[si]; return true; }
-    }
-    return false;
+    return plan_rows(IN / QBLK, OUT, S, sm_count(), want_gs, want_st, p);
 }
 
-template <int MH, int GS, int STAGES, typename ST, bool PEER, bool MULTI = false>
+template <int MH, int GS, int STAGES, typename ST, bool PEER, bool RLY, bool MULTI = false>
 inline int launch_p(const int8_t *xq, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int IN, int OUT, int S,
                     cudaStream_t st, const OutArgs &oa, const std::conditional_t<MULTI, Mats, NoMats> &mats = {}) {
     const int nb = IN / QBLK;
-    const size_t smem = smem_bytes(MH, S, nb, GS, STAGES);
-    auto kern = gemv_w4a8_mma_kernel<MH, GS, STAGES, ST, PEER, MULTI>;
+    const size_t smem = launch_smem(MH, S, nb, GS, STAGES);
+    auto kern = gemv_w4a8_mma_kernel<MH, GS, STAGES, ST, PEER, MULTI, RLY>;
     static PerDevice<size_t> configured_dev;            // grow-only; the opt-in is a per-device function attribute
     size_t &configured = configured_dev.get();
     if (smem > configured) {
@@ -514,20 +473,22 @@ inline int launch_p(const int8_t *xq, const float *xs, const uint8_t *Wq, const 
     return launch_status("gemv_w4a8_mma");
 }
 
-template <int MH, int GS, int STAGES, typename ST>
+template <int MH, int GS, int STAGES, typename ST, bool RLY>
 inline int launch_t(const int8_t *xq, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int IN, int OUT, int S,
                     cudaStream_t st, const OutArgs &oa) {
-    if (oa.peers) return launch_p<MH, GS, STAGES, ST, true>(xq, xs, Wq, sw, Y, IN, OUT, S, st, oa);
-    return launch_p<MH, GS, STAGES, ST, false>(xq, xs, Wq, sw, Y, IN, OUT, S, st, oa);
+    if (oa.peers) return launch_p<MH, GS, STAGES, ST, true, RLY>(xq, xs, Wq, sw, Y, IN, OUT, S, st, oa);
+    return launch_p<MH, GS, STAGES, ST, false, RLY>(xq, xs, Wq, sw, Y, IN, OUT, S, st, oa);
 }
 
 template <typename ST>
 inline int launch_st(const int8_t *xq, const float *xs, const uint8_t *Wq, const ST *sw, float *Y, int IN, int OUT, int S,
                      const Plan &p, cudaStream_t st, const OutArgs &oa) {
-#define W4A8_MMA_CASE(MH_, GS_, ST_) \
-    if (p.MH == MH_ && p.GS == GS_ && p.STAGES == ST_) return launch_t<MH_, GS_, ST_, ST>(xq, xs, Wq, sw, Y, IN, OUT, S, st, oa);
-    W4A8_MMA_CASE(1, 16, 4) W4A8_MMA_CASE(1, 16, 3) W4A8_MMA_CASE(1, 16, 2) W4A8_MMA_CASE(1, 8, 8) W4A8_MMA_CASE(1, 8, 6) W4A8_MMA_CASE(1, 8, 3)
-    W4A8_MMA_CASE(2, 16, 4) W4A8_MMA_CASE(2, 16, 3) W4A8_MMA_CASE(2, 16, 2) W4A8_MMA_CASE(2, 8, 8) W4A8_MMA_CASE(2, 8, 6) W4A8_MMA_CASE(2, 8, 3)
+#define W4A8_MMA_CASE(MH_, GS_, ST_, R_) \
+    if (p.MH == MH_ && p.GS == GS_ && p.STAGES == ST_ && (MH_ == 1 || p.relay == R_)) return launch_t<MH_, GS_, ST_, ST, R_>(xq, xs, Wq, sw, Y, IN, OUT, S, st, oa);
+    W4A8_MMA_CASE(1, 16, 4, RELAY) W4A8_MMA_CASE(1, 16, 3, RELAY) W4A8_MMA_CASE(1, 16, 2, RELAY)
+    W4A8_MMA_CASE(1, 8, 8, RELAY) W4A8_MMA_CASE(1, 8, 6, RELAY) W4A8_MMA_CASE(1, 8, 3, RELAY)
+    W4A8_MMA_CASE(2, 16, 4, false) W4A8_MMA_CASE(2, 16, 3, false) W4A8_MMA_CASE(2, 16, 2, false)
+    W4A8_MMA_CASE(2, 8, 8, false) W4A8_MMA_CASE(2, 8, 6, false) W4A8_MMA_CASE(2, 8, 3, false) W4A8_MMA_CASE(2, 8, 3, true)
 #undef W4A8_MMA_CASE
     return fail(W4A8_ERR_UNSUPPORTED, "gemv_mma: no kernel for plan MH=%d GS=%d STAGES=%d", p.MH, p.GS, p.STAGES);
 }
@@ -542,18 +503,21 @@ inline int launch(const int8_t *xq, const float *xs, const uint8_t *Wq, const vo
 // release and the staging of the rows.
 inline int launch_multi(const int8_t *xq, const float *xs, const Mats &m, int IN, int S, int scale_dtype, const Plan &p, cudaStream_t st) {
     const int OUT = 16 * m.tile0[MAX_MATS];
-    const auto run = [&](auto mh, auto gs, auto stages, auto *w) {
+    const auto run = [&](auto mh, auto gs, auto stages, auto rly, auto *w) {
         using ST = std::remove_const_t<std::remove_pointer_t<decltype(w)>>;
-        return launch_p<decltype(mh)::value, decltype(gs)::value, decltype(stages)::value, ST, false, true>(xq, xs, m.Wq[0], w, m.Y[0], IN, OUT, S, st, OutArgs(), m);
+        return launch_p<decltype(mh)::value, decltype(gs)::value, decltype(stages)::value, ST, false, decltype(rly)::value, true>(xq, xs, m.Wq[0], w, m.Y[0], IN, OUT, S, st, OutArgs(), m);
     };
-    const auto typed = [&](auto mh, auto gs, auto stages) {
-        return scale_dtype == 1 ? run(mh, gs, stages, (const __half *)m.sw[0]) : run(mh, gs, stages, (const float *)m.sw[0]);
+    const auto typed = [&](auto mh, auto gs, auto stages, auto rly) {
+        return scale_dtype == 1 ? run(mh, gs, stages, rly, (const __half *)m.sw[0]) : run(mh, gs, stages, rly, (const float *)m.sw[0]);
     };
     using std::integral_constant;
-    if (p.MH == 1 && p.GS == 16) return typed(integral_constant<int, 1>(), integral_constant<int, 16>(), integral_constant<int, 2>());
-    if (p.MH == 1) return typed(integral_constant<int, 1>(), integral_constant<int, 8>(), integral_constant<int, 3>());
-    if (p.GS == 16) return typed(integral_constant<int, 2>(), integral_constant<int, 16>(), integral_constant<int, 2>());
-    return typed(integral_constant<int, 2>(), integral_constant<int, 8>(), integral_constant<int, 3>());
+    using Rly = integral_constant<bool, RELAY>;
+    using NoRly = integral_constant<bool, false>;
+    if (p.MH == 1 && p.GS == 16) return typed(integral_constant<int, 1>(), integral_constant<int, 16>(), integral_constant<int, 2>(), Rly());
+    if (p.MH == 1) return typed(integral_constant<int, 1>(), integral_constant<int, 8>(), integral_constant<int, 3>(), Rly());
+    if (p.GS == 16) return typed(integral_constant<int, 2>(), integral_constant<int, 16>(), integral_constant<int, 2>(), NoRly());
+    if (p.relay) return typed(integral_constant<int, 2>(), integral_constant<int, 8>(), integral_constant<int, 3>(), Rly());
+    return typed(integral_constant<int, 2>(), integral_constant<int, 8>(), integral_constant<int, 3>(), NoRly());
 }
 inline bool multi_serves(const Plan &p) { return p.STAGES == (p.GS == 16 ? 2 : 3); }
 
