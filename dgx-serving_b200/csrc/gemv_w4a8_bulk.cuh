@@ -178,6 +178,12 @@ __global__ void __launch_bounds__(THREADS) gemv_w4a8_bulk_kernel(
 #pragma unroll
             for (int i = 0; i < 4; i++) split_even_odd(v[2 * i], v[2 * i + 1], xe[j][i], xo[j][i]);
         }
+        // six groups a lane fit the registers with the longer form only: with the other one ptxas spills 104 bytes.
+        constexpr bool EXPR = NG == 6 && !PEER && !FUSE;
+        const auto unpack = [](uint32_t w, uint32_t &e, uint32_t &o) {
+            if constexpr (EXPR) unpack8_x16_expr(w, e, o);
+            else unpack8_x16(w, e, o);
+        };
         const int grp = warp / CW, lw = warp - grp * CW;        // group and warp inside the group
         for (int c = grp; c < nchunks; c += G) {
             Ring r(nstages);
@@ -199,8 +205,8 @@ __global__ void __launch_bounds__(THREADS) gemv_w4a8_bulk_kernel(
                             const uint4 wv = *reinterpret_cast<const uint4 *>(stage_p + (size_t)lr * wrow + (size_t)b * 16);
                             const float s = sval(reinterpret_cast<const ST *>(stage_p + (size_t)ROWS * wrow + (size_t)lr * srow)[b]);
                             uint32_t e0, o0, e1, o1, e2, o2, e3, o3;
-                            unpack8_x16(wv.x, e0, o0); unpack8_x16(wv.y, e1, o1);
-                            unpack8_x16(wv.z, e2, o2); unpack8_x16(wv.w, e3, o3);
+                            unpack(wv.x, e0, o0); unpack(wv.y, e1, o1);
+                            unpack(wv.z, e2, o2); unpack(wv.w, e3, o3);
                             int d = __dp4a((int)xe[j][0], (int)e0, 0);
                             d = __dp4a((int)xo[j][0], (int)o0, d);
                             d = __dp4a((int)xe[j][1], (int)e1, d);
