@@ -248,11 +248,20 @@ inline int launch_rmsnorm_quantize(const float *X, const float *W, float eps, in
     return launch_status("rmsnorm_quantize_x_q8");
 }
 
+// Eight elements a thread or four: `ctas` CTAs of the wide kernel, each with the work of two narrow ones.  With few of them per SM what
+// counts is how evenly they divide over the SMs, and wide ones divide worse.  us, narrow / wide, SwiGLU, by wide CTAs: 170 1.91 / 2.31, 211 2.05 / 2.43, 261 2.64 / 2.41, 401 2.70 / 2.77, 552 3.38 / 3.14, 723 3.89 / 4.25, 869 4.55 / 4.40,
+// 938 4.64 / 4.44, 1255 5.99 / 4.78, 4236 18.6 / 12.7.  GeGLU, whose tanh costs more than the loads: 180 1.97 / 2.15, 203 1.95 / 2.20,
+// 224 2.60 / 2.29, 356 2.73 / 2.62, 651 3.83 / 4.21, 810 4.33 / 4.18, 4153 18.5 / 12.5.
+constexpr bool glu_takes_wide(long ctas, int sms, int act) {
+    const long per_sm = (ctas + sms - 1) / sms;
+    if (act == 1) return 2 * ctas > 3L * sms && per_sm != 5;
+    return per_sm > 6 || (per_sm % 2 == 0 && 2 * ctas > (2 * per_sm - 1) * sms);
+}
+
 inline int launch_glu_quantize(const float *G, const float *U, int act, float *Y, int8_t *xq, float *xs, int32_t *xsum, int IN,
                                int S, cudaStream_t st, long pitch = 0 /* floats between rows of G / U; 0 = IN */) {
     const long n8 = (long)S * IN / 8, w8 = (n8 + 255) / 256, c8 = (long)sm_count() * 8;
-    // a row of 17408 would be nine CTAs of eight exponentials a thread, seventeen of four otherwise (MLP of one row 42.9 us, 43.8 with them)
-    if (w8 >= sm_count() && aligned(G, 32) && aligned(U, 32) && aligned(xq, 8) && pitch % 8 == 0 && (long)S * IN < (1L << 33)) {
+    if (glu_takes_wide(w8, sm_count(), act) && aligned(G, 32) && aligned(U, 32) && aligned(xq, 8) && pitch % 8 == 0 && (long)S * IN < (1L << 33)) {
         const cudaError_t e = launch_pdl(act == 0 ? glu_quantize_wide_kernel<0> : glu_quantize_wide_kernel<1>, dim3((unsigned)(w8 < c8 ? w8 : c8)), dim3(256), 0, st,
                                          G, U, Y, reinterpret_cast<uint2 *>(xq), xs, xsum, (uint32_t)n8, (uint32_t)(IN / 8), (uint32_t)((pitch > 0 ? pitch : IN) / 8));
         if (e != cudaSuccess) return cuda_fail(e, "glu_quantize_x_q8 launch");
