@@ -119,6 +119,8 @@ def check_stages(oracle, case, lay, ws, out, S, topk, E, H, MI, gemm, act=0):
     (3, 4, 6, 1536, 768, 0, 0),         # the same with two groups per lane in gate|up
     (37, 3, 5, 1120, 416, 2, 0),        # sorted grouped GEMM, rows of 35 and 13 scales: element by element, more K-tiles than the ring has stages
     (150, 3, 5, 1120, 416, 2, 1),       # the same with fp16 scales and two items per expert
+    (19, 9, 12, 160, 64, 2, 0),         # more experts a token than the combine asks for at once, several times
+    (13, 10, 16, 128, 64, 1, 1),        # the same in slot order, fp16 scales
     (40, 2, 300, 64, 32, 2, 0),         # more experts than the sort kernel's per-warp histograms hold
 ])
 def test_moe_block_stages(w4a8, oracle, cuda, S, topk, E, H, MI, kernel, sd):
