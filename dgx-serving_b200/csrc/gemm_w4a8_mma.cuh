@@ -98,6 +98,7 @@ constexpr int ITEM_ROWS = 64;
 struct GroupList {
     const int4 *items = nullptr;
     const int *num_items = nullptr;
+    long likely_items = 0;                                 // what the host expects, for the form of the launch only
 };
 
 template <class C, typename ST, bool GROUPED, bool VEC>
@@ -380,11 +381,16 @@ inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const S
     const bool pairs = scales_pair_up(sw, K, nsplit, gsplit);
     const long units = GROUPED ? (long)max_items * n_tiles : (long)m_tiles * n_tiles * nsplit;
     if (units > 0x7FFFFFFFL) return fail(W4A8_ERR_UNSUPPORTED, "gemm: %ld work units", units);
-    if (GROUPED) {
-        const cudaError_t e = launch_pdl(kern, dim3((unsigned)units), dim3(C::THREADS), C::SMEM, st, tmX, tmW, xs, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs, 0, gl);
+    // Grouped: dependent where the items fill the SMs.  With fewer units than two per SM the CTAs that start early pair up beside what is
+    // still running.  Expert block, us, dependent / not: 94 tokens, 16 experts, 8 of them, 1024 x 512 (128 units) 37.2 / 30.5;
+    // 21, 8, 8, 2048 x 768 (96, 128) 38.0 / 31.6; 362, 32, 4, 512 x 1024 (512, 128) 47.1 / 43.5; 176, 8, 8, 1024 x 512 (192) 40.7 / 39.7;
+    // 300, 16, 8, 1024 x 512 (384) 60.4 / 61.1; 400, 64, 2, 1024 x 512 (512) 41.0 / 41.9; 20, 64, 8, 2048 x 768 (768) 80.8 / 81.5.
+    const bool dependent = GROUPED && gl.likely_items * n_tiles > 2L * sm_count();
+    const int stagger = GROUPED ? 0 : stagger_cycles(units, C::CTAS, C::BM, nsplit > 1 ? gsplit : K / QBLK);
+    if (dependent) {
+        const cudaError_t e = launch_pdl(kern, dim3((unsigned)units), dim3(C::THREADS), C::SMEM, st, tmX, tmW, xs, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs, stagger, gl);
         if (e != cudaSuccess) return cuda_fail(e, "gemm_w4a8_mma launch");
-    } else kern<<<(unsigned)units, C::THREADS, C::SMEM, st>>>(tmX, tmW, xs, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs,
-                                                       GROUPED ? 0 : stagger_cycles(units, C::CTAS, C::BM, nsplit > 1 ? gsplit : K / QBLK), gl);
+    } else kern<<<(unsigned)units, C::THREADS, C::SMEM, st>>>(tmX, tmW, xs, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs, stagger, gl);
     return launch_status("gemm_w4a8_mma");
 }
 

@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float4 *__restri
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         // Four slots' rows are asked for at once: one after the other each waited for its position and its row, and eight cost too much
         // where there are fewer.  Block of 1 token x 2 experts 7.47 us one by one, 7.76 by eight, 7.34 by four; 3 x 4 14.6, 14.1, 13.4; 8 x 8
-        // 39.0, 35.2, 34.7; 79 x 4 61.1, 61.0, 59.9.
+        // 39.0, 35.2, 34.7; 79 x 4 66.5, 61.0, 59.9.
         for (int k0 = 0; k0 < topk; k0 += COMBINE) {
             long row[COMBINE];
             float w[COMBINE];
@@ -403,6 +403,9 @@ inline int launch_experts(const BlockArgs &a, const Buffers &b, bool use_gemm, l
         if (rc != W4A8_OK) return rc;
         gemm_mma::GroupList gl;
         gl.items = b.items; gl.num_items = b.num_items;
+        // slots spread evenly over the experts of all ranks
+        const long all = (long)a.experts * (a.world > 1 ? a.world : 1), rows = (nslots + all - 1) / all;
+        gl.likely_items = (nslots < all ? (nslots * (long)a.experts + all - 1) / all : a.experts) * ((rows + gemm_mma::ITEM_ROWS - 1) / gemm_mma::ITEM_ROWS);
         rc = gemm_mma::launch_grouped(b.xq_g, b.xs_g, a.gu_wq, a.gu_sc, b.gu, nslots, 2 * a.MI, a.H, a.scale_dtype, gl, b.max_items, (long)a.experts * 2 * a.MI, st);
         if (rc != W4A8_OK) return rc;
         rc = launch_glu_quantize(b.gu, b.gu + a.MI, a.act, nullptr, b.xq_h, b.xs_h, nullptr, a.MI, nslots, st, 2L * a.MI);
