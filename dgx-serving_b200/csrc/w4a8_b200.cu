@@ -294,14 +294,32 @@ W4A8_API int w4a8_gemv(const int8_t *xq, const float *xs, const uint8_t *Wq, con
     return gemv_dispatch(xq, xs, Wq, sw, Y, IN, OUT, S, scale_dtype, (cudaStream_t)stream, nullptr);
 }
 
+static bool overlap(const void *a, size_t na, const void *b, size_t nb) {
+    const char *pa = static_cast<const char *>(a), *pb = static_cast<const char *>(b);
+    return a && b && pa < pb + nb && pb < pa + na;
+}
+// No output of several products shares memory with another one or with an input: only then may they run at the same time.
+static bool outputs_apart(const int8_t *xq, const float *xs, int count, const uint8_t *const *Wq, const void *const *sw, float *const *Y,
+                          const int *OUT, int IN, int S, int scale_dtype) {
+    const size_t row = (size_t)IN / QBLK, ssize = scale_dtype == 1 ? 2 : 4;
+    for (int i = 0; i < count; i++) {
+        const size_t yb = (size_t)S * OUT[i] * sizeof(float);
+        if (overlap(Y[i], yb, xq, (size_t)S * IN) || overlap(Y[i], yb, xs, S * row * sizeof(float))) return false;
+        for (int j = 0; j < count; j++)
+            if (overlap(Y[i], yb, Wq[j], (size_t)OUT[j] * IN / 2) || overlap(Y[i], yb, sw[j], OUT[j] * row * ssize) ||
+                (j > i && overlap(Y[i], yb, Y[j], (size_t)S * OUT[j] * sizeof(float)))) return false;
+    }
+    return true;
+}
+
 W4A8_API int w4a8_gemv_multi(const int8_t *xq, const float *xs, int count, const uint8_t *const *Wq, const void *const *sw,
                              float *const *Y, const int *OUT, int IN, int S, int scale_dtype, void *stream) {
     if (count < 0 || count > gemv_bulk::MAX_MATS) return fail(W4A8_ERR_ARG, "gemv_multi: count=%d (0..%d)", count, gemv_bulk::MAX_MATS);
     if (count == 0 || S == 0) return W4A8_OK;
     if (!Wq || !sw || !Y || !OUT) return fail(W4A8_ERR_ARG, "gemv_multi: null array argument");
-    // One launch when every matrix can take the bulk-copy stream (one row, the auto policy's conditions); else the
-    // matrices go one after the other through w4a8_gemv, or two to sixteen rows in one launch of the tensor-path kernel.  Either way each
-    // output equals w4a8_gemv's, bit for bit.
+    // One launch when every matrix can take the bulk-copy stream (one row, the auto policy's conditions) or, two to sixteen rows, the
+    // tensor-path kernel; else, and where an output overlaps another or an input, the matrices go one after the other through w4a8_gemv.
+    // Either way each output equals w4a8_gemv's, bit for bit.
     bool one = S == 1 && (gemv_policy() == 3 || (gemv_policy() == 0 && IN >= 2048));
     gemv_bulk::Plan bp;
     gemv_bulk::Mats m = {};
@@ -312,8 +330,8 @@ W4A8_API int w4a8_gemv_multi(const int8_t *xq, const float *xs, int count, const
         bp = pi;
         m.Wq[i] = Wq[i]; m.sw[i] = sw[i]; m.Y[i] = Y[i]; m.OUT[i] = OUT[i];
     }
-    if (one) {
-        if (scale_dtype != 0 && scale_dtype != 1) return fail(W4A8_ERR_ARG, "gemv_multi: scale_dtype=%d", scale_dtype);
+    if (one && scale_dtype != 0 && scale_dtype != 1) return fail(W4A8_ERR_ARG, "gemv_multi: scale_dtype=%d", scale_dtype);
+    if (one && outputs_apart(xq, xs, count, Wq, sw, Y, OUT, IN, S, scale_dtype)) {
         int rc = require_sm100();
         if (rc != W4A8_OK) return rc;
         m.count = count;
@@ -329,7 +347,8 @@ W4A8_API int w4a8_gemv_multi(const int8_t *xq, const float *xs, int count, const
         mm.Wq[i] = Wq[i]; mm.sw[i] = sw[i]; mm.Y[i] = Y[i]; mm.OUT[i] = OUT[i]; mm.tile0[i] = (int)tiles;
         tiles += ((long)OUT[i] + 15) / 16;
     }
-    if (one && tiles < (1L << 27) && gemv_mma::plan_for(Wq[0], sw[0], IN, (int)(tiles * 16), S, &mp) && gemv_mma::multi_serves(mp)) {
+    if (one && tiles < (1L << 27) && gemv_mma::plan_for(Wq[0], sw[0], IN, (int)(tiles * 16), S, &mp) && gemv_mma::multi_serves(mp) &&
+        outputs_apart(xq, xs, count, Wq, sw, Y, OUT, IN, S, scale_dtype)) {
         int rc = require_sm100();
         if (rc != W4A8_OK) return rc;
         for (int i = count; i <= gemv_mma::MAX_MATS; i++) mm.tile0[i] = (int)tiles;
@@ -520,10 +539,6 @@ static int linear_row(const float *X, int8_t *xq, float *xs, int32_t *xsum, cons
     const size_t mb32 = nb > 192 ? (size_t)-1 >> 20 : nb > 160 ? 32 : nb > 128 ? 18 : 96;
     const bool bulk = bulk_fits && (pol == 3 || (K >= 2048 && wbytes >= ((scale_dtype == 1 ? 5 : mb32) << 20)));
     if (!bulk && !(scale_dtype == 1 ? gemv_row_pays<__half>(K, N) : gemv_row_pays<float>(K, N))) return W4A8_OK;
-    const auto overlap = [](const void *a, size_t na, const void *b, size_t nb) {
-        const char *pa = static_cast<const char *>(a), *pb = static_cast<const char *>(b);
-        return a && b && pa < pb + nb && pb < pa + na;
-    };
     const size_t xb = (size_t)K * 4, sb = (size_t)(K / QBLK) * 4, yb = (size_t)N * 4;
     if (overlap(X, xb, Y, yb) || overlap(xq, K, Y, yb) || overlap(xs, sb, Y, yb) || overlap(xsum, sb, Y, yb) || overlap(X, xb, xq, K) ||
         overlap(X, xb, xs, sb) || overlap(X, xb, xsum, sb)) return W4A8_OK;

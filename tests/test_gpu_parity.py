@@ -414,8 +414,8 @@ def test_config5_moe_shapes(w4a8, oracle, cuda):
 @pytest.mark.parametrize("S,K,OUTS", [(1, 5120, (1000, 1000)), (1, 2048, (40, 3000, 7)), (1, 4096, (512, 256, 256, 77)),
                                       (1, 512, (100, 60)), (5, 2048, (300, 200)), (1, 5120, (17408,))])
 def test_gemv_multi_equals_separate_calls(w4a8, oracle, cuda, S, K, OUTS, scale_dtype):
-    """w4a8_gemv_multi (one launch on the bulk-copy kernel for a single row of 2048..8192 elements; else one call per
-    matrix) gives each matrix the bits of its own w4a8_gemv call, and those are the documented order."""
+    """w4a8_gemv_multi (one launch on the bulk-copy kernel for a single row of 2048..8192 elements, one on the tensor-path kernel for
+    two to sixteen rows; else one call per matrix) gives each matrix the bits of its own w4a8_gemv call, and those are the documented order."""
     mats = [make_case(oracle, S, n, K, seed=4000 + n + i, scale_dtype=scale_dtype) for i, n in enumerate(OUTS)]
     xq, xs = mats[0][0], mats[0][1]
     xq_d, xs_d = to_dev(xq, cuda), to_dev(xs, cuda)
