@@ -22,7 +22,8 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.mark.parametrize("world", [2, 4, 8])
-@pytest.mark.parametrize("S,N,K", [(1, 520, 512), (5, 520, 512), (16, 1000, 1024), (20, 264, 256), (3, 37, 96), (1, 1000, 2048)])
+@pytest.mark.parametrize("S,N,K", [(1, 520, 512), (5, 520, 512), (16, 1000, 1024), (20, 264, 256), (3, 37, 96), (1, 1000, 2048),
+                                   (12, 520, 1536), (9, 130, 768), (16, 1000, 2304)])     # more than eight rows, sums handed from warp to warp
 def test_fused_allgather_ranks_emulated(w4a8, oracle, cuda, S, N, K, world):
     """`world` ranks emulated on one GPU: their kernels run one after the other over `world` arenas (never two waiting
     kernels at once), then every rank's wait finds all flags set."""

@@ -3,6 +3,8 @@ against the kernel for X aligned to 16 bytes with what is not finite, subnormal 
 import numpy as np
 import pytest
 
+from conftest import launched_kernels
+
 pytestmark = pytest.mark.gpu
 
 
@@ -14,7 +16,13 @@ def _run(w4a8, cuda, X, shift):
     xq = torch.full((S + 1, K), 77, dtype=torch.int8, device=cuda)
     xs = torch.full((S + 1, K // 32), 7.0, dtype=torch.float32, device=cuda)
     xsum = torch.full((S + 1, K // 32), 7, dtype=torch.int32, device=cuda)
-    w4a8.launch_quantize_x_q8(flat[shift:], xq, xs, xsum, K, S)
+
+    def call(stream):
+        w4a8.launch_quantize_x_q8(flat[shift:], xq, xs, xsum, K, S, stream)
+
+    call(None)
+    torch.cuda.synchronize()
+    assert [("wide_kernel" in n, "vec_kernel" in n) for n in launched_kernels(call)] == [(shift == 0, shift != 0)]
     assert bool((xq[S] == 77).all()) and bool((xs[S] == 7.0).all()) and bool((xsum[S] == 7).all())
     return xq[:S].cpu().numpy(), xs[:S].cpu().numpy().view(np.uint32), xsum[:S].cpu().numpy()
 
