@@ -254,9 +254,11 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) gemm_w4a8_mma_kernel(
                 }
             }
             uint32_t b0, b1;
-            // two tiles that ptxas orders worse with the shorter form (64 rows, fp32 scales: 768 x 9000 x 3840 156 us, 164 with it, 1024 x 17408 x
-            // 5120 504 and 560; 80 rows, fp16: 2048 x 17408 x 5120 952 and 966); every other one gains, up to 11 %
-            constexpr bool EXPR = !GROUPED && ((TM == 4 && sizeof(ST) == 4) || (TM == 5 && sizeof(ST) == 2));
+            // Two tiles that the shorter form of the unpacking slows down, timed on the shapes that take them with the second CTA of an SM
+            // starting later: time of the longer form over the shorter one, 64 rows with fp32 scales 0.97 (scales that do not line up 1.00,
+            // and steadier), 80 rows with fp16 scales that line up 0.995, that do not 1.02; 32 and 48 rows 1.01 to 1.03, 64 rows fp16 1.04,
+            // 80 rows fp32 1.02, 96 rows 1.02 to 1.03.
+            constexpr bool EXPR = !GROUPED && ((TM == 4 && sizeof(ST) == 4) || (TM == 5 && sizeof(ST) == 2 && VEC));
             const uint32_t word = *reinterpret_cast<const uint32_t *>(Bs + (boff ^ ((bfirst + bg) << 4)) + j * 512);
             if constexpr (EXPR) unpack8_x16_expr(word, b0, b1);
             else unpack8_x16(word, b0, b1);
@@ -351,15 +353,18 @@ inline bool scales_pair_up(const ST *sw, int K, int nsplit, int gsplit) {
     return (K / QBLK) % 2 == 0 && (nsplit == 1 || gsplit % 2 == 0) && aligned(sw, 4);
 }
 // Two CTAs of an SM that start together end together, and those of the last wave then pair up on the SMs that come free first; they
-// also want the same pipes at the same time.  So where there is more than one wave the second CTA of an SM starts 5 % of a tile's time
-// later, which is more than SMs differ by.  us, without / with: 768 x 9000 x 3840 in 80-row tiles 173 / 152, fp16 scales 182 / 167;
-// 500 x 9000 x 2048 in 96-row tiles 79 / 69; 1500 x 5000 x 4096 in 96-row tiles, fp16, 216 / 191; 2048 x 17408 x 5120 911 / 905.  Where
-// nothing pairs up it costs up to 1.5 %: 768 x 9000 x 3840 in 96-row tiles 144.6 / 145.9.  2 % of a tile's time is too little (172.8 in
-// the first case), 10 % dearer.  Three and four CTAs per SM drift apart by themselves (48 rows: 154.8 / 155.1; 333 x 15360 x 3840
-// 116 / 118).  Not on a chip whose number of SMs is another one.
-inline int stagger_cycles(long ctas, int per_sm, int rows, int groups) {
+// also want the same pipes at the same time.  So where there is more than one wave the second CTA of an SM starts later: 5 % of a tile's
+// time, which is about what SMs differ by, or 12 % where the last wave has at most one CTA per SM and pairing up costs most.  Time over
+// that without, 0 / 3 / 5 / 8 / 12 %, mean over the shapes of 17967 random ones: last wave of at most one CTA per SM behind one full
+// wave, 64 rows 1 / 0.92 / 0.88 / 0.86 / 0.85, 80 rows 1 / 0.87 / 0.84 / 0.83 / 0.83 (and the worst twentieth of them 1.00 of the time
+// before the shorter unpacking, 1.12 with 5 %), behind two 80 rows 1 / 0.96 / 0.95 / 0.94 / 0.93; larger last waves, 80 rows
+// 1 / 1.00 / 1.00 / 1.00 / 1.01.  96 rows with fp32 scales that line up gain nothing from more than 5 %: 1 / 0.93 / 0.92 / 0.93 / 0.94.
+// Three and four CTAs per SM drift apart by themselves (48 rows: 154.8 / 155.1; 333 x 15360 x 3840 116 / 118).  Not on a chip whose
+// number of SMs is another one.
+inline int stagger_cycles(long ctas, int per_sm, int rows, int groups, bool more) {
     if (per_sm != 2 || sm_count() != (int)SMS || ctas <= 2 * (long)SMS) return 0;
-    const long cycles = (long)groups * rows * 12 / 20;         // a group of a tile's row takes about 12 cycles with two CTAs on the SM
+    const long rest = ctas % (2 * (long)SMS);
+    const long cycles = (long)groups * rows * 12 * (more && rest > 0 && rest <= (long)SMS ? 12 : 5) / 100;  // a group of a tile's row takes about 12 with two CTAs on the SM
     return (int)(cycles < 100000 ? cycles : 100000);
 }
 template <class C, typename ST, bool GROUPED, bool VEC>
@@ -386,7 +391,7 @@ inline int launch_c(const int8_t *X, const float *xs, const uint8_t *Wq, const S
     // 21, 8, 8, 2048 x 768 (96, 128) 38.0 / 31.6; 362, 32, 4, 512 x 1024 (512, 128) 47.1 / 43.5; 176, 8, 8, 1024 x 512 (192) 40.7 / 39.7;
     // 300, 16, 8, 1024 x 512 (384) 60.4 / 61.1; 400, 64, 2, 1024 x 512 (512) 41.0 / 41.9; 20, 64, 8, 2048 x 768 (768) 80.8 / 81.5.
     const bool dependent = GROUPED && gl.likely_items * n_tiles > 2L * sm_count();
-    const int stagger = GROUPED ? 0 : stagger_cycles(units, C::CTAS, C::BM, nsplit > 1 ? gsplit : K / QBLK);
+    const int stagger = GROUPED ? 0 : stagger_cycles(units, C::CTAS, C::BM, nsplit > 1 ? gsplit : K / QBLK, !(C::BM == 96 && sizeof(ST) == 4 && VEC));
     if (dependent) {
         const cudaError_t e = launch_pdl(kern, dim3((unsigned)units), dim3(C::THREADS), C::SMEM, st, tmX, tmW, xs, sw, Y, M, N, K, m_tiles, n_tiles, gsplit, pairs, stagger, gl);
         if (e != cudaSuccess) return cuda_fail(e, "gemm_w4a8_mma launch");
@@ -409,8 +414,9 @@ using Cfg96 = Cfg<6, 4, 1, 4, 4, 2>;
 // K.  ns: a group of K with 1, 2, 3, 4 of its kind on an SM.  tail_ns: the same in a wave behind full ones, which starts as slots
 // come free.  Five columns each: fp32 scales that line up, fp32 scales copied 4 bytes at a time, pairs of fp16 scales, fp16 scales
 // of an odd K / 32 (plain loads), fp16 scales that line up.  Fitted to 16874 shapes, M = 1 .. 2048, N = 64 .. 20000, one to eight
-// ranges of 1 to 200 groups, on which every tile was timed: the choice is 0.6 to 0.9 % slower than the fastest tile on average, 12 to
-// 15 % at the 99th percentile.  A tile taller than one that holds all rows has only more padding; 16 rows were not timed above
+// ranges of 1 to 200 groups, on which every tile was timed, with the longer unpacking and no later start.  With both as they are now, on
+// 9482 other shapes of these ranges: the choice is 0.6 to 0.8 % slower than the fastest tile on average, 10 to 12 % at the 99th
+// percentile.  A tile taller than one that holds all rows has only more padding; 16 rows were not timed above
 // max_rows.  Not among them because never or hardly ever ahead: 128 x 128 tiles (fastest for 32 of 15284 shapes, by a few per cent)
 // and the tcgen05 kernel (for none).
 enum class Tile { R16, R32, R48, R64, R64X3, R80, R96 };
@@ -451,7 +457,9 @@ inline Tile pick(long M, long N, int K, int nsplit, int gsplit, Scales scales) {
         const long ctas = (M + k.rows - 1) / k.rows * n_tiles, wave = sms * k.per_sm, full = ctas / wave, rest = ctas % wave;
         const long last = (rest + sms - 1) / sms;           // CTAs per SM in the last wave
         const long last_ns = last == 0 ? 0 : full == 0 || last == k.per_sm ? k.ns[scales][last - 1] : k.tail_ns[scales][last - 1];
-        const long t = (full + (last != 0)) * k.wave_ns[scales] + (full * k.ns[scales][k.per_sm - 1] + last_ns) * groups;
+        long t = (full + (last != 0)) * k.wave_ns[scales] + (full * k.ns[scales][k.per_sm - 1] + last_ns) * groups;
+        // 96 rows whose last wave behind a full one pairs up now and then whatever the later start: 801 x 6272 x 3968 141 us, 118 in 48 rows
+        if (k.tile == Tile::R96 && scales == LINED_UP && full == 1 && last == 1) t += t / 20;
         if (best_ns == 0 || t < best_ns) { best = k.tile; best_ns = t; }
     }
     return best;
