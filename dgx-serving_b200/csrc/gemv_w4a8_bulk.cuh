@@ -178,8 +178,9 @@ __global__ void __launch_bounds__(THREADS) gemv_w4a8_bulk_kernel(
 #pragma unroll
             for (int i = 0; i < 4; i++) split_even_odd(v[2 * i], v[2 * i + 1], xe[j][i], xo[j][i]);
         }
-        // six groups a lane fit the registers with the longer form only: with the other one ptxas spills 104 bytes.
-        constexpr bool EXPR = NG == 6 && !PEER && !FUSE;
+        // Six groups a lane fit the registers with the longer form only (with the other one ptxas spills 104 bytes); eight spill with
+        // either: 7936 x 5494 fp16 11.0 us, 11.6 with the shorter one, 7680 x 18057 26.5 and 28.1.
+        constexpr bool EXPR = (NG == 6 || NG == 8) && !PEER && !FUSE;
         const auto unpack = [](uint32_t w, uint32_t &e, uint32_t &o) {
             if constexpr (EXPR) unpack8_x16_expr(w, e, o);
             else unpack8_x16(w, e, o);
