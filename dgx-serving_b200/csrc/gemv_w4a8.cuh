@@ -89,7 +89,8 @@ __device__ __forceinline__ void gemv_load_batch(GemvBatch<U, ST> &bt, const uint
     }
 }
 
-template <int MT, int U, typename ST>
+// EXPR: the weights unpacked by the longer form, which leaves registers for one more CTA per SM in the kernels that name it.
+template <int MT, int U, typename ST, bool EXPR>
 __device__ __forceinline__ void gemv_compute_batch(const GemvBatch<U, ST> &bt, float (&acc)[MT], const uint4 *plane0,
                                                    const uint4 *plane1, const float *sxs, int slot0, int lane, int nb) {
 #pragma unroll
@@ -97,8 +98,12 @@ __device__ __forceinline__ void gemv_compute_batch(const GemvBatch<U, ST> &bt, f
         const int b = lane + 32 * (slot0 + u);
         if (b < nb) {
             uint32_t e0, o0, e1, o1, e2, o2, e3, o3;
-            unpack8_x16(bt.w[u].x, e0, o0); unpack8_x16(bt.w[u].y, e1, o1);
-            unpack8_x16(bt.w[u].z, e2, o2); unpack8_x16(bt.w[u].w, e3, o3);
+            const auto unpack = [](uint32_t w, uint32_t &e, uint32_t &o) {
+                if constexpr (EXPR) unpack8_x16_expr(w, e, o);
+                else unpack8_x16(w, e, o);
+            };
+            unpack(bt.w[u].x, e0, o0); unpack(bt.w[u].y, e1, o1);
+            unpack(bt.w[u].z, e2, o2); unpack(bt.w[u].w, e3, o3);
 #pragma unroll
             for (int m = 0; m < MT; m++) {
                 const uint4 xa = plane0[m * nb + b], xb = plane1[m * nb + b];
@@ -227,6 +232,10 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_w4a8_dp4a_kernel(
 #pragma unroll
     for (int m = 0; m < MT; m++) acc[m] = 0.f;
 
+    // Two rows, three fp16 slots in flight: 64 registers with the longer unpacking, 69 with the shorter one, so four CTAs per SM instead of
+    // three: 6080 x 4244 7.0 us, 10.0 with three, 2912 x 4708 4.1 and 5.0, although 8672 x 2823 takes 7.8 and 6.6; held to 64 registers by
+    // the launch bounds the shorter form is 3 % slower than the longer on average.  Four rows, two fp16 slots, peer stores: 80 and 90.
+    constexpr bool EXPR = sizeof(ST) == 2 && ((MT == 2 && U == 3) || (MT == 4 && U == 2 && PEER));
     // item i: row = r0 + warp + 8*(i / nbatch), batch = i % nbatch.  Two items per trip so that the two
     // register buffers alternate without copies.
     int row = r0 + warp, batch = 0;
@@ -245,13 +254,13 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_w4a8_dp4a_kernel(
         int nrow = row, nbt = batch;
         advance(nrow, nbt);
         if (i + 1 < nitems) gemv_load_batch<U, ST>(bb, Wq + (size_t)nrow * wpitch, sw + (size_t)nrow * nb, nbt * U, lane, nb, w_a16);
-        gemv_compute_batch<MT, U, ST>(ba, acc, plane0, plane1, sxs, batch * U, lane, nb);
+        gemv_compute_batch<MT, U, ST, EXPR>(ba, acc, plane0, plane1, sxs, batch * U, lane, nb);
         if (batch == nbatch - 1) finish_row(row);
         if (i + 1 >= nitems) break;
         row = nrow; batch = nbt;
         advance(nrow, nbt);
         if (i + 2 < nitems) gemv_load_batch<U, ST>(ba, Wq + (size_t)nrow * wpitch, sw + (size_t)nrow * nb, nbt * U, lane, nb, w_a16);
-        gemv_compute_batch<MT, U, ST>(bb, acc, plane0, plane1, sxs, batch * U, lane, nb);
+        gemv_compute_batch<MT, U, ST, EXPR>(bb, acc, plane0, plane1, sxs, batch * U, lane, nb);
         if (batch == nbatch - 1) finish_row(row);
         row = nrow; batch = nbt;
     }
