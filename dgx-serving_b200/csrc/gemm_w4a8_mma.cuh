@@ -10,11 +10,11 @@
 // cycles per 128 x 128 outputs and group, at 6 % tensor-pipe use, and always for 128 rows.  mma.sync m16n8k32 leaves the
 // dots in the registers that the epilogue reads: no hand-off, and a tile has as many rows as there are, in steps of 16.
 // Alone (a loop without loads) MMA 270, I2F 256 (on the ALU pipe) and packed mul + fma 278 cycles per 128 x 128 group; together
-// 630, because the legacy tensor path and the packed fp32 pipe take turns: that is the floor of this kernel.  By the times below
-// and at 1965 MHz it needs 750 to 790 with two CTAs of 80 or 96 rows per SM, 860 with three of 48, 1070 with one of 48: a lone
-// CTA has one warp per scheduler, and nothing covers its waits.  Measured, us, with cp.async operands / with TMA:
-// 2048 x 17408 x 5120 1088 / 942, 333 x 15360 x 3840 164 / 123, 48 x 3840 x 15360 in three K ranges, twice, with the quantizer,
-// 106 / 85.  Slower in the first versions, in cycles per 128 x 128 group: integer-to-float through a preset accumulator (1.5 * 2^23)
+// 630, because the legacy tensor path and the packed fp32 pipe take turns: that is the floor of this kernel.  At 1965 MHz it needs
+// 750 at 2048 x 17408 x 5120 (two CTAs of 80 rows per SM), 880 at 333 x 15360 x 3840 (three of 48) and about 1100 where an SM has one
+// CTA of 48: it has one warp per scheduler, and nothing covers its waits.  Measured, us, with the quantizer, with cp.async operands /
+// with TMA / with the shorter unpacking and the later start as well: these two 1088 / 942 / 913 and 164 / 123 / 119, 48 x 3840 x 15360
+// in three K ranges, twice, 106 / 86 / 80.  Slower in the first versions, in cycles per 128 x 128 group: integer-to-float through a preset accumulator (1.5 * 2^23)
 // instead of I2F (1133 against 989), scalar instead of packed fp32 (1044 against 864), scales through registers (977 against 864;
 // they spill).  Thin tiles with cp.async operands, 32 x 3840 x 15360 in three ranges: 41 us; 8 and 16 warps per CTA 45 and 49,
 // K-tiles of 8 groups 43, rows prefetched to L2 47 to 61.  A barrier asked ahead of time, so that a CTA does not wait for the answer:
@@ -22,7 +22,7 @@
 //
 // Data flow.  TMA brings K-tiles of 4 groups into a STAGES-deep ring, one barrier per stage: activations in the 128-byte swizzle
 // (a row's 4 groups), packed weights in the 64-byte one.  With cp.async the same copies, 16 bytes a lane, ran at 13 bytes per cycle
-// and SM and took the issue slots of the warps that multiply: without any copies 333 x 15360 x 3840 took 119 us instead of 164.
+// and SM and took the issue slots of the warps that multiply: without any copies 333 x 15360 x 3840 then took 119 us instead of 164.
 // Fragment reads are contiguous up to the swizzle (LDS.64 and LDS.32, no conflicts).  A lane's word of weights expands to its two B
 // registers with three logic operations (unpack8_x16: even and odd elements), the matching A registers are two byte permutes of
 // eight activations.  Any order of K inside a group gives the same integer.  Scales travel with their K-tile by cp.async,

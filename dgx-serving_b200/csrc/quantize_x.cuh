@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(256) quantize_x_q8_vec_kernel(const float4 *__
 // element = 6.1 TB/s of the measured 6.56; 4000 x 3840 18.8 -> 14.2, 2048 x 5120 14.2 -> 9.7, one row of 5120 2.7 -> 2.2.  One vector a
 // thread: two, three and four in flight 1 to 5 us more at 8192 rows, and fewer threads hide less in the small cases (16 x 5120 2.9,
 // 3.2, 3.7).
-constexpr int WIDE_CTAS = 6;                     // of 256 threads on an SM with 42 registers; a grid of eight per SM is 1.3 waves: 44.0 us
+constexpr int WIDE_CTAS = 6;                     // of 256 threads on an SM with up to 40 registers (it has 37); a grid of eight per SM is 1.3 waves: 44.0 us
 __device__ __forceinline__ void load8(const float *p, float (&v)[8]) {
     asm volatile("ld.global.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
