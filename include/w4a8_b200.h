@@ -124,7 +124,8 @@ int w4a8_gemv(const int8_t *xq, const float *xs, const uint8_t *Wq, const void *
  * models/gemma4_decode.cu:110-112).  Y[i][S, OUT[i]] = w4a8_gemv(xq, xs, Wq[i], sw[i]) for i < count <= 4, bit for bit.
  * A single row whose matrices all qualify for the bulk-copy streaming kernel goes out as ONE kernel launch with the
  * SMs divided between the matrices in proportion to their rows, and so do 2 to 16 rows whose matrices all qualify for the
- * tensor-path kernel; anything else is the same as `count` calls. */
+ * tensor-path kernel; anything else, outputs that share memory with one another or with an input among it, is the same as
+ * `count` calls. */
 int w4a8_gemv_multi(const int8_t *xq, const float *xs, int count, const uint8_t *const *Wq,
                     const void *const *sw, float *const *Y, const int *OUT, int IN, int S, int scale_dtype,
                     void *stream);
