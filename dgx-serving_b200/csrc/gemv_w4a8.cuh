@@ -89,7 +89,6 @@ __device__ __forceinline__ void gemv_load_batch(GemvBatch<U, ST> &bt, const uint
     }
 }
 
-// EXPR: the weights unpacked by the longer form, which leaves registers for one more CTA per SM in the kernels that name it.
 template <int MT, int U, typename ST, bool EXPR>
 __device__ __forceinline__ void gemv_compute_batch(const GemvBatch<U, ST> &bt, float (&acc)[MT], const uint4 *plane0,
                                                    const uint4 *plane1, const float *sxs, int slot0, int lane, int nb) {
@@ -130,7 +129,8 @@ __device__ __forceinline__ void gemv_compute_batch(const GemvBatch<U, ST> &bt, f
 // 112, 57 with 160; four 3840 -> 4096: 18.9, 16.4, 16.3, 16.3; start 56.1 and 23.7).
 constexpr int FUSE_WARPS = 24;
 constexpr uint32_t FUSE_PREFETCH = 96 * 1024;
-template <int MT, int U, typename ST, bool PEER, int WARPS>
+// EXPR: the weights unpacked by the longer form (gemv_takes_longer).
+template <int MT, int U, typename ST, bool PEER, int WARPS, bool EXPR>
 __global__ void __launch_bounds__(WARPS * 32) gemv_w4a8_dp4a_kernel(
     const int8_t *__restrict__ xq, const float *__restrict__ xs, const uint8_t *__restrict__ Wq,
     const ST *__restrict__ sw, float *__restrict__ Y, int IN, int OUT, int S, bool w_a16, GroupedArgs ga, OutArgs oa, RowSrc src) {
@@ -232,10 +232,6 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_w4a8_dp4a_kernel(
 #pragma unroll
     for (int m = 0; m < MT; m++) acc[m] = 0.f;
 
-    // Two rows, three fp16 slots in flight: 64 registers with the longer unpacking, 69 with the shorter one, so four CTAs per SM instead of
-    // three: 6080 x 4244 7.0 us, 10.0 with three, 2912 x 4708 4.1 and 5.0, although 8672 x 2823 takes 7.8 and 6.6; held to 64 registers by
-    // the launch bounds the shorter form is 3 % slower than the longer on average.  Four rows, two fp16 slots, peer stores: 80 and 90.
-    constexpr bool EXPR = sizeof(ST) == 2 && ((MT == 2 && U == 3) || (MT == 4 && U == 2 && PEER));
     // item i: row = r0 + warp + 8*(i / nbatch), batch = i % nbatch.  Two items per trip so that the two
     // register buffers alternate without copies.
     int row = r0 + warp, batch = 0;
@@ -268,7 +264,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_w4a8_dp4a_kernel(
 }
 
 // CTAs that an SM holds at once; asked of the runtime once per kernel variant and smem size.
-template <int MT, int U, typename ST, bool PEER, int WARPS>
+template <int MT, int U, typename ST, bool PEER, int WARPS, bool EXPR = false>
 inline cudaError_t gemv_ctas_per_sm(size_t smem, int *ctas) {
     struct Occ { size_t smem_plus1; int occ; };          // per device: another GPU may answer differently
     static PerDevice<Occ> occ_dev;
@@ -277,7 +273,7 @@ inline cudaError_t gemv_ctas_per_sm(size_t smem, int *ctas) {
     *ctas = oc.occ > 0 ? oc.occ : 1;
     if (oc.smem_plus1 == 0 || occ_smem != smem) {
         int n = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gemv_w4a8_dp4a_kernel<MT, U, ST, PEER, WARPS>, WARPS * 32, smem);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gemv_w4a8_dp4a_kernel<MT, U, ST, PEER, WARPS, EXPR>, WARPS * 32, smem);
         if (e != cudaSuccess) return e;
         oc.occ = *ctas = n > 0 ? n : 1;
         oc.smem_plus1 = smem + 1;
@@ -287,11 +283,11 @@ inline cudaError_t gemv_ctas_per_sm(size_t smem, int *ctas) {
 
 inline size_t gemv_smem_bytes(int MT, int IN) { return (size_t)MT * IN + (size_t)MT * (IN / QBLK) * sizeof(float); }
 
-template <int MT, int U, typename ST, bool PEER, int WARPS = GEMV_WARPS>
+template <int MT, int U, typename ST, bool PEER, int WARPS = GEMV_WARPS, bool EXPR = false>
 inline int launch_gemv_dp4a_p(const int8_t *xq, const float *xs, const uint8_t *Wq, const ST *sw, float *Y,
                               int IN, int OUT, int S, cudaStream_t st, const GroupedArgs &ga, const OutArgs &oa, const RowSrc &src = RowSrc()) {
     const size_t smem = gemv_smem_bytes(MT, IN);
-    auto kern = gemv_w4a8_dp4a_kernel<MT, U, ST, PEER, WARPS>;
+    auto kern = gemv_w4a8_dp4a_kernel<MT, U, ST, PEER, WARPS, EXPR>;
     if (smem > 48 * 1024) {
         static PerDevice<size_t> configured_dev;        // grow-only; the opt-in is a per-device function attribute
         size_t &configured = configured_dev.get();
@@ -304,7 +300,7 @@ inline int launch_gemv_dp4a_p(const int8_t *xq, const float *xs, const uint8_t *
     // Persistent: as many CTAs as are resident at once (fewer when there are not enough rows, or when grouped
     // slots already fill the GPU).
     int occ = 1;
-    cudaError_t oe = gemv_ctas_per_sm<MT, U, ST, PEER, WARPS>(smem, &occ);
+    cudaError_t oe = gemv_ctas_per_sm<MT, U, ST, PEER, WARPS, EXPR>(smem, &occ);
     if (oe != cudaSuccess) return cuda_fail(oe, "gemv occupancy query");
     long want = WARPS == GEMV_WARPS ? (OUT + WARPS - 1) / WARPS : OUT;     // one CTA per SM: every SM takes part in a narrow matrix
     long cap = (long)sm_count() * occ;
@@ -316,10 +312,21 @@ inline int launch_gemv_dp4a_p(const int8_t *xq, const float *xs, const uint8_t *
     return launch_status("gemv_w4a8");
 }
 
+// Two rows, three fp16 slots in flight: unpacked by the longer form the kernel has 64 registers and four CTAs per SM, by the shorter one 69
+// and three but a seventh fewer instructions.  The longer one where four per SM take fewer rounds over the rows than three.  us, longer /
+// shorter, by CTAs of eight rows per SM: 6080 x 1327 (1.1) 5.4 / 4.7, 8672 x 2823 (2.4) 7.8 / 6.6, 6080 x 4244 (3.6) 7.0 / 10.0,
+// 8320 x 5991 (5.1) 15.0 / 13.7, 5248 x 7913 (6.7) 10.8 / 13.2, 5152 x 9650 (8.2) 14.6 / 13.4, 5440 x 11965 (10.1) 15.6 / 17.6.
+inline bool gemv_takes_longer(int OUT, int sms) {
+    const long ctas = (OUT + GEMV_WARPS - 1) / GEMV_WARPS;
+    return (ctas + 4L * sms - 1) / (4L * sms) < (ctas + 3L * sms - 1) / (3L * sms);
+}
 template <int MT, int U, typename ST>
 inline int launch_gemv_dp4a_t(const int8_t *xq, const float *xs, const uint8_t *Wq, const ST *sw, float *Y,
                               int IN, int OUT, int S, cudaStream_t st, const GroupedArgs &ga, const OutArgs &oa) {
-    if (oa.peers) return launch_gemv_dp4a_p<MT, U, ST, true>(xq, xs, Wq, sw, Y, IN, OUT, S, st, ga, oa);
+    // four rows, two fp16 slots, peer stores: 80 registers with the longer form, 90 with the shorter one
+    if (oa.peers) return launch_gemv_dp4a_p<MT, U, ST, true, GEMV_WARPS, MT == 4 && U == 2 && sizeof(ST) == 2>(xq, xs, Wq, sw, Y, IN, OUT, S, st, ga, oa);
+    if constexpr (MT == 2 && U == 3 && sizeof(ST) == 2)
+        if (!ga.idx && gemv_takes_longer(OUT, sm_count())) return launch_gemv_dp4a_p<MT, U, ST, false, GEMV_WARPS, true>(xq, xs, Wq, sw, Y, IN, OUT, S, st, ga, oa);
     return launch_gemv_dp4a_p<MT, U, ST, false>(xq, xs, Wq, sw, Y, IN, OUT, S, st, ga, oa);
 }
 
